@@ -38,6 +38,7 @@ void load_kernels()
     if (done[d]) return;
     done[d] = 1;
     load_mixed_kernels();
+    load_fx_kernels();
     load_fused_kernels();
     load_varsize_kernels();
     load_extras_kernels();
@@ -163,15 +164,20 @@ bool sync_ok(const char *what) { return cuda_ok(cudaDeviceSynchronize(), what); 
 // Workspace of ves_eigensolve: the FP64 solver's slots, and for the mixed
 // form also its FP32 slots, the fallback list and its counter (256-byte aligned).
 struct WsPlan {
-    size_t fp64, mixed, list, count, total;
+    size_t fp64, mixed, list, count;
+    size_t flist;  // matrices the fixed-point solve leaves to the FP64 kernels: counter (256 bytes), then the list
+    size_t total;
+    size_t flist_at() const { return fp64 + mixed + list + count; }
 };
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+size_t flist_bytes(int n, long long N) { return ves::fx_order(n) ? 256 + align256((size_t)N * sizeof(int)) : 0; }
 WsPlan workspace_plan(int precision, int n, long long N, bool vectors, int bps)
 {
     WsPlan p{};
     if (!vectors) {
         p.fp64 = align256(ves::eigvals_workspace_bytes(n, N, bps));
-        p.total = p.fp64;
+        p.flist = flist_bytes(n, N);
+        p.total = p.fp64 + p.flist;
         return p;
     }
     // FP64: blocks_per_sm shapes the fused kernel; FP32 + refinement: it shapes
@@ -183,7 +189,8 @@ WsPlan workspace_plan(int precision, int n, long long N, bool vectors, int bps)
         p.list = align256((size_t)N * sizeof(int));
         p.count = 256;
     }
-    p.total = p.fp64 + p.mixed + p.list + p.count;
+    p.flist = flist_bytes(n, N);
+    p.total = p.fp64 + p.mixed + p.list + p.count + p.flist;
     return p;
 }
 
@@ -262,7 +269,8 @@ bool do_eigensolver(int dim, int bc, int tc, double *rA, double *iA, double *rE,
     nchunks = std::min<long long>(nchunks, bc);
     const long long cb = (bc + nchunks - 1) / nchunks;  // blocks per chunk
     nchunks = (bc + cb - 1) / cb;
-    const size_t wsb = ves::fused_workspace_bytes(dim, cb * (long long)tc, 0, nullptr, nullptr);
+    const size_t wsf = align256(ves::fused_workspace_bytes(dim, cb * (long long)tc, 0, nullptr, nullptr));
+    const size_t wsb = wsf + flist_bytes(dim, cb * (long long)tc);
     void *ws[2] = {b.raw(6, wsb), nchunks > 1 ? b.raw(9, wsb) : nullptr};
     NEED(ws[0]);
     if (nchunks > 1) NEED(ws[1]);
@@ -292,7 +300,8 @@ bool do_eigensolver(int dim, int bc, int tc, double *rA, double *iA, double *rE,
         a.ws = ws[c & 1];
         a.max_its = 30;
         a.vnorm = VES_VNORM_REFERENCE;
-        return cuda_ok(ves::launch_fused_fp64(a, s), "eigensolver kernel launch");
+        int *fcount = reinterpret_cast<int *>(static_cast<char *>(a.ws) + wsf);
+        return cuda_ok(ves::launch_plain(a, fcount + 64, fcount, s), "eigensolver kernel launch");
     };
     auto copy_out = [&](long long c) -> bool {
         ves::NvtxRange r("ves chunk: copy out");
@@ -729,14 +738,31 @@ int ves_eigensolve(int dim, int block_cnt, int thread_cnt, const double *rA, con
     a.vnorm = o.vnorm;
     a.blocks_per_sm = o.precision == VES_PREC_FP64 ? o.blocks_per_sm : 0;
     cudaStream_t st = (cudaStream_t)stream;
-    if (!vectors)
-        return native(cuda_ok(
-            ves::launch_eigvals(g, rA, iA, rE, iE, status, sweeps, ws, o.max_its, o.blocks_per_sm, st),
-            "eigenvalues kernel launch"));
-    if (o.precision == VES_PREC_FP64)
-        return native(cuda_ok(ves::launch_fused_fp64(a, st), "eigensolve kernel launch"));
-
     char *base = static_cast<char *>(ws);
+    int *fcount = reinterpret_cast<int *>(base + plan.flist_at()), *flist = fcount + 64;
+    if (!vectors) {
+        if (ves::fx_order(dim)) {
+            ves::FxArgs f{};
+            f.g = g;
+            f.rA = rA; f.iA = iA; f.rE = rE; f.iE = iE;
+            f.status = status; f.sweeps = sweeps;
+            f.max_its = o.max_its;
+            f.out_list = flist; f.out_count = fcount;
+            f.ws = ws;
+            f.lane_blocks = ves::eigvals_blocks(dim, g.N, o.blocks_per_sm);
+            if (!cuda_ok(cudaMemsetAsync(fcount, 0, sizeof(int), st), "list counter reset") ||
+                !cuda_ok(ves::launch_fx(f, false, st), "eigenvalues kernel launch"))
+                return VES_ERR_CUDA;
+        } else {
+            flist = fcount = nullptr;
+        }
+        return native(cuda_ok(ves::launch_eigvals(g, rA, iA, rE, iE, status, sweeps, ws, o.max_its, o.blocks_per_sm,
+                                                  flist, fcount, st),
+                              "eigenvalues kernel launch"));
+    }
+    if (o.precision == VES_PREC_FP64)
+        return native(cuda_ok(ves::launch_plain(a, flist, fcount, st), "eigensolve kernel launch"));
+
     int *list = reinterpret_cast<int *>(base + plan.fp64 + plan.mixed);
     int *count = reinterpret_cast<int *>(base + plan.fp64 + plan.mixed + plan.list);
     if (!cuda_ok(cudaMemsetAsync(count, 0, sizeof(int), st), "fallback counter reset")) return VES_ERR_CUDA;
@@ -784,7 +810,8 @@ int ves_eigensolve(int dim, int block_cnt, int thread_cnt, const double *rA, con
     if (!cuda_ok(me, "mixed-precision kernel launch")) return VES_ERR_CUDA;
     a.list = list;
     a.list_count = count;
-    return native(cuda_ok(ves::launch_fp64_list(a, st), "fallback kernel launch"));
+    a.status_or = VES_STATUS_REFINE_FALLBACK;
+    return native(cuda_ok(ves::launch_plain(a, flist, fcount, st), "fallback kernel launch"));
 }
 
 size_t ves_polyroots_workspace_size(int degree, int block_cnt, int thread_cnt)
@@ -865,14 +892,15 @@ int ves_complex_from_soa_vec(int dim, int block_cnt, int thread_cnt, const doubl
 // for the polish pre-pass (shift_polish > 0, dim <= 32) the polished
 // predictions (two SoA vector planes).
 struct ShiftsPlan {
-    size_t fused, polish, total;
+    size_t fused, polish, flist, total;
 };
 ShiftsPlan shifts_plan(int dim, long long N, const ves_options &o)
 {
     ShiftsPlan p{};
     p.fused = align256(ves::fused_workspace_bytes(dim, N, o.blocks_per_sm, nullptr, nullptr, true));
     p.polish = (o.shift_polish > 0 && dim <= 32) ? align256((size_t)N * dim * 2 * sizeof(double)) : 0;
-    p.total = p.fused + p.polish;
+    p.flist = flist_bytes(dim, N);
+    p.total = p.fused + p.polish + p.flist;
     return p;
 }
 
@@ -946,7 +974,8 @@ int ves_eigensolve_shifts(int dim, int block_cnt, int thread_cnt, const double *
         a.iS = iP;
         a.shift_polish = 0;
     }
-    return native(cuda_ok(ves::launch_fused_fp64(a, st), "learned-shift solve launch"));
+    int *fcount = reinterpret_cast<int *>(static_cast<char *>(ws) + plan.fused + plan.polish);
+    return native(cuda_ok(ves::launch_shifts(a, fcount + 64, fcount, st), "learned-shift solve launch"));
 }
 
 int ves_gemm_bf16(int M, int N, int K, const void *A, int lda, const void *Bt, int ldb, const float *bias, int act,

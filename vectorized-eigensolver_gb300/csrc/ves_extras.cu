@@ -30,18 +30,20 @@ __device__ __forceinline__ long long soa_off(long long m, long long len, int tc)
 // Eigenvalues only.  Workspace per warp: H (n*n) and tau (n), double2.
 __global__ void __launch_bounds__(kThreads) eigvals_fp64_kernel(const Geom g, const double *rA, const double *iA,
                                                                 double *rE, double *iE, int *status_out,
-                                                                int *sweeps_out, void *ws, int max_its)
+                                                                int *sweeps_out, void *ws, int max_its,
+                                                                const int *list, const int *list_count)
 {
     const int n = g.n, tc = g.tc, lane = threadIdx.x & 31;
     const long long slot = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const long long nslots = (long long)gridDim.x * (kThreads / 32);
-    const long long ngroups = (g.N + 31) / 32;
+    const long long Nw = list ? (long long)*list_count : g.N;
+    const long long ngroups = (Nw + 31) / 32;
     double2 *base = reinterpret_cast<double2 *>(ws) + slot * ((long long)n * n + n) * 32 + lane;
     const MatIlv<double> H{base, n};
     const VecIlv<double> W{base + (long long)n * n * 32};
     for (long long gr = slot; gr < ngroups; gr += nslots) {
-        const long long m = gr * 32 + lane;
-        const bool valid = m < g.N;
+        const bool valid = gr * 32 + lane < Nw;
+        const long long m = !valid ? 0 : list ? (long long)list[gr * 32 + lane] : gr * 32 + lane;
         const long long mo = valid ? soa_off(m, (long long)n * n, tc) : 0;
         const long long vo = valid ? soa_off(m, n, tc) : 0;
         int status = 0, sweeps = 0;
@@ -191,13 +193,16 @@ size_t eigvals_workspace_bytes(int n, long long N, int blocks_per_sm)
     return (size_t)persistent_blocks(n, N, blocks_per_sm) * 4 * ((size_t)n * n + n) * 32 * sizeof(double2);
 }
 
+int eigvals_blocks(int n, long long N, int blocks_per_sm) { return (int)persistent_blocks(n, N, blocks_per_sm); }
+
 cudaError_t launch_eigvals(Geom g, const double *rA, const double *iA, double *rE, double *iE, int *status,
-                           int *sweeps, void *ws, int max_its, int blocks_per_sm, cudaStream_t st)
+                           int *sweeps, void *ws, int max_its, int blocks_per_sm, const int *list,
+                           const int *list_count, cudaStream_t st)
 {
     if (g.N <= 0) return cudaSuccess;
     eigvals_fp64_kernel<<<(unsigned)persistent_blocks(g.n, g.N, blocks_per_sm), kThreads, 0, st>>>(g, rA, iA, rE, iE,
                                                                                               status, sweeps, ws,
-                                                                               max_its);
+                                                                               max_its, list, list_count);
     return cudaGetLastError();
 }
 

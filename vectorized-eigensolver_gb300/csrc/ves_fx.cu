@@ -1,0 +1,216 @@
+// ves_fx.cu -- kernels of the fixed-point FP64 solve (ves_fx.cuh): fixed-size
+// batches, with and without eigenvectors, optionally over a device list.
+#include "ves_fx.cuh"
+#include "ves_internal.h"
+
+#include <algorithm>
+#include <cstdlib>
+
+namespace ves {
+
+namespace {
+
+template <int G> struct FxShape {
+    static constexpr int threads = G > 32 ? G : 32;
+    static constexpr int mats = G < 32 ? 32 / G : 1;  // matrices per block
+};
+
+template <int G, bool kVec>
+__global__ void __launch_bounds__(FxShape<G>::threads) fx_kernel(const FxArgs a)
+{
+    extern __shared__ longlong2 fxsm[];
+    const FxGroup<G> gr;
+    constexpr int M = FxShape<G>::mats;
+    const int n = a.g.n, tc = a.g.tc;
+    longlong2 *sm = fxsm + (G < 32 ? (threadIdx.x / G) * fx_slot(n, G, kVec) : 0);
+    const int lda = fx_lda(n);
+    const FxMat<1> H{sm, lda, n}, Z{sm + (kVec ? n * lda : 0), lda, n};
+    const FxVec<1> U{sm + (kVec ? 2 : 1) * n * lda};
+    const long long Nw = a.list ? (long long)*a.list_count : a.g.N;
+    for (long long base = (long long)blockIdx.x * M; base < Nw; base += (long long)gridDim.x * M) {
+        const long long w = base + (G < 32 ? threadIdx.x / G : 0);
+        const bool valid = w < Nw;
+        const long long m = !valid ? 0 : a.list ? (long long)a.list[w] : a.m_begin + w;
+        const long long mo = (m / tc) * (long long)tc * n * n + m % tc, vo = (m / tc) * (long long)tc * n + m % tc;
+        FxOut o{a.rE + vo, a.iE + vo, nullptr, nullptr, nullptr, nullptr, tc, tc};
+        if (kVec) {
+            o.rV = a.rV + mo;
+            o.iV = a.iV + mo;
+            if (a.rT) { o.rT = a.rT + mo; o.iT = a.iT + mo; }
+        }
+        int sweeps = 0, status = 0;
+        const bool ok = fx_solve<G, kVec>(gr, n, H, Z, U, valid, a.rA + mo, a.iA + mo, tc, o, a.max_its,
+                                          a.vnorm, sweeps, status);
+        if (valid && gr.gl == 0) {
+            if (ok) {
+                if (a.status) a.status[m] = status | a.status_or;
+                if (a.sweeps) a.sweeps[m] = sweeps;
+            } else {
+                a.out_list[atomicAdd(a.out_count, 1)] = (int)m;
+            }
+        }
+    }
+}
+
+// One matrix per lane, 32 in lockstep, H, Z and U in the warp's workspace
+// ([element][lane], as in the FP64 lane kernel): the FP64 steps of a rotation
+// serve 32 matrices per instruction.
+constexpr int kLaneThreads = 128;
+// kShifts: with predicted shifts, whose storage follows U in the slot.
+template <bool kVec, bool kShifts>
+__device__ __forceinline__ void fx_lanes(const FxArgs &a)
+{
+    __shared__ longlong2 chs[kLaneThreads * kFxChunk];
+    __shared__ i64 chi[kLaneThreads * kFxChunk];
+    const FxGroup<1> gr;
+    const int n = a.g.n, tc = a.g.tc, lane = threadIdx.x & 31;
+    const int ch0 = (threadIdx.x >> 5) * 32 * kFxChunk + lane;
+    const FxChunk ch{chs + ch0, chi + ch0};
+    const long long slot = (long long)blockIdx.x * (kLaneThreads / 32) + (threadIdx.x >> 5);
+    const long long nslots = (long long)gridDim.x * (kLaneThreads / 32);
+    const long long nn = (long long)n * n, nu = (kVec ? 2 : 1) * nn;
+    longlong2 *base = static_cast<longlong2 *>(a.ws) + slot * (kShifts ? shift_slot_elems(n) : nu + n) * 32 + lane;
+    const FxMat<32> H{base, n, n}, Z{base + (kVec ? nn * 32 : 0), n, n};
+    const FxVec<32> U{base + nu * 32};
+    const long long Nw = a.list ? (long long)*a.list_count : a.g.N;
+    for (long long base_w = slot * 32; base_w < Nw; base_w += nslots * 32) {
+        const long long w = base_w + lane;
+        const bool valid = w < Nw;
+        const long long m = !valid ? 0 : a.list ? (long long)a.list[w] : a.m_begin + w;
+        const long long mo = (m / tc) * (long long)tc * n * n + m % tc, vo = (m / tc) * (long long)tc * n + m % tc;
+        FxOut o{a.rE + vo, a.iE + vo, nullptr, nullptr, nullptr, nullptr, tc, tc};
+        if (kVec) {
+            o.rV = a.rV + mo;
+            o.iV = a.iV + mo;
+            if (a.rT) { o.rT = a.rT + mo; o.iT = a.iT + mo; }
+        }
+        int sweeps = 0, status = 0;
+        bool ok;
+        if constexpr (kShifts) {
+            FxShifts sh;
+            float2 *const region = reinterpret_cast<float2 *>(base - lane + (nu + n) * 32);
+            sh.Hf = MatIlv<float>{region + lane, n};
+            sh.P = VecIlv<double>{reinterpret_cast<double2 *>(base + (nu + n + (nn + 1) / 2) * 32)};
+            sh.scratch = n >= 6 ? Z.p : base + (shift_slot_elems(n) - 6 * n) * 32;
+            sh.polish = a.shift_polish;
+            sh.newton = a.shift_newton64;
+            sh.sweeps_used = a.shift_sweeps;
+            sh.gate = a.shift_gate;
+            for (int k = 1; k <= n; ++k)
+                sh.P.st(k, valid ? mk(a.rS[vo + (long long)(k - 1) * tc], a.iS[vo + (long long)(k - 1) * tc]) : mk(0.0, 0.0));
+            ok = fx_solve<1, kVec>(gr, n, H, Z, U, valid, a.rA + mo, a.iA + mo, tc, o, a.max_its, a.vnorm, sweeps,
+                                   status, ch, &sh);
+            if (sh.sp.fallbacks) status |= ST_SHIFT_FALLBACK;
+            if (ok && a.fallbacks) a.fallbacks[m] = sh.sp.fallbacks;
+        } else {
+            ok = fx_solve<1, kVec>(gr, n, H, Z, U, valid, a.rA + mo, a.iA + mo, tc, o, a.max_its, a.vnorm, sweeps,
+                                   status, ch);
+        }
+        if (valid) {
+            if (ok) {
+                if (a.status) a.status[m] = status | a.status_or;
+                if (a.sweeps) a.sweeps[m] = sweeps;
+            } else {
+                a.out_list[atomicAdd(a.out_count, 1)] = (int)m;
+            }
+        }
+    }
+}
+template <bool kVec> __global__ void __launch_bounds__(kLaneThreads, 4) fx_lane_kernel(const FxArgs a)
+{
+    fx_lanes<kVec, false>(a);
+}
+__global__ void __launch_bounds__(kLaneThreads, 4) fx_shifts_kernel(const FxArgs a) { fx_lanes<true, true>(a); }
+
+int fx_sms()
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
+
+template <int G> size_t fx_smem(int n, bool vec) { return (size_t)FxShape<G>::mats * fx_slot(n, G, vec) * sizeof(longlong2); }
+constexpr size_t kMaxSmem = 227 * 1024;
+
+template <int G, bool kVec> cudaError_t launch_fx_g(const FxArgs &a, cudaStream_t st)
+{
+    const size_t smem = fx_smem<G>(a.g.n, kVec);
+    if (smem > kMaxSmem) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(fx_kernel<G, kVec>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 1;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fx_kernel<G, kVec>, FxShape<G>::threads, smem);
+    if (e != cudaSuccess) return e;
+    const long long need = (a.g.N + FxShape<G>::mats - 1) / FxShape<G>::mats;
+    const long long blocks = std::min<long long>(need, (long long)fx_sms() * std::max(per_sm, 1));
+    fx_kernel<G, kVec><<<(unsigned)std::max<long long>(blocks, 1), FxShape<G>::threads, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <bool kVec> cudaError_t launch_fx_v(const FxArgs &a, int G, cudaStream_t st)
+{
+    switch (G) {
+    case 1: return launch_fx_g<1, kVec>(a, st);
+    case 2: return launch_fx_g<2, kVec>(a, st);
+    case 4: return launch_fx_g<4, kVec>(a, st);
+    case 8: return launch_fx_g<8, kVec>(a, st);
+    case 16: return launch_fx_g<16, kVec>(a, st);
+    case 32: return launch_fx_g<32, kVec>(a, st);
+    case 64: return launch_fx_g<64, kVec>(a, st);
+    default: return launch_fx_g<128, kVec>(a, st);
+    }
+}
+
+}  // namespace
+
+// Lanes per matrix: 0 = the lane kernel, whose 32 matrices share every FP64
+// instruction, once a batch is large enough to fill it; below, a group of
+// lanes per matrix in shared memory, more of them for fewer matrices.
+int fx_group_size(int n, long long N, bool vec)
+{
+    if (const char *e = getenv("VES_FX_LANES")) {  // tuning
+        const int v = atoi(e);
+        if (v >= 0 && v <= 128 && (v & (v - 1)) == 0) return v;
+    }
+    if (N > 6000) return 0;
+    return n <= 8 ? 8 : n <= 24 ? 16 : n <= 32 ? 32 : n <= 48 ? 64 : 128;
+}
+
+cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, cudaStream_t st)
+{
+    if (vec) fx_lane_kernel<true><<<a.lane_blocks, kLaneThreads, 0, st>>>(a);
+    else fx_lane_kernel<false><<<a.lane_blocks, kLaneThreads, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fx_shifts(const FxArgs &a, cudaStream_t st)
+{
+    fx_shifts_kernel<<<a.lane_blocks, kLaneThreads, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fx(const FxArgs &a, bool vec, cudaStream_t st)
+{
+    if (a.g.N <= 0) return cudaSuccess;
+    if (!fx_order(a.g.n)) return cudaErrorInvalidValue;
+    const int G = fx_group_size(a.g.n, a.g.N, vec);
+    if (G == 0) return launch_fx_lanes(a, vec, st);
+    return vec ? launch_fx_v<true>(a, G, st) : launch_fx_v<false>(a, G, st);
+}
+
+template <int G> static void load_fx_g()
+{
+    load_kernel(fx_kernel<G, true>);
+    load_kernel(fx_kernel<G, false>);
+}
+void load_fx_kernels()
+{
+    load_kernel(fx_lane_kernel<true>);
+    load_kernel(fx_lane_kernel<false>);
+    load_kernel(fx_shifts_kernel);
+    load_fx_g<1>(); load_fx_g<2>(); load_fx_g<4>(); load_fx_g<8>(); load_fx_g<16>(); load_fx_g<32>(); load_fx_g<64>();
+    load_fx_g<128>();
+}
+
+}  // namespace ves

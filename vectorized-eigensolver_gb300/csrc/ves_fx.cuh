@@ -1,0 +1,1117 @@
+// ves_fx.cuh -- the FP64 solver's unitary transformations in 64-bit fixed
+// point on the integer pipe.
+//
+// Why.  GB300 retires 1.8 FP64 FMAs per clock and SM but about 26 32x32+64-bit
+// integer multiply-adds (IMAD.WIDE).  The Hessenberg reduction and the QR
+// sweeps only apply unitary transformations, under which no entry of the
+// matrix can grow past ||A||_F, so one scale per matrix is enough and the
+// exponent that a floating-point format carries per number is not needed.  A
+// complex rotation of a pair of entries takes 36 IMAD.WIDE here: 0.71 pairs
+// per clock and SM measured, against 0.14 as 12 FP64 instructions.
+//
+// Format.  H is held in units of 2^(e-61), 2^e >= ||A||_F, so |entry| <= 2^61;
+// Q, Z and the Householder vectors in units of 2^-61, rotation coefficients in
+// units of 2^-62.  A product of two such numbers is formed from 32-bit halves
+// (signed high half, signed low half), leaving out low x low, and is rounded
+// to one unit: an absolute error of about 2^-61 ||A||_F per operation, against
+// 2^-53 |entry| in FP64, where the entries of an n x n matrix are of size
+// ||A||_F / n: for n <= 64 the fixed-point transformation is the more accurate
+// one.  Rotations and reflectors are computed in FP64 (53 bits), as before.
+// Sums of products are exact modulo 2^64 until they are rounded, so a result
+// does not depend on how a sum is spread over lanes: every kernel that uses
+// these routines, with any number of lanes per matrix, gives the same bits.
+//
+// One scale per matrix means errors relative to the whole matrix.  FP64 can do
+// better on a matrix whose rows, columns or blocks differ widely in size, and
+// there this form is not used: a matrix goes to the FP64 kernels when a row or
+// column has no entry above 2^-9 of the scale, when its Hessenberg form has a
+// subdiagonal below 2^-30 of the scale (it is numerically reducible: blocks
+// that may differ in size), or when it is zero, not finite or of an extreme
+// exponent.  The rule uses integer comparisons of the matrix alone, so every
+// kernel sends the same matrices the same way.
+#pragma once
+
+#include "ves_device.cuh"
+
+namespace ves {
+
+typedef long long i64;
+
+struct fx { int h, l; };  // value = h 2^32 + l, both signed
+struct cfx { fx r, i; };
+struct cx64 { i64 r, i; };
+
+__device__ __forceinline__ fx fx_split(i64 x)
+{
+    fx f;
+    f.l = (int)x;
+    f.h = (int)(x >> 32) + (int)((unsigned)f.l >> 31);
+    return f;
+}
+__device__ __forceinline__ cfx fx_split(cx64 z) { return {fx_split(z.r), fx_split(z.i)}; }
+// a b + c as one IMAD.WIDE (written as PTX: from C the compiler also emits
+// a multiply and an add, which doubled the instructions of a rotation)
+__device__ __forceinline__ i64 wide(int a, int b, i64 c)
+{
+#ifdef __CUDA_ARCH__
+    i64 d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+#else
+    return (i64)a * b + c;
+#endif
+}
+
+// Sum of products in units of (unit a)(unit b): c carries the cross halves
+// (weight 2^32) with the rounding constant, a the high halves (weight 2^64).
+struct facc { i64 c, a; };
+template <int SH> __device__ __forceinline__ facc fx_zero() { return {1LL << (SH - 33), 0}; }
+__device__ __forceinline__ void fx_mac(facc &s, fx a, fx b)
+{
+    s.c = wide(a.h, b.l, s.c);
+    s.c = wide(a.l, b.h, s.c);
+    s.a = wide(a.h, b.h, s.a);
+}
+// keeps the cross sum small: |c| < 2^63 holds for 8 products of vectors whose
+// norms are at most 2^61 and sqrt(2) 2^61 (4 complex terms)
+__device__ __forceinline__ void fx_flush(facc &s)
+{
+    s.a += s.c >> 32;
+    s.c = (i64)(unsigned)s.c;
+}
+// The sum (t 2^64 + low half of c 2^32) / 2^SH.
+template <int SH> __device__ __forceinline__ i64 fx_join(const i64 c, const i64 t)
+{
+    const unsigned lo = __funnelshift_l((unsigned)c, (unsigned)t, 64 - SH);
+    const unsigned hi = __funnelshift_l((unsigned)t, (unsigned)(t >> 32), 64 - SH);
+    return (i64)(((unsigned long long)hi << 32) | lo);
+}
+template <int SH> __device__ __forceinline__ i64 fx_end(const facc s)
+{
+    return fx_join<SH>(s.c, s.a + (s.c >> 32));
+}
+// Two and three products, the cross halves first: their carry starts the sum
+// of the high halves.
+template <int SH> __device__ __forceinline__ i64 fx_dot2(fx a, fx x, fx b, fx y)
+{
+    i64 c = 1LL << (SH - 33);
+    c = wide(a.h, x.l, c);
+    c = wide(a.l, x.h, c);
+    c = wide(b.h, y.l, c);
+    c = wide(b.l, y.h, c);
+    i64 t = c >> 32;
+    t = wide(a.h, x.h, t);
+    t = wide(b.h, y.h, t);
+    return fx_join<SH>(c, t);
+}
+__device__ __forceinline__ i64 fx_dot3(fx a, fx x, fx b, fx y, fx p, fx z)
+{
+    i64 c = 1LL << 29;
+    c = wide(a.h, x.l, c);
+    c = wide(a.l, x.h, c);
+    c = wide(b.h, y.l, c);
+    c = wide(b.l, y.h, c);
+    c = wide(p.h, z.l, c);
+    c = wide(p.l, z.h, c);
+    i64 t = c >> 32;
+    t = wide(a.h, x.h, t);
+    t = wide(b.h, y.h, t);
+    t = wide(p.h, z.h, t);
+    return fx_join<62>(c, t);
+}
+
+// Matrix and vector accessors, 1-based; element e of a matrix or vector at
+// p + e * ST: ST = 1 in shared memory, 32 in a warp's workspace (one matrix
+// per lane, a warp's copies of one element contiguous).
+template <int ST> struct FxMat {
+    longlong2 *p;
+    int lda, n;
+    __device__ __forceinline__ longlong2 *at(int i, int j) const
+    {
+        VES_CHECK_IJ(i, j, n);
+        return p + ((i - 1) + (j - 1) * lda) * ST;
+    }
+    __device__ __forceinline__ cx64 ld(int i, int j) const { const longlong2 v = *at(i, j); return {v.x, v.y}; }
+    __device__ __forceinline__ void st(int i, int j, cx64 v) const { *at(i, j) = make_longlong2(v.r, v.i); }
+    __device__ __forceinline__ cx<double> ldd(int i, int j) const
+    {
+        const double2 v = *reinterpret_cast<const double2 *>(at(i, j));
+        return mk(v.x, v.y);
+    }
+    __device__ __forceinline__ void std(int i, int j, cx<double> v) const
+    {
+        *reinterpret_cast<double2 *>(at(i, j)) = make_double2(v.r, v.i);
+    }
+};
+template <int ST> struct FxVec {
+    longlong2 *p;
+    __device__ __forceinline__ longlong2 *at(int k) const
+    {
+        VES_CHECK_I(k);
+        return p + (k - 1) * ST;
+    }
+    __device__ __forceinline__ cx64 ld(int k) const { const longlong2 v = *at(k); return {v.x, v.y}; }
+    __device__ __forceinline__ void st(int k, cx64 v) const { *at(k) = make_longlong2(v.r, v.i); }
+    __device__ __forceinline__ cx<double> ldd(int k) const
+    {
+        const double2 v = *reinterpret_cast<const double2 *>(at(k));
+        return mk(v.x, v.y);
+    }
+    __device__ __forceinline__ void std(int k, cx<double> v) const
+    {
+        *reinterpret_cast<double2 *>(at(k)) = make_double2(v.r, v.i);
+    }
+};
+
+__device__ __forceinline__ cx<double> fx_d(cx64 z) { return mk((double)z.r, (double)z.i); }
+__device__ __forceinline__ i64 fx_abs(i64 x) { return x < 0 ? -x : x; }
+__device__ __forceinline__ i64 fx_abs1(cx64 z) { return fx_abs(z.r) + fx_abs(z.i); }
+
+// Rotation [c s; -conj(s) c], c real: in FP64, and in units of 2^-62.
+struct FxRot {
+    double dc;
+    cx<double> ds;
+    i64 c, sr, si;
+};
+struct FxCoef {
+    fx c, sr, nsr, si, nsi;
+    __device__ __forceinline__ FxCoef(i64 ic, i64 isr, i64 isi)
+        : c(fx_split(ic)), sr(fx_split(isr)), nsr(fx_split(-isr)), si(fx_split(isi)), nsi(fx_split(-isi))
+    {
+    }
+    __device__ __forceinline__ explicit FxCoef(const FxRot &q) : FxCoef(q.c, q.sr, q.si) {}
+};
+
+__device__ __forceinline__ cx64 fx_i(cx<double> z) { return {__double2ll_rn(z.r), __double2ll_rn(z.i)}; }
+
+// The rotation that maps (x0, x1) to (r, 0), from one reciprocal square root:
+// with f = |x0|^2, g = |x1|^2, p = 1 / sqrt(f (f + g)): c = f p,
+// s = x0 conj(x1) p, r = x0 (f + g) p.
+__device__ __forceinline__ FxRot fx_rot(const cx<double> x0, const cx<double> x1, cx<double> &r)
+{
+    const double one = 4611686018427387904.0;  // 2^62
+    const double f = fma(x0.r, x0.r, x0.i * x0.i), g = fma(x1.r, x1.r, x1.i * x1.i);
+    const double n2 = f + g, w = f * n2;
+    const bool deg = !(w > 1e-280);  // x0 = 0 (or both far below one unit)
+    const double p = rsqrt(deg ? fmax(g, 1e-280) : w);
+    const double a = deg ? 1.0 : x0.r, b = deg ? 0.0 : x0.i;
+    FxRot q;
+    q.dc = deg ? 0.0 : f * p;
+    q.ds = mk(fma(a, x1.r, b * x1.i) * p, fma(b, x1.r, -(a * x1.i)) * p);
+    if (deg && !(g > 1e-280)) { q.dc = 1.0; q.ds = mk(0.0, 0.0); }
+    const double np = deg ? g * p : n2 * p;
+    r = mk(a * np, b * np);
+    const cx64 s = fx_i(cscal(q.ds, one));
+    q.c = __double2ll_rn(q.dc * one);
+    q.sr = s.r;
+    q.si = s.i;
+    return q;
+}
+
+// Rotate the pair (x1, x2): x1' = c x1 + s x2, x2' = c x2 - conj(s) x1 (rows of
+// H), with conj(s) for s on columns (kCol).
+template <bool kCol> __device__ __forceinline__ void fx_pair(cx64 &x1, cx64 &x2, const FxCoef &q)
+{
+    const fx si = kCol ? q.nsi : q.si, nsi = kCol ? q.si : q.nsi;
+    const cfx a = fx_split(x1), b = fx_split(x2);
+    x1.r = fx_dot3(q.c, a.r, q.sr, b.r, nsi, b.i);
+    x1.i = fx_dot3(q.c, a.i, q.sr, b.i, si, b.r);
+    x2.r = fx_dot3(q.c, b.r, q.nsr, a.r, nsi, a.i);
+    x2.i = fx_dot3(q.c, b.i, q.nsr, a.i, si, a.r);
+}
+
+// Wilkinson's shift of the trailing 2 x 2 block [a b; c d] (any phases) in
+// FP64, in the units of H: t = d - bc / (x + y), x = (a - d) / 2,
+// y = sqrt(x^2 + bc) on x's side.  Entries are integers up to 2^61: nothing
+// here overflows or underflows, so no scaling is needed.
+__device__ __forceinline__ cx<double> fx_wilkinson(const cx<double> a, const cx<double> b, const cx<double> c,
+                                                   const cx<double> d)
+{
+    const cx<double> bc = cmul(b, c);
+    const cx<double> x = cscal(csub(a, d), 0.5);
+    const cx<double> z = cadd(cmul(x, x), bc);
+    const double n2 = fma(z.r, z.r, z.i * z.i);
+    cx<double> y = mk(0.0, 0.0);
+    if (n2 > 0.0) {
+        const double az = n2 * rsqrt(n2);
+        const double h = 0.5 * (az + fabs(z.r));
+        const double rh = rsqrt(h), zr = h * rh, zi = 0.5 * fabs(z.i) * rh;
+        y = z.r < 0.0 ? mk(zi, zr) : mk(zr, zi);
+        if (z.i < 0.0) y.i = -y.i;
+    }
+    if (fma(x.r, y.r, x.i * y.i) < 0.0) y = mk(-y.r, -y.i);
+    const cx<double> v = cadd(x, y);
+    const double v2 = fma(v.r, v.r, v.i * v.i);
+    if (!(v2 > 0.0)) return d;
+    return csub(d, cscal(cmulc(bc, v), 1.0 / v2));
+}
+
+// Is the subdiagonal H(K, K-1) = S(K-1) negligible?  The reference's test
+// (Toolbox.hpp:810-867: |h| <= ulp (|h_kk| + |h_k-1,k-1|) and the Ahues-
+// Tisseur condition, multiplied through by its denominator) in FP32, which
+// moves the thresholds by a few 2^-23; anything below half a unit is
+// negligible too.  The reference keeps subdiagonals real by a diagonal phase
+// similarity: there H(K, K-1) is |s| and H(K-1, K) is turned by the phase of s.
+__device__ __forceinline__ float fx_absf(cx<double> z)
+{
+    const float r = (float)z.r, i = (float)z.i;
+    return sqrtf(fmaf(r, r, i * i));
+}
+template <int ST>
+__device__ __forceinline__ bool fx_negligible(const FxMat<ST> &H, const FxVec<ST> &S, const int K, const int n)
+{
+    const cx<double> s = S.ldd(K - 1);
+    const cx64 d1 = H.ld(K - 1, K - 1), d2 = H.ld(K, K);
+    const float sr = (float)s.r, si = (float)s.i, hk = sqrtf(fmaf(sr, sr, si * si));
+    if (hk <= 0.5f) return true;
+    float tst = (float)(fx_abs1(d1) + fx_abs1(d2));
+    if (tst == 0.f) {
+        if (K - 2 >= 1) tst += fx_absf(S.ldd(K - 2));
+        if (K + 1 <= n) tst += fx_absf(S.ldd(K));
+    }
+    if (hk > 0x1p-52f * tst) return false;
+    const cx64 u = H.ld(K - 1, K);
+    const float ur = (float)u.r, ui = (float)u.i, ih = 1.f / hk, pr = sr * ih, pi = si * ih;
+    const float up = fabsf(ur * pr - ui * pi) + fabsf(ur * pi + ui * pr);
+    const float kk = (float)fx_abs1(d2), df = (float)fx_abs1({d1.r - d2.r, d1.i - d2.i});
+    return fminf(hk, up) * fmaxf(hk, up) <= 0x1p-52f * fminf(kk, df) * fmaxf(kk, df);
+}
+
+// A group of G lanes that owns one matrix: part of a warp (G < 32), a warp, or
+// a block of G threads.  Reductions run over RG lanes, in a block of several
+// warps redundantly in each of them.
+template <int G> struct FxGroup {
+    static constexpr int RG = G < 32 ? G : 32;
+    int gl, rl, shift;
+    unsigned mask;
+    __device__ __forceinline__ FxGroup()
+    {
+        const int lane = threadIdx.x & 31;
+        gl = threadIdx.x & (G - 1);
+        rl = gl & (RG - 1);
+        shift = lane & ~(RG - 1);
+        mask = RG == 32 ? FULL : ((1u << (RG & 31)) - 1u) << shift;
+    }
+    __device__ __forceinline__ void sync() const
+    {
+        if (G > 32) __syncthreads();
+        else if (G > 1) __syncwarp(mask);
+    }
+    // lanes of the group (from the lowest) with p
+    __device__ __forceinline__ unsigned ballot(bool p) const
+    {
+        return RG == 1 ? (unsigned)p : __ballot_sync(mask, p) >> shift;
+    }
+    __device__ __forceinline__ bool all(bool p) const { return ballot(!p) << (32 - RG) == 0; }
+    __device__ __forceinline__ i64 sum(i64 v) const
+    {
+#pragma unroll
+        for (int o = RG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+    __device__ __forceinline__ i64 orr(i64 v) const
+    {
+#pragma unroll
+        for (int o = RG / 2; o > 0; o >>= 1) v |= __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+    __device__ __forceinline__ int maxi(int v) const
+    {
+#pragma unroll
+        for (int o = RG / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(mask, v, o));
+        return v;
+    }
+};
+
+__host__ __device__ __forceinline__ int fx_lda(int n) { return n | 1; }
+// 16-byte elements of a matrix's slot in shared memory: H, Z (vectors only),
+// and n entries for the reflectors' first elements and the column scales;
+// padded so that the slots of a warp's matrices start G elements apart modulo
+// 8 (eight lanes' 16-byte accesses fill the banks once).
+__host__ __device__ __forceinline__ int fx_slot(int n, int G, bool vec)
+{
+    int e = (vec ? 2 : 1) * n * fx_lda(n) + n;
+    if (G < 8) e += ((G - e % 8) + 8) % 8;
+    return e;
+}
+
+// Row and column of element e = i - 1 + (j - 1) n, advanced without a division.
+struct FxIndex {
+    int i, j;
+    __device__ __forceinline__ FxIndex(int e, int n) : i(e % n + 1), j(e / n + 1) {}
+    __device__ __forceinline__ void next(int step, int n)
+    {
+        for (i += step; i > n; i -= n) ++j;
+    }
+};
+
+struct FxOut {
+    double *rE, *iE, *rV, *iV, *rT, *iT;
+    long long sv, sm;  // element strides of vectors and matrices
+};
+
+// Load A (element e of the column-major matrix at e * s) into H as integers.
+// Returns false for a matrix that is left to the FP64 kernels; unit = 2^(e-61).
+template <int G, int ST>
+__device__ __forceinline__ bool fx_load(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const bool valid,
+                                        const double *rA, const double *iA, const long long s, double &unit)
+{
+    unit = 1.0;
+    int emax = 0;
+    FxIndex i0(gr.gl, n);
+    for (int e = gr.gl; e < n * n; e += G, i0.next(G, n)) {
+        double re = 0.0, im = 0.0;
+        if (valid) { re = rA[e * s]; im = iA[e * s]; }
+        emax = max(emax, max(__double2hiint(re) & 0x7fffffff, __double2hiint(im) & 0x7fffffff));
+        H.std(i0.i, i0.j, mk(re, im));
+    }
+    gr.sync();
+    if (G > 32) {  // each warp reduces over the whole matrix
+        for (int e = gr.rl; e < n * n; e += 32) {
+            const cx<double> v = H.ldd(e % n + 1, e / n + 1);
+            emax = max(emax, max(__double2hiint(v.r) & 0x7fffffff, __double2hiint(v.i) & 0x7fffffff));
+        }
+    }
+    emax = gr.maxi(emax) >> 20;
+    const bool range = valid && emax >= 128 && emax <= 1900;
+    // ||A||_F^2 from above: |component| < (q + 1) 2^(emax - 1043), q its leading 21 bits
+    i64 q2 = 0;
+    FxIndex i1(gr.rl, n);
+    for (int e = gr.rl; e < n * n; e += FxGroup<G>::RG, i1.next(FxGroup<G>::RG, n)) {
+        const cx<double> v = H.ldd(i1.i, i1.j);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int hi = __double2hiint(c ? v.i : v.r) & 0x7fffffff, ex = hi >> 20;
+            const int q = ((hi & 0xfffff) | 0x100000) >> min(emax - ex, 31);
+            q2 += (i64)(q + 1) * (q + 1);
+        }
+    }
+    q2 = gr.sum(q2);
+    const int E = ((64 - __clzll(q2)) + 1) / 2 + emax - 1043;
+    gr.sync();  // every warp has read the matrix
+    if (range) {
+        const double sc = __hiloint2double((61 - E + 1023) << 20, 0);
+        unit = __hiloint2double((E - 61 + 1023) << 20, 0);
+        FxIndex i2(gr.gl, n);
+        for (int e = gr.gl; e < n * n; e += G, i2.next(G, n)) {
+            const cx<double> v = H.ldd(i2.i, i2.j);
+            H.st(i2.i, i2.j, {__double2ll_rn(v.r * sc), __double2ll_rn(v.i * sc)});
+        }
+    } else {
+        FxIndex i2(gr.gl, n);
+        for (int e = gr.gl; e < n * n; e += G, i2.next(G, n)) H.st(i2.i, i2.j, {0, 0});
+    }
+    gr.sync();
+    // every row and column has an entry of at least 2^-9 of the scale
+    bool ok = range;
+    for (int r = gr.rl + 1; r <= n; r += FxGroup<G>::RG) {
+        int mr = 0, mc = 0;
+        for (int j = 1; j <= n; ++j) {
+            const cx64 a = H.ld(r, j), b = H.ld(j, r);
+            mr = max(mr, max(abs((int)(a.r >> 32)), abs((int)(a.i >> 32))));
+            mc = max(mc, max(abs((int)(b.r >> 32)), abs((int)(b.i >> 32))));
+        }
+        ok = ok && mr >= (1 << 20) && mc >= (1 << 20);
+    }
+    return gr.all(ok);
+}
+
+// Householder reduction to Hessenberg form with Hermitian reflectors
+// P = I - u u^H, ||u||^2 = 2 (the subdiagonal comes out complex).  u_k, k >=
+// i + 2, stays below the subdiagonal of column i, u_{i+1} in U(i).
+template <int G, int ST>
+__device__ __forceinline__ void fx_reduce(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxVec<ST> &U)
+{
+    constexpr int RG = FxGroup<G>::RG;
+    for (int i = 1; i <= n - 2; ++i) {
+        const cx64 al = H.ld(i + 1, i);
+        i64 o = 0;
+        for (int k = i + 2 + gr.rl; k <= n; k += RG) { const cx64 x = H.ld(k, i); o |= fx_abs(x.r) | fx_abs(x.i); }
+        o = gr.orr(o);
+        // squared norm of the entries, to about 2^-55, as a sum of integers
+        const int sh = o ? __clzll(o) - 2 : 0;  // |x| << sh < 2^62
+        i64 q = 0;
+        for (int k = i + 2 + gr.rl; k <= n; k += RG) {
+            const cx64 x = H.ld(k, i);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const unsigned long long a = (unsigned long long)fx_abs(c ? x.i : x.r) << sh;
+                const unsigned long long hi = __umul64hi(a, a);
+                q += (i64)((hi + 4) >> 3);
+            }
+        }
+        q = gr.sum(q);
+        double scale = 0.0;  // u_k = x_k scale (units of 2^-61)
+        cx64 u1 = {0, 0}, beta = al;
+        if (o) {
+            // q 2^67 / 2^(2 sh); the sum is unsigned (up to 2^64)
+            const double xn2 = (double)(unsigned long long)q * __hiloint2double((67 - 2 * sh + 1023) << 20, 0);
+            const double one = 2305843009213693952.0;  // 2^61
+            const cx<double> a = fx_d(al);
+            const double a2 = fma(a.r, a.r, a.i * a.i), n2 = a2 + xn2;
+            const double ra = a2 > 0.0 ? rsqrt(a2) : 0.0;
+            const cx<double> ph = a2 > 0.0 ? mk(a.r * ra, a.i * ra) : mk(1.0, 0.0);
+            const double nrm = n2 * rsqrt(n2), s = fma(a2, ra, nrm);
+            const double r = rsqrt(nrm * s);
+            scale = r * one;
+            u1 = {__double2ll_rn(ph.r * (s * scale)), __double2ll_rn(ph.i * (s * scale))};
+            beta = {-__double2ll_rn(ph.r * nrm), -__double2ll_rn(ph.i * nrm)};
+        }
+        gr.sync();  // every lane has read column i
+        for (int k = i + 2 + gr.gl; k <= n; k += G) {
+            const cx64 x = H.ld(k, i);
+            H.st(k, i, {__double2ll_rn((double)x.r * scale), __double2ll_rn((double)x.i * scale)});
+        }
+        if (gr.gl == 0) {
+            U.st(i, u1);
+            H.st(i + 1, i, u1);  // so that u is column i from here on; beta at the end
+        }
+        gr.sync();
+        // right: row r of A(:, i+1:n) -= (A u)_r u^H
+        for (int r = gr.gl + 1; r <= n; r += G) {
+            facc sr = fx_zero<61>(), si = sr;
+            for (int k = i + 1; k <= n; ++k) {
+                const cfx u = fx_split(H.ld(k, i));
+                const cx64 x = H.ld(r, k);
+                const cfx a = fx_split(x);
+                const fx na = fx_split(-x.i);
+                fx_mac(sr, a.r, u.r);
+                fx_mac(sr, na, u.i);
+                fx_mac(si, a.r, u.i);
+                fx_mac(si, a.i, u.r);
+                if (((k - i) & 3) == 0) { fx_flush(sr); fx_flush(si); }
+            }
+            const cx64 y = {fx_end<61>(sr), fx_end<61>(si)};
+            const cfx ny = fx_split(cx64{-y.r, -y.i});
+            const fx yr = fx_split(y.r);
+            for (int k = i + 1; k <= n; ++k) {
+                const cfx u = fx_split(H.ld(k, i));
+                const cx64 x = H.ld(r, k);
+                H.st(r, k, {x.r + fx_dot2<61>(ny.r, u.r, ny.i, u.i), x.i + fx_dot2<61>(ny.i, u.r, yr, u.i)});
+            }
+        }
+        gr.sync();
+        // left: column c of A(i+1:n, i+1:n) -= u (u^H A)_c
+        for (int c = i + 1 + gr.gl; c <= n; c += G) {
+            facc sr = fx_zero<61>(), si = sr;
+            for (int k = i + 1; k <= n; ++k) {
+                const cx64 uk = H.ld(k, i);
+                const cfx u = fx_split(uk), a = fx_split(H.ld(k, c));
+                const fx nu = fx_split(-uk.i);
+                fx_mac(sr, u.r, a.r);
+                fx_mac(sr, u.i, a.i);
+                fx_mac(si, u.r, a.i);
+                fx_mac(si, nu, a.r);
+                if (((k - i) & 3) == 0) { fx_flush(sr); fx_flush(si); }
+            }
+            const cx64 z = {fx_end<61>(sr), fx_end<61>(si)};
+            const cfx nz = fx_split(cx64{-z.r, -z.i});
+            const fx zi = fx_split(z.i);
+            for (int k = i + 1; k <= n; ++k) {
+                const cfx u = fx_split(H.ld(k, i));
+                const cx64 x = H.ld(k, c);
+                H.st(k, c, {x.r + fx_dot2<61>(nz.r, u.r, zi, u.i), x.i + fx_dot2<61>(nz.i, u.r, nz.r, u.i)});
+            }
+        }
+        gr.sync();
+        if (gr.gl == 0) H.st(i + 1, i, beta);
+        gr.sync();
+    }
+}
+
+// Z = P_1 P_2 ... P_{n-2} from the reflectors.
+template <int G, int ST>
+__device__ __forceinline__ void fx_form_q(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
+                                          const FxVec<ST> &U)
+{
+    for (int c = gr.gl + 1; c <= n; c += G)
+        for (int r = 1; r <= n; ++r) Z.st(r, c, {r == c ? 1LL << 61 : 0, 0});
+    // a lane's columns are its own: no synchronisation between reflectors
+    for (int i = n - 2; i >= 1; --i) {
+        const cx64 u1 = U.ld(i);
+        for (int c = gr.gl + 1; c <= n; c += G) {
+            if (c < i + 1) continue;
+            facc sr = fx_zero<61>(), si = sr;
+            for (int k = i + 1; k <= n; ++k) {
+                const cx64 uk = k == i + 1 ? u1 : H.ld(k, i);
+                const cfx u = fx_split(uk), a = fx_split(Z.ld(k, c));
+                const fx nu = fx_split(-uk.i);
+                fx_mac(sr, u.r, a.r);
+                fx_mac(sr, u.i, a.i);
+                fx_mac(si, u.r, a.i);
+                fx_mac(si, nu, a.r);
+                if (((k - i) & 3) == 0) { fx_flush(sr); fx_flush(si); }
+            }
+            const cx64 z = {fx_end<61>(sr), fx_end<61>(si)};
+            const cfx nz = fx_split(cx64{-z.r, -z.i});
+            const fx zi = fx_split(z.i);
+            for (int k = i + 1; k <= n; ++k) {
+                const cfx u = fx_split(k == i + 1 ? u1 : H.ld(k, i));
+                const cx64 x = Z.ld(k, c);
+                Z.st(k, c, {x.r + fx_dot2<61>(nz.r, u.r, zi, u.i), x.i + fx_dot2<61>(nz.i, u.r, nz.r, u.i)});
+            }
+        }
+    }
+    gr.sync();
+}
+
+// no subdiagonal below 2^-30 of the scale
+template <int G, int ST>
+__device__ __forceinline__ bool fx_irreducible(const FxGroup<G> &gr, const int n, const FxMat<ST> &H)
+{
+    bool ok = true;
+    for (int k = gr.rl + 2; k <= n; k += FxGroup<G>::RG) ok = ok && fx_abs1(H.ld(k, k - 1)) >= (1LL << 31);
+    return gr.all(ok);
+}
+
+// Deflate at the bottom of the window [L, I] (the reference's test and sweep
+// cap, which moves on) until an eigenvalue needs a sweep; false when none is
+// left.  (a0, a1): the vector of the sweep's first rotation, from Wilkinson's
+// shift or, at the 10th and 20th sweep, the reference's exceptional ones.
+// sp: predicted shifts, in the units of H.
+template <int G, int ST, class SP = NoShiftPredictions>
+__device__ __forceinline__ bool fx_next_sweep(const FxGroup<G> &gr, const int n, const FxMat<ST> &H,
+                                              const FxVec<ST> &S, const int max_its, int &I, int &L, int &its,
+                                              int &status, cx<double> &a0, cx<double> &a1, SP *sp = nullptr)
+{
+    constexpr int RG = FxGroup<G>::RG;
+    for (;;) {
+        if (I <= 1) return false;
+        if (its > max_its) { status |= ST_ITCAP; --I; L = 1; its = 0; continue; }
+        // the largest K in (L, I] whose subdiagonal is negligible, else L
+        int K = L;
+        for (int top = I; top > L; top -= RG) {
+            const int k = top - gr.rl;
+            const unsigned b = gr.ballot(k > L && fx_negligible(H, S, k > L ? k : L + 1, n)) &
+                               (RG == 32 ? FULL : (1u << (RG & 31)) - 1u);
+            if (b) { K = top - (__ffs(b) - 1); break; }
+        }
+        L = K;
+        if (G > 32) __syncthreads();  // the scans have read S
+        if (L > 1) S.std(L - 1, mk(0.0, 0.0));  // every lane: the same value
+        if (L >= I) {
+            if (sp) sp->deflated(its);
+            --I; L = 1; its = 0;
+            continue;
+        }
+        const cx<double> hll = fx_d(H.ld(L, L));
+        a1 = S.ldd(L);
+        cx<double> t;
+        if (its == 10) t = mk(fma(0.75, cabs(a1), hll.r), hll.i);
+        else {
+            const cx<double> si = S.ldd(I - 1);
+            t = fx_d(H.ld(I, I));
+            if (its == 20) t.r = fma(0.75, cabs(si), t.r);
+            else t = fx_wilkinson(fx_d(H.ld(I - 1, I - 1)), fx_d(H.ld(I - 1, I)), si, t);
+        }
+        if (sp) sp->template pick<double>(its, I, t, cabs(S.ldd(I - 1)));
+        a0 = csub(hll, t);
+        ++its;
+        return true;
+    }
+}
+
+// Single-shift QR (reference Toolbox.hpp:690-1031): the same deflation test,
+// exceptional shifts and sweep cap as zlahqr_warp, with rotations of real
+// cosine, so the subdiagonals stay complex and need no phase fix.  The
+// matrices of a warp move in lockstep per sweep, each group with its own
+// window [L, I].  kVec = false: the active block only, no Z.
+//
+// The subdiagonals and the bulge stay in FP64 (S(k) = H(k+1, k)): they
+// become small against the matrix as the iteration converges, and the rotation
+// that a small pair defines must keep its relative accuracy for the shift to
+// reach the end of the window.  With them in fixed point (an absolute
+// rounding) the transformations are as accurate, but the subdiagonals stall at
+// 2^-46 of the matrix.  Every other entry is only rotated.
+template <int G, bool kVec, int ST>
+__device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z, const FxVec<ST> &S,
+                                      const bool run, const int max_its, int &sweeps, int &status)
+{
+    int I = n, L = 1, its = 0;
+    bool done = !run || n <= 1;
+    for (;;) {
+        cx<double> a0, a1, sub;  // the pair of the next rotation; H(K+1, K)
+        const bool sweep = !done && fx_next_sweep<G>(gr, n, H, S, max_its, I, L, its, status, a0, a1);
+        done = !sweep;
+        sub = a1;
+        sweeps += sweep;
+        int Kmin, Kmax;
+        if (G < 32) {
+            if (!__any_sync(FULL, sweep)) break;
+            Kmin = __reduce_min_sync(FULL, sweep ? L : INT_MAX);
+            Kmax = __reduce_max_sync(FULL, sweep ? I - 1 : 0);
+        } else {
+            if (!sweep) break;
+            Kmin = L;
+            Kmax = I - 1;
+        }
+        gr.sync();
+        if (G < 32) __syncwarp();
+        const int jmax = kVec ? n : I, jmin = kVec ? 1 : L;
+        for (int K = Kmin; K <= Kmax; ++K) {
+            if (sweep && K >= L && K < I) {
+                cx<double> r;
+                const FxRot R = fx_rot(a0, a1, r);
+                const FxCoef C(R);
+                const cx64 ssub = fx_i(sub);
+                const cx<double> hkk = fx_d(H.ld(K, K));
+                const cx<double> nxt = K + 1 < I ? S.ldd(K + 1) : mk(0.0, 0.0);  // H(K+2, K+1)
+                const cx<double> ks = conj(R.ds);
+                // H(K+1, K) after the row operation
+                const cx<double> x1 = cnmac(cscal(sub, R.dc), ks, hkk);
+                gr.sync();  // every lane has read H(K, K) and S
+                if (gr.gl == 0) {
+                    if (K > L) S.std(K - 1, r);
+                    if (K + 1 < I) S.std(K + 1, cscal(nxt, R.dc));
+                }
+                // rows K, K+1 of columns K..jmax; H(K+1, K) is the FP64 subdiagonal
+                for (int j = K + gr.gl; j <= jmax; j += G) {
+                    cx64 y1 = H.ld(K, j), y2 = H.ld(K + 1, j);
+                    if (j == K) y2 = ssub;
+                    fx_pair<false>(y1, y2, C);
+                    H.st(K, j, y1);
+                    if (j > K) H.st(K + 1, j, y2);
+                }
+                gr.sync();
+                // columns K, K+1 of H (rows up to K+1), then of Z
+                const cx<double> x2 = fx_d(H.ld(K + 1, K + 1));
+                const cx64 sx1 = fx_i(x1);
+                a0 = cmac(cscal(x1, R.dc), ks, x2);
+                a1 = cmul(ks, nxt);  // the bulge H(K+2, K)
+                sub = cscal(nxt, R.dc);
+                gr.sync();  // every lane has read H(K+1, K+1)
+                const int nc = K + 2 - jmin;
+                for (int q = gr.gl; q < nc + (kVec ? n : 0); q += G) {
+                    const bool h = !kVec || q < nc;
+                    const int row = h ? K + 1 - q : q - nc + 1;
+                    longlong2 *p1 = h ? H.at(row, K) : Z.at(row, K), *p2 = h ? H.at(row, K + 1) : Z.at(row, K + 1);
+                    const longlong2 w1 = *p1, w2 = *p2;
+                    cx64 y1 = {w1.x, w1.y}, y2 = {w2.x, w2.y};
+                    if (q == 0) y1 = sx1;
+                    fx_pair<true>(y1, y2, C);
+                    if (q != 0) *p1 = make_longlong2(y1.r, y1.i);
+                    *p2 = make_longlong2(y2.r, y2.i);
+                }
+                if (K == I - 1 && gr.gl == 0) S.std(I - 1, a0);
+                gr.sync();
+            }
+            if (G < 32) __syncwarp();
+        }
+    }
+}
+
+// Rotations of the current chunk of a sweep, in shared memory, one set per lane.
+constexpr int kFxChunk = 8;
+constexpr int kFxStream = 2;  // chains streamed together
+struct FxChunk {
+    longlong2 *cs;  // (c, sr) of rotation k at cs[k * 32]
+    i64 *si;
+    __device__ __forceinline__ void put(int k, const FxRot &q) const
+    {
+        cs[k * 32] = make_longlong2(q.c, q.sr);
+        si[k * 32] = q.si;
+    }
+    __device__ __forceinline__ FxCoef get(int k) const
+    {
+        const longlong2 a = cs[k * 32];
+        return FxCoef(a.x, a.y, si[k * 32]);
+    }
+};
+
+// Apply rotations k0 .. k0 + ns - 1 of the chunk to NB chains of entries: chain
+// b's entries at p + b blk + k step, rotation k on entries k and k + 1.  The
+// entry that two rotations share stays in registers, so each entry is read
+// and written once per chunk.
+template <int NB, bool kCol>
+__device__ __forceinline__ void fx_stream(longlong2 *p, const int step, const int blk, const FxChunk &ch,
+                                          const int k0, const int ns)
+{
+    cx64 x[NB];
+    longlong2 y[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const longlong2 v = p[b * blk];
+        x[b] = {v.x, v.y};
+        y[b] = p[b * blk + step];
+    }
+    for (int k = 0; k < ns; ++k) {
+        const FxCoef q = ch.get(k0 + k);
+        longlong2 *const p1 = p + step;
+        cx64 z[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            z[b] = {y[b].x, y[b].y};
+            if (k + 1 < ns) y[b] = p1[b * blk + step];  // the next rotation's entries
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            fx_pair<kCol>(x[b], z[b], q);
+            p[b * blk] = make_longlong2(x[b].r, x[b].i);
+            x[b] = z[b];
+        }
+        p = p1;
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) p[b * blk] = make_longlong2(x[b].r, x[b].i);
+}
+template <bool kCol>
+__device__ __forceinline__ void fx_stream_all(longlong2 *p, const int step, const int blk, const int count,
+                                              const FxChunk &ch, const int ns)
+{
+    int b = 0;
+    for (; b + kFxStream <= count; b += kFxStream) fx_stream<kFxStream, kCol>(p + b * blk, step, blk, ch, 0, ns);
+    for (; b < count; ++b) fx_stream<1, kCol>(p + b * blk, step, blk, ch, 0, ns);
+}
+
+// fx_qr for one matrix per lane, 32 in lockstep per sweep, in the warp's
+// workspace.  A sweep runs in chunks of kFxChunk rotations: first the chain of
+// rotations, which needs of the matrix only the chunk's own columns (the left
+// rotations of the chunk are applied to column K + 1 when rotation K is due)
+// and the diagonal; then the chunk's rotations are streamed over the rows of Z,
+// the rows above and the columns to the right.  A lane whose window does not
+// contain K takes part with the identity, which leaves integers unchanged.
+// The entries see the same operations as in fx_qr.
+template <bool kVec, class SP>
+__device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, const FxMat<32> &Z, const FxVec<32> &S,
+                                           const FxChunk &ch, const bool run, const int max_its, int &sweeps,
+                                           int &status, SP *sp)
+{
+    const FxGroup<1> gr;
+    const int rs = 32, cs = n * 32;  // steps to the next row, the next column
+    int I = n, L = 1, its = 0;
+    bool done = !run || n <= 1;
+    for (;;) {
+        cx<double> a0, a1, sub;
+        const bool sweep = !done && fx_next_sweep<1>(gr, n, H, S, max_its, I, L, its, status, a0, a1, sp);
+        done = !sweep;
+        sub = a1;
+        sweeps += sweep;
+        if (!__any_sync(FULL, sweep)) break;
+        const int Kmin = __reduce_min_sync(FULL, sweep ? L : INT_MAX);
+        const int Kmax = __reduce_max_sync(FULL, sweep ? I - 1 : 0);
+        cx64 hkk = {0, 0};
+        for (int Kc = Kmin; Kc <= Kmax; Kc += kFxChunk) {
+            const int Ke = min(Kc + kFxChunk - 1, Kmax), ns = Ke - Kc + 1;
+            for (int K = Kc; K <= Ke; ++K) {
+                const bool act = sweep && K >= L && K < I;
+                FxRot R;
+                R.dc = 1.0;
+                R.ds = mk(0.0, 0.0);
+                R.c = 1LL << 62;
+                R.sr = R.si = 0;
+                // column K + 1: the chunk's rotations so far
+                longlong2 *pc = H.at(Kc, K + 1);
+                longlong2 v = pc[0];
+                cx64 x = {v.x, v.y};
+                v = pc[rs];
+                cx<double> r, nxt = mk(0.0, 0.0);
+                if (act) {
+                    R = fx_rot(a0, a1, r);
+                    if (K == L) hkk = H.ld(K, K);
+                    if (K + 1 < I) nxt = S.ldd(K + 1);
+                }
+                ch.put(K - Kc, R);
+                for (int q = Kc; q < K; ++q) {
+                    cx64 y = {v.x, v.y};
+                    v = pc[2 * rs];
+                    fx_pair<false>(x, y, ch.get(q - Kc));
+                    pc[0] = make_longlong2(x.r, x.i);
+                    x = y;
+                    pc += rs;
+                }
+                const FxCoef C(R);
+                cx64 y = {v.x, v.y};
+                fx_pair<false>(x, y, C);
+                pc[0] = make_longlong2(x.r, x.i);
+                if (act) {
+                    // column K, then row K + 1 of the columns K, K + 1
+                    const cx<double> ks = conj(R.ds), dk = fx_d(hkk);
+                    const cx<double> x1 = cnmac(cscal(sub, R.dc), ks, dk);  // H(K+1, K) after the row operation
+                    cx64 y2 = fx_i(sub);
+                    fx_pair<false>(hkk, y2, C);
+                    H.st(K, K, hkk);
+                    if (K > L) S.std(K - 1, r);
+                    if (K + 1 < I) S.std(K + 1, cscal(nxt, R.dc));
+                    a0 = cmac(cscal(x1, R.dc), ks, fx_d(y));
+                    a1 = cmul(ks, nxt);  // the bulge H(K+2, K)
+                    sub = cscal(nxt, R.dc);
+                    cx64 z1 = fx_i(x1);
+                    fx_pair<true>(z1, y, C);
+                    hkk = y;
+                    if (K == I - 1) S.std(I - 1, a0);
+                }
+                H.st(K + 1, K + 1, y);
+            }
+            // rows above the chunk, then the chunk's own rows, whose first rotation is their own
+            const int r0 = kVec ? 1 : Kmin;
+            if (Kc > r0) fx_stream_all<true>(H.at(r0, Kc), cs, rs, Kc - r0, ch, ns);
+            for (int r = Kc; r <= Ke; ++r) fx_stream<1, true>(H.at(r, r), cs, rs, ch, r - Kc, Ke - r + 1);
+            if (kVec) fx_stream_all<true>(Z.at(1, Kc), cs, rs, n, ch, ns);
+            const int je = kVec ? n : Kmax + 1;
+            if (je > Ke + 1) fx_stream_all<false>(H.at(Kc, Ke + 2), rs, cs, je - Ke - 1, ch, ns);
+        }
+    }
+}
+
+// T-eigenvectors (ztrevc back substitution) on H converted to FP64, x of
+// column k in row k of H's lower triangle; then V = Z X in Z, in FP64.
+template <int G, int ST>
+__device__ __forceinline__ void fx_vectors(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
+                                           const FxVec<ST> &U)
+{
+    const double ulp = lim<double>::eps();
+    const int nsets = (n + G - 1) / G;
+    for (int t = 0; t < nsets; ++t) {
+        const int ki = t * G + gr.gl + 1, kmax = min(n, (t + 1) * G);
+        const bool own = ki <= n;
+        const cx<double> tkk = own ? H.ldd(ki, ki) : mk(0.0, 0.0);
+        // entries of T are integers: a difference is 0 or at least 1
+        const double smin = fmax(ulp * cabs1(tkk), 0.25);
+        double s = 1.0;
+        if (own)
+            for (int k = 1; k < ki; ++k) { const cx<double> v = H.ldd(k, ki); H.std(ki, k, mk(-v.r, -v.i)); }
+        for (int j = kmax - 1; j >= 1; --j) {
+            if (own && j < ki) {
+                cx<double> d = csub(H.ldd(j, j), tkk);
+                if (cabs1(d) < smin) d = mk(smin, 0.0);
+                cx<double> xj = H.ldd(ki, j);
+                // |x_j / d| about to exceed 1e150 (an exponent difference of 498): scale the vector
+                const int ex = max(__double2hiint(xj.r) & 0x7fffffff, __double2hiint(xj.i) & 0x7fffffff) >> 20;
+                const int ed = max(__double2hiint(d.r) & 0x7fffffff, __double2hiint(d.i) & 0x7fffffff) >> 20;
+                if (ex - ed > 497) {
+                    const double f = __hiloint2double((1023 - (ex - ed)) << 20, 0);
+                    for (int i = 1; i < ki; ++i) H.std(ki, i, cscal(H.ldd(ki, i), f));
+                    xj = cscal(xj, f);
+                    s *= f;
+                }
+                const double rd = 1.0 / fma(d.r, d.r, d.i * d.i);
+                xj = cscal(cmulc(xj, d), rd);
+                H.std(ki, j, xj);
+                for (int i = j - 1; i >= 1; --i) H.std(ki, i, cnmac(H.ldd(ki, i), H.ldd(i, j), xj));
+            }
+        }
+        if (own) U.std(ki, mk(s, 0.0));  // scale of the unit entry
+    }
+    gr.sync();
+    for (int r = gr.gl + 1; r <= n; r += 2 * G) {  // two rows of Z at a time, columns n down to 2
+        const bool two = r + G <= n;
+        const int r2 = two ? r + G : r;
+        for (int ki = n; ki >= 2; --ki) {
+            const double s = U.ldd(ki).r;
+            cx<double> a = cscal(Z.ldd(r, ki), s), b = cscal(Z.ldd(r2, ki), s);
+            for (int q = 1; q < ki; ++q) {
+                const cx<double> x = H.ldd(ki, q);
+                a = cmac(a, Z.ldd(r, q), x);
+                if (two) b = cmac(b, Z.ldd(r2, q), x);
+            }
+            Z.std(r, ki, a);
+            if (two) Z.std(r2, ki, b);
+        }
+    }
+    gr.sync();
+}
+
+// Predicted shifts of the lane kernel (the learned-shift form).
+struct FxNoShifts {
+    static constexpr bool kOn = false;
+    typedef NoShiftPredictions Picker;
+};
+
+// newton64_shifts_lane on the fixed-point Hessenberg matrix (units of H; its
+// FP64 subdiagonals in Sub), for two predictions at a time: they share each
+// entry's conversion to FP64.  Hf: FP32 copy of H in units of 2^61.  w: 5 n
+// elements of scratch (x and x' of the two, the inverse subdiagonals).
+__device__ __forceinline__ void fx_newton(const int n, const FxMat<32> &H, const FxVec<32> &Sub, const MatIlv<float> &Hf,
+                                          const VecIlv<double> &P, double2 *w, const double maxstep)
+{
+    const VecIlv<double> X[2] = {{w}, {w + n * 32}}, Inv{w + 4 * n * 32};
+    const int lane = threadIdx.x & 31;
+    float2 *const f = reinterpret_cast<float2 *>(w - lane + 2 * n * 32) + lane;
+    const VecIlv<float> D[2] = {{f}, {f + n * 32}};
+    for (int i = 2; i <= n; ++i) Inv.st(i, cinv(Sub.ldd(i - 1)));
+    for (int k = 1; k <= n; k += 2) {
+        cx<double> s[2], x[2];
+        cx<float> sf[2], d[2];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            s[b] = P.ld(min(k + b, n));
+            sf[b] = mk((float)(s[b].r * 0x1p-61), (float)(s[b].i * 0x1p-61));
+            x[b] = mk(1.0, 0.0);
+            d[b] = mk(0.f, 0.f);
+            X[b].st(n, x[b]);
+            D[b].st(n, d[b]);
+        }
+        cx<double> acc[2];
+        cx<float> dacc[2];
+        for (int i = n; i >= 1; --i) {
+            const cx<double> hii = fx_d(H.ld(i, i));
+            const cx<float> hf = Hf.ld(i, i);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {  // x(i), x'(i) are in x, d
+                acc[b] = cmul(csub(hii, s[b]), x[b]);
+                dacc[b] = csub(cmul(csub(hf, sf[b]), d[b]), mk((float)x[b].r, (float)x[b].i));
+            }
+            for (int j = i + 1; j <= n; ++j) {
+                const cx<double> h = fx_d(H.ld(i, j));
+                const cx<float> g = Hf.ld(i, j);
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    acc[b] = cmac(acc[b], h, X[b].ld(j));
+                    dacc[b] = cmac(dacc[b], g, D[b].ld(j));
+                }
+            }
+            if (i == 1) break;
+            const cx<double> inv = Inv.ld(i);
+            const cx<float> invf = mk((float)(inv.r * 0x1p61), (float)(inv.i * 0x1p61));
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                x[b] = cmul(mk(-acc[b].r, -acc[b].i), inv);
+                d[b] = cmul(mk(-dacc[b].r, -dacc[b].i), invf);
+                if (cabs1(x[b]) > 1e18) {
+                    for (int j = i; j <= n; ++j) {
+                        X[b].st(j, cscal(X[b].ld(j), 1e-18));
+                        D[b].st(j, cscal(D[b].ld(j), 1e-18f));
+                    }
+                    x[b] = cscal(x[b], 1e-18);
+                    d[b] = cscal(d[b], 1e-18f);
+                }
+                X[b].st(i - 1, x[b]);
+                D[b].st(i - 1, d[b]);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            if (k + b > n) continue;
+            const cx<double> delta = cdiv(acc[b], mk((double)dacc[b].r, (double)dacc[b].i));
+            if (!nonfinite(delta.r) && !nonfinite(delta.i) && cabs1(delta) <= maxstep) P.st(k + b, csub(s[b], delta));
+        }
+    }
+}
+
+struct FxShifts {
+    static constexpr bool kOn = true;
+    typedef ShiftPredictions Picker;
+    VecIlv<double> P;   // the matrix's predictions, as given (or polished by the pre-pass)
+    MatIlv<float> Hf;   // FP32 copy of H
+    longlong2 *scratch;  // 6 n elements, free until Q is formed
+    int polish, newton, sweeps_used;
+    float gate;
+    ShiftPredictions sp;
+    // rA, iA (stride s): the matrix; unit: the units of H
+    __device__ __forceinline__ ShiftPredictions *prepare(const int n, const FxMat<32> &H, const FxVec<32> &Sub,
+                                                         const bool ok, const double *rA, const double *iA,
+                                                         const long long s, const double unit)
+    {
+        double fro2 = 0.0;
+        const double iu = 1.0 / unit;  // a power of two
+        if (ok) {
+            for (int e = 0; e < n * n; ++e) fro2 = fma(iA[e * s], iA[e * s], fma(rA[e * s], rA[e * s], fro2));
+            const double scale = sqrt(fro2 / (double)n);
+            if (polish > 0 || newton > 0)
+                for (int j = 1; j <= n; ++j)
+                    for (int i = 1; i <= (j + 1 < n ? j + 1 : n); ++i) {
+                        const cx<double> h = i == j + 1 ? Sub.ldd(j) : fx_d(H.ld(i, j));
+                        Hf.st(i, j, mk((float)(h.r * 0x1p-61), (float)(h.i * 0x1p-61)));
+                    }
+            // FP32 steps in units of 2^61 of H, then everything in the units of H
+            const double nu = iu * 0x1p-61;
+            for (int k = 1; k <= n; ++k) P.st(k, cscal(P.ld(k), nu));
+            if (polish > 0) {
+                const float tol = (float)(1e-6 * scale * nu), keep = (float)(1e-3 * scale * nu), dup = (float)(1e-5 * scale * nu);
+                if (n <= 16) polish_shifts_lane<16>(n, Hf, P, polish, tol, keep, dup);
+                else if (n <= 32) polish_shifts_lane<32>(n, Hf, P, polish, tol, keep, dup);
+                else polish_shifts_lane<64>(n, Hf, P, polish, tol, keep, dup);
+            }
+            for (int k = 1; k <= n; ++k) P.st(k, cscal(P.ld(k), 0x1p61));
+            if (n >= 2)
+                for (int t = 0; t < newton; ++t)
+                    fx_newton(n, H, Sub, Hf, P, reinterpret_cast<double2 *>(scratch), 1e-4 * scale * iu);
+        }
+        sp.S = P;
+        sp.n = n;
+        sp.sweeps = sweeps_used;
+        sp.gate = (double)gate * sqrt(fro2 / (double)n) * iu;
+        sp.used = 0;
+        sp.current = -1;
+        sp.fallbacks = 0;
+        return &sp;
+    }
+};
+
+// The whole solve of one matrix per group, with H, Z (vectors only) and U (n
+// entries) its storage.  Returns false (group-uniform) for a valid matrix
+// that is left to the FP64 kernels; nothing is written then.
+template <int G, bool kVec, int ST, class SH = FxNoShifts>
+__device__ __forceinline__ bool fx_solve(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
+                                         const FxVec<ST> &U, const bool valid, const double *rA, const double *iA,
+                                         const long long s, const FxOut &o, const int max_its, const int vnorm,
+                                         int &sweeps, int &status, const FxChunk ch = {}, SH *shifts = nullptr)
+{
+    double unit;
+    bool ok = fx_load<G>(gr, n, H, valid, rA, iA, s, unit);
+    fx_reduce<G>(gr, n, H, U);
+    ok = ok && fx_irreducible<G>(gr, n, H);
+    typename SH::Picker *sp = nullptr;
+    if constexpr (SH::kOn) {
+        const FxVec<32> Sub{shifts->scratch + 5 * n * 32};
+        for (int k = 1; k < n; ++k) Sub.std(k, fx_d(H.ld(k + 1, k)));
+        sp = shifts->prepare(n, H, Sub, ok, rA, iA, s, unit);
+    }
+    if (kVec) fx_form_q<G>(gr, n, H, Z, U);
+    // subdiagonals in FP64 from here on
+    for (int k = gr.gl + 1; k < n; k += G) U.std(k, fx_d(H.ld(k + 1, k)));
+    gr.sync();
+    if constexpr (ST == 32) fx_qr_lane<kVec>(n, H, Z, U, ch, ok, max_its, sweeps, status, sp);
+    else fx_qr<G, kVec>(gr, n, H, Z, U, ok, max_its, sweeps, status);
+    gr.sync();
+    if (ok)
+        for (int k = gr.gl + 1; k <= n; k += G) {
+            const cx<double> e = cscal(fx_d(H.ld(k, k)), unit);
+            o.rE[(k - 1) * o.sv] = e.r;
+            o.iE[(k - 1) * o.sv] = e.i;
+        }
+    if (kVec) {
+        FxIndex ix(gr.gl, n);
+        for (int e = gr.gl; e < n * n; e += G, ix.next(G, n)) {
+            const cx<double> t = ix.i <= ix.j ? fx_d(H.ld(ix.i, ix.j)) : mk(0.0, 0.0);
+            H.std(ix.i, ix.j, t);
+            if (ok && o.rT) {
+                o.rT[e * o.sm] = t.r * unit;
+                o.iT[e * o.sm] = t.i * unit;
+            }
+            Z.std(ix.i, ix.j, fx_d(Z.ld(ix.i, ix.j)));
+        }
+        gr.sync();
+        fx_vectors<G>(gr, n, H, Z, U);
+        // scale of each column: the units of Z, and the caller's normalisation
+        for (int c = gr.gl + 1; c <= n; c += G) {
+            double sc = 0x1p-61;
+            if (vnorm == 1) {
+                double mx = 0.0;
+                for (int r = 1; r <= n; ++r) mx = fmax(mx, cabs1(Z.ldd(r, c)));
+                sc = mx > 0.0 ? 1.0 / mx : 1.0;
+            } else if (vnorm == 2) {
+                double s2 = 0.0;
+                for (int r = 1; r <= n; ++r) {
+                    const cx<double> z = cscal(Z.ldd(r, c), 0x1p-61);
+                    s2 = fma(z.i, z.i, fma(z.r, z.r, s2));
+                }
+                sc = s2 > 0.0 ? 0x1p-61 / sqrt(s2) : 1.0;
+            }
+            U.std(c, mk(sc, 0.0));
+        }
+        gr.sync();
+        if (ok) {
+            FxIndex iv(gr.gl, n);
+            for (int e = gr.gl; e < n * n; e += G, iv.next(G, n)) {
+                const cx<double> v = cscal(Z.ldd(iv.i, iv.j), U.ldd(iv.j).r);
+                o.rV[e * o.sm] = v.r;
+                o.iV[e * o.sm] = v.i;
+            }
+        }
+    }
+    gr.sync();  // the storage is reused for the next matrix
+    return ok;
+}
+
+}  // namespace ves

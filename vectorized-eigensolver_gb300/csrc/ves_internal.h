@@ -39,11 +39,13 @@ struct FusedArgs {
     int max_its;
     int vnorm;
     // optional index list: solve only matrices list[0 .. *list_count) (the
-    // mixed-precision form's fallback pass); status gets ST_REFINE_FALLBACK.
+    // mixed-precision form's fallback pass, matrices outside the fixed-point
+    // form's range); status gets the bits of status_or.
     // The lane kernel takes entries from list_split on, fp64_warp_kernel the
     // ones before it (launch_fp64_list sets it).
     const int *list;
     const int *list_count;
+    int status_or;
     long long list_split;
     // optional predicted eigenvalues (SoA vectors, n per matrix) used as the
     // first `shift_sweeps` QR shifts of every eigenvalue; `fallbacks` (nullable)
@@ -87,6 +89,45 @@ cudaError_t launch_mixed(const MixedArgs &a, cudaStream_t st);
 // sweeps, the FP64 pipe), forked from and joined back into `st`.
 cudaError_t launch_mixed_overlap(const MixedArgs &a, cudaStream_t st, cudaStream_t s_schur, cudaStream_t s_refine);
 
+// The fixed-point FP64 solve (ves_fx.cuh) of the whole batch, or of the
+// matrices on a list; matrices it leaves to the FP64 kernels are appended to
+// out_list (its counter is zero before the launch).
+constexpr int kFxMinDim = 3, kFxMaxDim = 64;
+// Orders that take the fixed-point form.  Order 2 has no reduction and one
+// rotation per sweep; its rounding there is finer than the reference's, which
+// needs a second sweep for a tenth of the matrices.
+__host__ __device__ inline bool fx_order(int n) { return n >= kFxMinDim && n <= kFxMaxDim; }
+struct FxArgs {
+    Geom g;
+    const double *rA, *iA;
+    double *rE, *iE, *rV, *iV, *rT, *iT;  // rT, iT nullable; rV, iV null without vectors
+    int *status, *sweeps;                 // nullable
+    int max_its, vnorm;
+    const int *list, *list_count;  // nullable: the matrices to solve
+    int status_or;                 // bits added to every solved matrix's status
+    int *out_list, *out_count;
+    void *ws;         // lane kernel: workspace of lane_blocks x 4 warp slots (fused_workspace_bytes)
+    int lane_blocks;
+    long long m_begin;  // without a list: the first of the g.N matrices
+    // predicted shifts (lane kernel; see FusedArgs)
+    const double *rS, *iS;
+    int shift_sweeps, shift_polish, shift_newton64;
+    float shift_gate;
+    int *fallbacks;
+};
+// 16-byte elements per lane of a shift-seeded slot: H, Z, a work vector, an FP32
+// copy of H, the n predictions, n FP32 elements for the FP64 kernel, and where
+// Z is smaller than the Newton step's 6 n elements, those.
+__host__ __device__ inline long long shift_slot_elems(int n)
+{
+    const long long nn = (long long)n * n;
+    return 2 * nn + n + (nn + 1) / 2 + n + (n + 1) / 2 + (n < 6 ? 6 * n : 0);
+}
+cudaError_t launch_fx(const FxArgs &a, bool vec, cudaStream_t st);
+cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, cudaStream_t st);  // one matrix per lane, on a.lane_blocks blocks
+
+cudaError_t launch_fx_shifts(const FxArgs &a, cudaStream_t st);  // the same with predicted shifts
+
 // Fused zgehrd -> zunghr -> zlahqr -> ztrevc, FP64.
 // blocks_per_sm = 0 takes the library default (VES_FUSED_BLOCKS_PER_SM, else 4; 3 for 21 <= n <= 28).
 // learned = the shift-seeded kernel, whose slots also hold an FP32 copy of H
@@ -112,9 +153,18 @@ cudaError_t launch_zgemv(Geom g, bool herm, const double *rA, const double *iA, 
                          double rbeta, double ibeta, double *ry, double *iy, cudaStream_t st);
 cudaError_t launch_backsubs(Geom g, const double *rT, const double *iT, double *rx, double *ix, cudaStream_t st);
 
-// The FP64 fused kernel on a caller-chosen grid of `blocks` x 4 warps; the
-// workspace must hold blocks * 4 warp slots.
-cudaError_t launch_fused_fp64_blocks(const FusedArgs &a, int blocks, cudaStream_t st);
+// The plain FP64 solve: fx_order(n) in fixed point, then the matrices that it
+// leaves to the FP64 kernels; other n in the FP64 kernels.  `a` as for
+// launch_fused_fp64 (a.list: those matrices only); flist holds a.g.N ints
+// (unused for other n), fcount one int.
+cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st);
+// The shift-seeded solve (a.rS) the same way, one matrix per lane.
+cudaError_t launch_shifts(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st);
+// launch_plain for matrices [m0, m0 + count) (n <= 64) with the lane kernels on a
+// caller-chosen grid of `blocks` x 4 warps, whose slots a.ws holds; no other
+// memory is used.
+cudaError_t launch_plain_blocks(const FusedArgs &a, long long m0, long long count, int blocks, int *flist, int *fcount,
+                                cudaStream_t st);
 
 // Learned-shift polish pre-pass (n <= 32): predictions (rS, iS) refined by
 // Aberth steps on the FP32 Hessenberg form, written to (rP, iP); NaN = dropped.
@@ -124,8 +174,10 @@ cudaError_t launch_polish32(Geom g, const double *rA, const double *iA, const do
 // Eigenvalues only (no Q, no Schur vectors), companion-matrix roots, and the
 // SoA <-> interleaved-complex transposes.
 size_t eigvals_workspace_bytes(int n, long long N, int blocks_per_sm);
+int eigvals_blocks(int n, long long N, int blocks_per_sm);  // of 4 warps, each with a slot of the workspace
 cudaError_t launch_eigvals(Geom g, const double *rA, const double *iA, double *rE, double *iE, int *status,
-                           int *sweeps, void *ws, int max_its, int blocks_per_sm, cudaStream_t st);
+                           int *sweeps, void *ws, int max_its, int blocks_per_sm, const int *list,
+                           const int *list_count, cudaStream_t st);  // list nullable: those matrices only
 cudaError_t launch_polyroots(Geom g, const double *rC, const double *iC, double *rR, double *iR, int *status,
                              void *ws, int max_its, cudaStream_t st);
 cudaError_t launch_transpose(bool to_soa, const double *src_re, const double *src_im, double *dst_re, double *dst_im,
@@ -177,6 +229,7 @@ enum { WORK_RES64 = 0, WORK_CORR32 = 1, WORK_RESFF = 2, WORK_POLISH = 3 };
 // file's list below is in that order.
 void load_kernels();
 void load_mixed_kernels();
+void load_fx_kernels();
 void load_fused_kernels();
 void load_varsize_kernels();
 void load_extras_kernels();

@@ -31,8 +31,7 @@ constexpr int kFusedThreads = 128;  // 4 warps per block
 // ceil(n^2 / 2) double2), the n predictions and an FP32 vector (n float2).
 __host__ __device__ __forceinline__ long long fused_slot_elems(int n, bool learned)
 {
-    const long long nn = (long long)n * n;
-    return 2 * nn + n + (learned ? (nn + 1) / 2 + n + (n + 1) / 2 : 0);
+    return learned ? shift_slot_elems(n) : 2LL * n * n + n;
 }
 
 __device__ __forceinline__ long long soa_mat_off(long long m, int n, int tc)
@@ -178,7 +177,7 @@ __global__ void __launch_bounds__(kFusedThreads) fused_fp64_kernel(const FusedAr
             ztrevc_lane<double>(n, H, Z, W);
             const MatSoA<double> V{a.rV + mo, a.iV + mo, tc, n};
             write_vectors<double>(n, Z, V, a.vnorm);
-            if (a.status) a.status[m] = status | (a.list ? ST_REFINE_FALLBACK : 0);
+            if (a.status) a.status[m] = status | a.status_or;
             if (a.sweeps) a.sweeps[m] = sweeps;
         }
     }
@@ -435,7 +434,7 @@ __global__ void __launch_bounds__(32) fp64_warp_kernel(const FusedArgs a)
             for (int i = 1; i <= n; ++i) V.st(i, j, cscal(Z.ld(i, j), scale));
         }
         if (lane == 0) {
-            if (a.status) a.status[m] = status | (a.list ? ST_REFINE_FALLBACK : 0);
+            if (a.status) a.status[m] = status | a.status_or;
             if (a.sweeps) a.sweeps[m] = sweeps;
         }
         __syncwarp();
@@ -811,10 +810,73 @@ cudaError_t launch_fp64_list(FusedArgs a, cudaStream_t st)
     return launch_fused_fp64(a, st);
 }
 
-cudaError_t launch_fused_fp64_blocks(const FusedArgs &a, int blocks, cudaStream_t st)
+static FxArgs fx_args(const FusedArgs &a, int *flist, int *fcount)
+{
+    FxArgs f{};
+    f.g = a.g;
+    f.rA = a.rA; f.iA = a.iA;
+    f.rE = a.rE; f.iE = a.iE; f.rV = a.rV; f.iV = a.iV; f.rT = a.rT; f.iT = a.iT;
+    f.status = a.status; f.sweeps = a.sweeps;
+    f.max_its = a.max_its; f.vnorm = a.vnorm;
+    f.list = a.list; f.list_count = a.list_count; f.status_or = a.status_or;
+    f.out_list = flist; f.out_count = fcount;
+    f.ws = a.ws;
+    return f;
+}
+
+cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st)
 {
     if (a.g.N <= 0) return cudaSuccess;
-    fused_fp64_kernel<false><<<blocks, kFusedThreads, 0, st>>>(a);
+    if (!fx_order(a.g.n)) return a.list ? launch_fp64_list(a, st) : launch_fused_fp64(a, st);
+    cudaError_t e = cudaMemsetAsync(fcount, 0, sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    FxArgs f = fx_args(a, flist, fcount);
+    fused_workspace_bytes(a.g.n, a.g.N, a.blocks_per_sm, &f.lane_blocks, nullptr);
+    if ((e = launch_fx(f, true, st)) != cudaSuccess) return e;
+    FusedArgs r = a;
+    r.list = flist;
+    r.list_count = fcount;
+    return launch_fp64_list(r, st);
+}
+
+cudaError_t launch_shifts(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st)
+{
+    if (a.g.N <= 0) return cudaSuccess;
+    if (!fx_order(a.g.n)) return launch_fused_fp64(a, st);
+    cudaError_t e = cudaMemsetAsync(fcount, 0, sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    FxArgs f = fx_args(a, flist, fcount);
+    f.rS = a.rS; f.iS = a.iS;
+    f.shift_sweeps = a.shift_sweeps; f.shift_gate = a.shift_gate;
+    f.shift_polish = a.shift_polish; f.shift_newton64 = a.shift_newton64;
+    f.fallbacks = a.fallbacks;
+    fused_workspace_bytes(a.g.n, a.g.N, a.blocks_per_sm, &f.lane_blocks, nullptr, true);
+    if ((e = launch_fx_shifts(f, st)) != cudaSuccess) return e;
+    FusedArgs r = a;
+    r.list = flist;
+    r.list_count = fcount;
+    r.list_split = 0;
+    return launch_fused_fp64(r, st);
+}
+
+cudaError_t launch_plain_blocks(const FusedArgs &a, long long m0, long long count, int blocks, int *flist, int *fcount,
+                                cudaStream_t st)
+{
+    cudaError_t e = cudaMemsetAsync(fcount, 0, sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    FxArgs f = fx_args(a, flist, fcount);
+    f.g.N = count;
+    f.m_begin = m0;
+    f.lane_blocks = blocks;
+    FusedArgs r = a;
+    if (!fx_order(a.g.n)) {
+        fused_fp64_kernel<false><<<blocks, kFusedThreads, 0, st>>>(r);
+        return cudaGetLastError();
+    }
+    if ((e = launch_fx_lanes(f, true, st)) != cudaSuccess) return e;
+    r.list = flist;
+    r.list_count = fcount;
+    fused_fp64_kernel<false><<<blocks, kFusedThreads, 0, st>>>(r);
     return cudaGetLastError();
 }
 

@@ -28,6 +28,10 @@
 namespace {
 
 constexpr size_t kScratchBytes = VES_NOALLOC_SCRATCH_BYTES;  // 64 MiB per device
+// the end of the array: counter and list of the matrices that the fixed-point
+// solve leaves to the FP64 kernel, for slices of kSlice matrices
+constexpr long long kSlice = 1 << 20;
+constexpr size_t kListBytes = 256 + kSlice * sizeof(int);
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -86,11 +90,8 @@ int ves_eigensolve_noalloc(int dim, int block_cnt, int thread_cnt, const double 
     // As many persistent warps as the array holds (4 warps per block), never
     // more than there are 32-matrix groups; each warp loops over groups.
     const long long per_warp = (2LL * dim * dim + dim) * 32 * (long long)sizeof(double2);
-    const long long warps_fit = (long long)kScratchBytes / per_warp;  // >= 15 for dim <= 64
+    const long long warps_fit = (long long)(kScratchBytes - kListBytes) / per_warp;  // >= 14 for dim <= 64
     if (warps_fit < 4) return fail(VES_ERR_ARG, "ves_eigensolve_noalloc: dim too large for the scratch array");
-    const long long groups = (N + 31) / 32;
-    const long long blocks = std::min<long long>((groups + 3) / 4, warps_fit / 4);
-
     ves::FusedArgs a{};
     a.g.n = dim;
     a.g.N = N;
@@ -102,8 +103,15 @@ int ves_eigensolve_noalloc(int dim, int block_cnt, int thread_cnt, const double 
     a.ws = scratch;
     a.max_its = 30;
     a.vnorm = VES_VNORM_REFERENCE;
-    const cudaError_t e = ves::launch_fused_fp64_blocks(a, (int)blocks, (cudaStream_t)stream);
-    if (e != cudaSuccess) return fail(VES_ERR_CUDA, "ves_eigensolve_noalloc: kernel launch failed");
+    int *count = reinterpret_cast<int *>(static_cast<unsigned char *>(scratch) + kScratchBytes - kListBytes);
+    const long long slice = ves::fx_order(dim) ? kSlice : N;  // other orders use no list
+    for (long long m0 = 0; m0 < N; m0 += slice) {
+        const long long n_slice = std::min(N - m0, slice);
+        const long long blocks = std::min<long long>((n_slice + 127) / 128, warps_fit / 4);
+        const cudaError_t e = ves::launch_plain_blocks(a, m0, n_slice, (int)blocks, count + 64, count,
+                                                       (cudaStream_t)stream);
+        if (e != cudaSuccess) return fail(VES_ERR_CUDA, "ves_eigensolve_noalloc: kernel launch failed");
+    }
     return VES_OK;
 }
 

@@ -18,7 +18,7 @@
 //                   fixed-size solver (same routines), one matrix per lane
 // The lockstep routines need all lanes of a warp at the same n; binning is
 // what lets a mixed batch keep them full.
-#include "ves_device.cuh"
+#include "ves_fx.cuh"
 #include "ves_internal.h"
 
 #include <algorithm>
@@ -161,7 +161,12 @@ struct VarArgs {
 
 __global__ void __launch_bounds__(kSolveThreads) varsize_solve_kernel(const VarArgs a)
 {
+    __shared__ longlong2 chs[kSolveThreads * kFxChunk];
+    __shared__ i64 chi[kSolveThreads * kFxChunk];
+    const FxGroup<1> gr;
     const int lane = threadIdx.x & 31;
+    const int ch0 = (threadIdx.x >> 5) * 32 * kFxChunk + lane;
+    const FxChunk ch{chs + ch0, chi + ch0};
     const long long slot = (long long)blockIdx.x * (kSolveThreads / 32) + (threadIdx.x >> 5);
     const int MD = a.max_dim;
     double2 *base = reinterpret_cast<double2 *>(a.ws) + slot * (2LL * MD * MD + MD) * 32 + lane;
@@ -176,10 +181,26 @@ __global__ void __launch_bounds__(kSolveThreads) varsize_solve_kernel(const VarA
         const MatIlv<double> H{base, n};
         const MatIlv<double> Z{base + (long long)n * n * 32, n};
         const VecIlv<double> W{base + 2LL * n * n * 32};
-        const bool valid = lane < item.count;
+        bool valid = lane < item.count;
         const long long m = valid ? a.sorted[item.at + lane] : 0;
         const long long ao = valid ? a.aoff[m] : 0, eo = valid ? a.eoff[m] : 0;
         int status = 0, sweeps = 0;
+        if (fx_order(n)) {
+            longlong2 *const fb = reinterpret_cast<longlong2 *>(base);
+            const FxMat<32> FH{fb, n, n}, FZ{fb + (long long)n * n * 32, n, n};
+            const FxVec<32> FU{fb + 2LL * n * n * 32};
+            const FxOut o{a.rE + eo, a.iE + eo, a.rV + ao, a.iV + ao, nullptr, nullptr, 1, 1};
+            const bool ok = fx_solve<1, true>(gr, n, FH, FZ, FU, valid, a.rA + ao, a.iA + ao, 1, o, a.max_its, a.vnorm,
+                                              sweeps, status, ch);
+            if (ok) {
+                if (a.status) a.status[m] = status;
+                if (a.sweeps) a.sweeps[m] = sweeps;
+            }
+            // what the fixed-point form leaves is solved in FP64 by the same warp
+            valid = valid && !ok;
+            if (!__any_sync(FULL, valid)) continue;
+            status = sweeps = 0;
+        }
         if (valid) {
             const MatSoA<double> A{const_cast<double *>(a.rA) + ao, const_cast<double *>(a.iA) + ao, 1, n};
             bool bad = false;
