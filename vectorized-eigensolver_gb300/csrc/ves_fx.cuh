@@ -180,6 +180,13 @@ struct FxCoef {
     {
     }
     __device__ __forceinline__ explicit FxCoef(const FxRot &q) : FxCoef(q.c, q.sr, q.si) {}
+    __device__ __forceinline__ FxCoef columns() const  // of the rotation with conj(s)
+    {
+        FxCoef q(*this);
+        q.si = nsi;
+        q.nsi = si;
+        return q;
+    }
 };
 
 __device__ __forceinline__ cx64 fx_i(cx<double> z) { return {__double2ll_rn(z.r), __double2ll_rn(z.i)}; }
@@ -209,15 +216,14 @@ __device__ __forceinline__ FxRot fx_rot(const cx<double> x0, const cx<double> x1
 }
 
 // Rotate the pair (x1, x2): x1' = c x1 + s x2, x2' = c x2 - conj(s) x1 (rows of
-// H), with conj(s) for s on columns (kCol).
-template <bool kCol> __device__ __forceinline__ void fx_pair(cx64 &x1, cx64 &x2, const FxCoef &q)
+// H; columns of H and Z take the coefficients of conj(s)).
+__device__ __forceinline__ void fx_pair(cx64 &x1, cx64 &x2, const FxCoef &q)
 {
-    const fx si = kCol ? q.nsi : q.si, nsi = kCol ? q.si : q.nsi;
     const cfx a = fx_split(x1), b = fx_split(x2);
-    x1.r = fx_dot3(q.c, a.r, q.sr, b.r, nsi, b.i);
-    x1.i = fx_dot3(q.c, a.i, q.sr, b.i, si, b.r);
-    x2.r = fx_dot3(q.c, b.r, q.nsr, a.r, nsi, a.i);
-    x2.i = fx_dot3(q.c, b.i, q.nsr, a.i, si, a.r);
+    x1.r = fx_dot3(q.c, a.r, q.sr, b.r, q.nsi, b.i);
+    x1.i = fx_dot3(q.c, a.i, q.sr, b.i, q.si, b.r);
+    x2.r = fx_dot3(q.c, b.r, q.nsr, a.r, q.nsi, a.i);
+    x2.i = fx_dot3(q.c, b.i, q.nsr, a.i, q.si, a.r);
 }
 
 // Wilkinson's shift of the trailing 2 x 2 block [a b; c d] (any phases) in
@@ -257,11 +263,11 @@ __device__ __forceinline__ float fx_absf(cx<double> z)
     const float r = (float)z.r, i = (float)z.i;
     return sqrtf(fmaf(r, r, i * i));
 }
+// (s, d1, d2): S(K-1), H(K-1, K-1), H(K, K).
 template <int ST>
-__device__ __forceinline__ bool fx_negligible(const FxMat<ST> &H, const FxVec<ST> &S, const int K, const int n)
+__device__ __forceinline__ bool fx_negligible(const FxMat<ST> &H, const FxVec<ST> &S, const int K, const int n,
+                                              const cx<double> s, const cx64 d1, const cx64 d2)
 {
-    const cx<double> s = S.ldd(K - 1);
-    const cx64 d1 = H.ld(K - 1, K - 1), d2 = H.ld(K, K);
     const float sr = (float)s.r, si = (float)s.i, hk = sqrtf(fmaf(sr, sr, si * si));
     if (hk <= 0.5f) return true;
     float tst = (float)(fx_abs1(d1) + fx_abs1(d2));
@@ -275,6 +281,12 @@ __device__ __forceinline__ bool fx_negligible(const FxMat<ST> &H, const FxVec<ST
     const float up = fabsf(ur * pr - ui * pi) + fabsf(ur * pi + ui * pr);
     const float kk = (float)fx_abs1(d2), df = (float)fx_abs1({d1.r - d2.r, d1.i - d2.i});
     return fminf(hk, up) * fmaxf(hk, up) <= 0x1p-52f * fminf(kk, df) * fmaxf(kk, df);
+}
+
+template <int ST>
+__device__ __forceinline__ bool fx_negligible(const FxMat<ST> &H, const FxVec<ST> &S, const int K, const int n)
+{
+    return fx_negligible(H, S, K, n, S.ldd(K - 1), H.ld(K - 1, K - 1), H.ld(K, K));
 }
 
 // A group of G lanes that owns one matrix: part of a warp (G < 32), a warp, or
@@ -416,6 +428,108 @@ __device__ __forceinline__ bool fx_load(const FxGroup<G> &gr, const int n, const
     return gr.all(ok);
 }
 
+// Functions below that are not inlined keep one copy of their code: the lane
+// kernel's warps run out of step, and with everything inlined its code did not
+// fit the instruction caches (n=16: 4.0 M/s on one wave, 2.6 M/s on eight).
+// ST tells the memory space: 1 = shared, 32 = global.
+template <int ST> __device__ __forceinline__ void fx_assume_space(const void *p)
+{
+#ifdef __CUDA_ARCH__
+    if (ST == 1) __builtin_assume(__isShared(p));
+    else __builtin_assume(__isGlobal(p));
+#endif
+}
+
+// Bring the line of p into L2 (no register is held for it).
+__device__ __forceinline__ void fx_prefetch(const void *p)
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+#endif
+}
+
+// a -= u (u^H a) for NB vectors a of m entries (vector b at a + b blk), or
+// with conj(u) for u (cj): the reflector from the left on columns, or from the
+// right on rows.  The first entry of u is u1, the others u[k * ustep].
+template <int NB, int ST>
+__device__ __noinline__ void fx_reflect(longlong2 *a, const int step, const int blk, const longlong2 *u,
+                                        const int ustep, const i64 u1r, const i64 u1i, const int m, const bool cj)
+{
+    fx_assume_space<ST>(a);
+    fx_assume_space<ST>(u);
+    facc sr[NB], si[NB];
+    longlong2 v[NB], uk = make_longlong2(u1r, u1i);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        sr[b] = si[b] = fx_zero<61>();
+        v[b] = a[b * blk];
+    }
+    longlong2 *p = a;
+    for (int k = 0; k < m; ++k) {
+        const cfx f = fx_split(cx64{uk.x, cj ? -uk.y : uk.y});
+        const fx nf = fx_split(cj ? uk.y : -uk.y);
+        cfx x[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) x[b] = fx_split(cx64{v[b].x, v[b].y});
+        p += step;
+        if (k + 1 < m) {  // the next entries
+            uk = u[k * ustep];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) v[b] = p[b * blk];
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            fx_mac(sr[b], f.r, x[b].r);
+            fx_mac(sr[b], f.i, x[b].i);
+            fx_mac(si[b], f.r, x[b].i);
+            fx_mac(si[b], nf, x[b].r);
+            if ((k & 3) == 3) { fx_flush(sr[b]); fx_flush(si[b]); }
+        }
+    }
+    cfx nz[NB];
+    fx zi[NB];
+    p = a;
+    uk = make_longlong2(u1r, u1i);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const i64 zr = fx_end<61>(sr[b]), zm = fx_end<61>(si[b]);
+        nz[b] = fx_split(cx64{-zr, -zm});
+        zi[b] = fx_split(zm);
+        v[b] = p[b * blk];
+    }
+    for (int k = 0; k < m; ++k) {
+        const cfx f = fx_split(cx64{uk.x, cj ? -uk.y : uk.y});
+        longlong2 w[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) w[b] = v[b];
+        longlong2 *const p1 = p + step;
+        if (k + 1 < m) {
+            uk = u[k * ustep];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) v[b] = p1[b * blk];
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+            p[b * blk] = make_longlong2(w[b].x + fx_dot2<61>(nz[b].r, f.r, zi[b], f.i),
+                                        w[b].y + fx_dot2<61>(nz[b].i, f.r, nz[b].r, f.i));
+        p = p1;
+    }
+}
+// vectors gl, gl + G, ... of count, kFxReflect at a time
+constexpr int kFxReflect = 4;
+template <int G, int ST>
+__device__ __forceinline__ void fx_reflect_all(const int gl, longlong2 *a, const int step, const int blk,
+                                               const int count, const longlong2 *u, const cx64 u1, const int m,
+                                               const bool cj)
+{
+    constexpr int NB = G > 8 ? 1 : kFxReflect;  // larger groups have one or two vectors per lane
+    int v = gl;
+    if (NB > 1)
+        for (; v + (NB - 1) * G < count; v += NB * G)
+            fx_reflect<NB, ST>(a + v * blk, step, G * blk, u, ST, u1.r, u1.i, m, cj);
+    for (; v < count; v += G) fx_reflect<1, ST>(a + v * blk, step, 0, u, ST, u1.r, u1.i, m, cj);
+}
+
 // Householder reduction to Hessenberg form with Hermitian reflectors
 // P = I - u u^H, ||u||^2 = 2 (the subdiagonal comes out complex).  u_k, k >=
 // i + 2, stays below the subdiagonal of column i, u_{i+1} in U(i).
@@ -423,6 +537,7 @@ template <int G, int ST>
 __device__ __forceinline__ void fx_reduce(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxVec<ST> &U)
 {
     constexpr int RG = FxGroup<G>::RG;
+    const int rs = ST, cs = H.lda * ST;  // steps to the next row, the next column
     for (int i = 1; i <= n - 2; ++i) {
         const cx64 al = H.ld(i + 1, i);
         i64 o = 0;
@@ -464,57 +579,13 @@ __device__ __forceinline__ void fx_reduce(const FxGroup<G> &gr, const int n, con
         }
         if (gr.gl == 0) {
             U.st(i, u1);
-            H.st(i + 1, i, u1);  // so that u is column i from here on; beta at the end
+            H.st(i + 1, i, beta);
         }
         gr.sync();
-        // right: row r of A(:, i+1:n) -= (A u)_r u^H
-        for (int r = gr.gl + 1; r <= n; r += G) {
-            facc sr = fx_zero<61>(), si = sr;
-            for (int k = i + 1; k <= n; ++k) {
-                const cfx u = fx_split(H.ld(k, i));
-                const cx64 x = H.ld(r, k);
-                const cfx a = fx_split(x);
-                const fx na = fx_split(-x.i);
-                fx_mac(sr, a.r, u.r);
-                fx_mac(sr, na, u.i);
-                fx_mac(si, a.r, u.i);
-                fx_mac(si, a.i, u.r);
-                if (((k - i) & 3) == 0) { fx_flush(sr); fx_flush(si); }
-            }
-            const cx64 y = {fx_end<61>(sr), fx_end<61>(si)};
-            const cfx ny = fx_split(cx64{-y.r, -y.i});
-            const fx yr = fx_split(y.r);
-            for (int k = i + 1; k <= n; ++k) {
-                const cfx u = fx_split(H.ld(k, i));
-                const cx64 x = H.ld(r, k);
-                H.st(r, k, {x.r + fx_dot2<61>(ny.r, u.r, ny.i, u.i), x.i + fx_dot2<61>(ny.i, u.r, yr, u.i)});
-            }
-        }
+        const longlong2 *u = H.at(i + 2, i);
+        fx_reflect_all<G, ST>(gr.gl, H.at(1, i + 1), cs, rs, n, u, u1, n - i, true);  // rows of A(:, i+1:n)
         gr.sync();
-        // left: column c of A(i+1:n, i+1:n) -= u (u^H A)_c
-        for (int c = i + 1 + gr.gl; c <= n; c += G) {
-            facc sr = fx_zero<61>(), si = sr;
-            for (int k = i + 1; k <= n; ++k) {
-                const cx64 uk = H.ld(k, i);
-                const cfx u = fx_split(uk), a = fx_split(H.ld(k, c));
-                const fx nu = fx_split(-uk.i);
-                fx_mac(sr, u.r, a.r);
-                fx_mac(sr, u.i, a.i);
-                fx_mac(si, u.r, a.i);
-                fx_mac(si, nu, a.r);
-                if (((k - i) & 3) == 0) { fx_flush(sr); fx_flush(si); }
-            }
-            const cx64 z = {fx_end<61>(sr), fx_end<61>(si)};
-            const cfx nz = fx_split(cx64{-z.r, -z.i});
-            const fx zi = fx_split(z.i);
-            for (int k = i + 1; k <= n; ++k) {
-                const cfx u = fx_split(H.ld(k, i));
-                const cx64 x = H.ld(k, c);
-                H.st(k, c, {x.r + fx_dot2<61>(nz.r, u.r, zi, u.i), x.i + fx_dot2<61>(nz.i, u.r, nz.r, u.i)});
-            }
-        }
-        gr.sync();
-        if (gr.gl == 0) H.st(i + 1, i, beta);
+        fx_reflect_all<G, ST>(gr.gl, H.at(i + 1, i + 1), rs, cs, n - i, u, u1, n - i, false);  // columns of A(i+1:n, i+1:n)
         gr.sync();
     }
 }
@@ -526,33 +597,11 @@ __device__ __forceinline__ void fx_form_q(const FxGroup<G> &gr, const int n, con
 {
     for (int c = gr.gl + 1; c <= n; c += G)
         for (int r = 1; r <= n; ++r) Z.st(r, c, {r == c ? 1LL << 61 : 0, 0});
-    // a lane's columns are its own: no synchronisation between reflectors
-    for (int i = n - 2; i >= 1; --i) {
-        const cx64 u1 = U.ld(i);
-        for (int c = gr.gl + 1; c <= n; c += G) {
-            if (c < i + 1) continue;
-            facc sr = fx_zero<61>(), si = sr;
-            for (int k = i + 1; k <= n; ++k) {
-                const cx64 uk = k == i + 1 ? u1 : H.ld(k, i);
-                const cfx u = fx_split(uk), a = fx_split(Z.ld(k, c));
-                const fx nu = fx_split(-uk.i);
-                fx_mac(sr, u.r, a.r);
-                fx_mac(sr, u.i, a.i);
-                fx_mac(si, u.r, a.i);
-                fx_mac(si, nu, a.r);
-                if (((k - i) & 3) == 0) { fx_flush(sr); fx_flush(si); }
-            }
-            const cx64 z = {fx_end<61>(sr), fx_end<61>(si)};
-            const cfx nz = fx_split(cx64{-z.r, -z.i});
-            const fx zi = fx_split(z.i);
-            for (int k = i + 1; k <= n; ++k) {
-                const cfx u = fx_split(k == i + 1 ? u1 : H.ld(k, i));
-                const cx64 x = Z.ld(k, c);
-                Z.st(k, c, {x.r + fx_dot2<61>(nz.r, u.r, zi, u.i), x.i + fx_dot2<61>(nz.i, u.r, nz.r, u.i)});
-            }
-        }
-    }
     gr.sync();
+    for (int i = n - 2; i >= 1; --i) {
+        fx_reflect_all<G, ST>(gr.gl, Z.at(i + 1, i + 1), ST, Z.lda * ST, n - i, H.at(i + 2, i), U.ld(i), n - i, false);
+        gr.sync();
+    }
 }
 
 // no subdiagonal below 2^-30 of the scale
@@ -580,7 +629,17 @@ __device__ __forceinline__ bool fx_next_sweep(const FxGroup<G> &gr, const int n,
         if (its > max_its) { status |= ST_ITCAP; --I; L = 1; its = 0; continue; }
         // the largest K in (L, I] whose subdiagonal is negligible, else L
         int K = L;
-        for (int top = I; top > L; top -= RG) {
+        if (RG == 1) {  // one lane per matrix: each diagonal entry is read once, one ahead
+            cx64 d2 = H.ld(I, I), d1 = L < I ? H.ld(I - 1, I - 1) : d2;
+            cx<double> s = L < I ? S.ldd(I - 1) : mk(0.0, 0.0);
+            for (int k = I; k > L; --k) {
+                const cx64 e2 = d2, e1 = d1;
+                const cx<double> es = s;
+                if (k - 1 > L) { d1 = H.ld(k - 2, k - 2); s = S.ldd(k - 2); }
+                d2 = e1;
+                if (fx_negligible(H, S, k, n, es, e1, e2)) { K = k; break; }
+            }
+        } else for (int top = I; top > L; top -= RG) {
             const int k = top - gr.rl;
             const unsigned b = gr.ballot(k > L && fx_negligible(H, S, k > L ? k : L + 1, n)) &
                                (RG == 32 ? FULL : (1u << (RG & 31)) - 1u);
@@ -652,7 +711,7 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
             if (sweep && K >= L && K < I) {
                 cx<double> r;
                 const FxRot R = fx_rot(a0, a1, r);
-                const FxCoef C(R);
+                const FxCoef C(R), CC = C.columns();
                 const cx64 ssub = fx_i(sub);
                 const cx<double> hkk = fx_d(H.ld(K, K));
                 const cx<double> nxt = K + 1 < I ? S.ldd(K + 1) : mk(0.0, 0.0);  // H(K+2, K+1)
@@ -668,7 +727,7 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
                 for (int j = K + gr.gl; j <= jmax; j += G) {
                     cx64 y1 = H.ld(K, j), y2 = H.ld(K + 1, j);
                     if (j == K) y2 = ssub;
-                    fx_pair<false>(y1, y2, C);
+                    fx_pair(y1, y2, C);
                     H.st(K, j, y1);
                     if (j > K) H.st(K + 1, j, y2);
                 }
@@ -688,7 +747,7 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
                     const longlong2 w1 = *p1, w2 = *p2;
                     cx64 y1 = {w1.x, w1.y}, y2 = {w2.x, w2.y};
                     if (q == 0) y1 = sx1;
-                    fx_pair<true>(y1, y2, C);
+                    fx_pair(y1, y2, CC);
                     if (q != 0) *p1 = make_longlong2(y1.r, y1.i);
                     *p2 = make_longlong2(y2.r, y2.i);
                 }
@@ -701,7 +760,7 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
 }
 
 // Rotations of the current chunk of a sweep, in shared memory, one set per lane.
-constexpr int kFxChunk = 8;
+constexpr int kFxChunk = 16;
 constexpr int kFxStream = 2;  // chains streamed together
 struct FxChunk {
     longlong2 *cs;  // (c, sr) of rotation k at cs[k * 32]
@@ -718,14 +777,24 @@ struct FxChunk {
     }
 };
 
-// Apply rotations k0 .. k0 + ns - 1 of the chunk to NB chains of entries: chain
-// b's entries at p + b blk + k step, rotation k on entries k and k + 1.  The
-// entry that two rotations share stays in registers, so each entry is read
-// and written once per chunk.
-template <int NB, bool kCol>
-__device__ __forceinline__ void fx_stream(longlong2 *p, const int step, const int blk, const FxChunk &ch,
-                                          const int k0, const int ns)
+// Apply ns rotations (c, s at cs[k * 32], si[k * 32]) to NB chains of entries:
+// chain b's entries at p + b blk + k step, rotation k on entries k and k + 1,
+// from the left or, with conj(s) for s, from the right (col).  The entry that
+// two rotations share stays in registers, so each entry is read and written
+// once per chunk.
+//
+// next (nullable): NB chains of the same shape, next_step apart per entry, that
+// the caller streams after these; their lines are brought into L2 meanwhile.
+// One rotation's entries ahead in registers, 16 warps keep 16 KB in flight per
+// SM, which against the latency of DRAM is 4.7 TB/s at most; with the lines
+// already in L2 the registers cover what is left.
+template <int NB>
+__device__ __noinline__ void fx_stream(longlong2 *p, const int step, const int blk, const longlong2 *cs, const i64 *si,
+                                       const int ns, const bool col, const longlong2 *next, const int next_step)
 {
+    fx_assume_space<32>(p);
+    fx_assume_space<1>(cs);
+    fx_assume_space<1>(si);
     cx64 x[NB];
     longlong2 y[NB];
 #pragma unroll
@@ -735,17 +804,21 @@ __device__ __forceinline__ void fx_stream(longlong2 *p, const int step, const in
         y[b] = p[b * blk + step];
     }
     for (int k = 0; k < ns; ++k) {
-        const FxCoef q = ch.get(k0 + k);
+        const longlong2 c = cs[k * 32];
+        const i64 s = si[k * 32];
+        const FxCoef q(c.x, c.y, col ? -s : s);
         longlong2 *const p1 = p + step;
         cx64 z[NB];
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             z[b] = {y[b].x, y[b].y};
             if (k + 1 < ns) y[b] = p1[b * blk + step];  // the next rotation's entries
+            if (next) fx_prefetch(next + b * blk);
         }
+        if (next) next += next_step;
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-            fx_pair<kCol>(x[b], z[b], q);
+            fx_pair(x[b], z[b], q);
             p[b * blk] = make_longlong2(x[b].r, x[b].i);
             x[b] = z[b];
         }
@@ -754,13 +827,17 @@ __device__ __forceinline__ void fx_stream(longlong2 *p, const int step, const in
 #pragma unroll
     for (int b = 0; b < NB; ++b) p[b * blk] = make_longlong2(x[b].r, x[b].i);
 }
-template <bool kCol>
 __device__ __forceinline__ void fx_stream_all(longlong2 *p, const int step, const int blk, const int count,
-                                              const FxChunk &ch, const int ns)
+                                              const FxChunk &ch, const int ns, const bool col,
+                                              const longlong2 *next = nullptr, const int next_step = 0)
 {
     int b = 0;
-    for (; b + kFxStream <= count; b += kFxStream) fx_stream<kFxStream, kCol>(p + b * blk, step, blk, ch, 0, ns);
-    for (; b < count; ++b) fx_stream<1, kCol>(p + b * blk, step, blk, ch, 0, ns);
+    for (; b + kFxStream <= count; b += kFxStream) {
+        const bool more = b + 2 * kFxStream <= count;
+        fx_stream<kFxStream>(p + b * blk, step, blk, ch.cs, ch.si, ns, col, more ? p + (b + kFxStream) * blk : next,
+                             more ? step : next_step);
+    }
+    for (; b < count; ++b) fx_stream<1>(p + b * blk, step, blk, ch.cs, ch.si, ns, col, nullptr, 0);
 }
 
 // fx_qr for one matrix per lane, 32 in lockstep per sweep, in the warp's
@@ -789,7 +866,7 @@ __device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, cons
         if (!__any_sync(FULL, sweep)) break;
         const int Kmin = __reduce_min_sync(FULL, sweep ? L : INT_MAX);
         const int Kmax = __reduce_max_sync(FULL, sweep ? I - 1 : 0);
-        cx64 hkk = {0, 0};
+        cx64 hkk = H.ld(Kmin, Kmin);
         for (int Kc = Kmin; Kc <= Kmax; Kc += kFxChunk) {
             const int Ke = min(Kc + kFxChunk - 1, Kmax), ns = Ke - Kc + 1;
             for (int K = Kc; K <= Ke; ++K) {
@@ -799,56 +876,60 @@ __device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, cons
                 R.ds = mk(0.0, 0.0);
                 R.c = 1LL << 62;
                 R.sr = R.si = 0;
-                // column K + 1: the chunk's rotations so far
-                longlong2 *pc = H.at(Kc, K + 1);
-                longlong2 v = pc[0];
+                // column K + 1: the chunk's left rotations so far; each row that is done takes
+                // rotation K from the right, with its entry of column K
+                longlong2 *pc = H.at(Kc, K + 1), *pl = H.at(Kc, K);
+                longlong2 v = pc[0], w = pl[0];
                 cx64 x = {v.x, v.y};
                 v = pc[rs];
                 cx<double> r, nxt = mk(0.0, 0.0);
                 if (act) {
                     R = fx_rot(a0, a1, r);
-                    if (K == L) hkk = H.ld(K, K);
                     if (K + 1 < I) nxt = S.ldd(K + 1);
                 }
                 ch.put(K - Kc, R);
+                const FxCoef C(R), CC = C.columns();
                 for (int q = Kc; q < K; ++q) {
-                    cx64 y = {v.x, v.y};
+                    cx64 y = {v.x, v.y}, z = {w.x, w.y};
                     v = pc[2 * rs];
-                    fx_pair<false>(x, y, ch.get(q - Kc));
+                    w = pl[rs];
+                    fx_pair(x, y, ch.get(q - Kc));
+                    fx_pair(z, x, CC);
+                    pl[0] = make_longlong2(z.r, z.i);
                     pc[0] = make_longlong2(x.r, x.i);
                     x = y;
                     pc += rs;
+                    pl += rs;
                 }
-                const FxCoef C(R);
-                cx64 y = {v.x, v.y};
-                fx_pair<false>(x, y, C);
+                // rows K, K + 1; H(K+1, K) is the FP64 subdiagonal
+                cx64 y = {v.x, v.y}, y2 = act ? fx_i(sub) : cx64{0, 0};
+                const cx64 h0 = hkk;
+                fx_pair(x, y, C);
+                fx_pair(hkk, y2, C);
+                fx_pair(hkk, x, CC);
+                pl[0] = make_longlong2(hkk.r, hkk.i);
                 pc[0] = make_longlong2(x.r, x.i);
                 if (act) {
-                    // column K, then row K + 1 of the columns K, K + 1
-                    const cx<double> ks = conj(R.ds), dk = fx_d(hkk);
-                    const cx<double> x1 = cnmac(cscal(sub, R.dc), ks, dk);  // H(K+1, K) after the row operation
-                    cx64 y2 = fx_i(sub);
-                    fx_pair<false>(hkk, y2, C);
-                    H.st(K, K, hkk);
+                    const cx<double> ks = conj(R.ds);
+                    const cx<double> x1 = cnmac(cscal(sub, R.dc), ks, fx_d(h0));  // H(K+1, K) after the row operation
                     if (K > L) S.std(K - 1, r);
                     if (K + 1 < I) S.std(K + 1, cscal(nxt, R.dc));
                     a0 = cmac(cscal(x1, R.dc), ks, fx_d(y));
                     a1 = cmul(ks, nxt);  // the bulge H(K+2, K)
                     sub = cscal(nxt, R.dc);
                     cx64 z1 = fx_i(x1);
-                    fx_pair<true>(z1, y, C);
-                    hkk = y;
+                    fx_pair(z1, y, CC);
                     if (K == I - 1) S.std(I - 1, a0);
                 }
+                hkk = y;
                 H.st(K + 1, K + 1, y);
             }
-            // rows above the chunk, then the chunk's own rows, whose first rotation is their own
+            // rows above the chunk
             const int r0 = kVec ? 1 : Kmin;
-            if (Kc > r0) fx_stream_all<true>(H.at(r0, Kc), cs, rs, Kc - r0, ch, ns);
-            for (int r = Kc; r <= Ke; ++r) fx_stream<1, true>(H.at(r, r), cs, rs, ch, r - Kc, Ke - r + 1);
-            if (kVec) fx_stream_all<true>(Z.at(1, Kc), cs, rs, n, ch, ns);
+            if (Kc > r0) fx_stream_all(H.at(r0, Kc), cs, rs, Kc - r0, ch, ns, true);
+            if (kVec) fx_stream_all(Z.at(1, Kc), cs, rs, n, ch, ns, true);
             const int je = kVec ? n : Kmax + 1;
-            if (je > Ke + 1) fx_stream_all<false>(H.at(Kc, Ke + 2), rs, cs, je - Ke - 1, ch, ns);
+            if (je > Ke + 1) fx_stream_all(H.at(Kc, Ke + 2), rs, cs, je - Ke - 1, ch, ns, false);
         }
     }
 }
