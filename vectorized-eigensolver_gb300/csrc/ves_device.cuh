@@ -708,6 +708,7 @@ __device__ __forceinline__ void hess32_warp(const int n, const SmemMat &H, float
 // the reference's shifts take over.  An eigenvalue that still needs more than
 // sweeps + 2 sweeps counts as a fallback to Wilkinson.
 struct NoShiftPredictions {
+    static constexpr bool kOn = false;
     template <class R> __device__ __forceinline__ void pick(int, int, cx<R> &, R) {}
     __device__ __forceinline__ void deflated(int) {}
 };
@@ -717,6 +718,7 @@ struct NoShiftPredictions {
 // starts: once it is that small the Wilkinson shift is already more accurate
 // than the predictions, and they are left alone.
 struct ShiftPredictions {
+    static constexpr bool kOn = true;
     VecIlv<double> S;  // this matrix's n predictions in the workspace (NaN: none)
     int n, sweeps;
     double gate;

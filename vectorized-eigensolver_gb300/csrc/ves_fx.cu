@@ -151,8 +151,6 @@ template <int G, bool kVec> cudaError_t launch_fx_g(const FxArgs &a, cudaStream_
 template <bool kVec> cudaError_t launch_fx_v(const FxArgs &a, int G, cudaStream_t st)
 {
     switch (G) {
-    case 1: return launch_fx_g<1, kVec>(a, st);
-    case 2: return launch_fx_g<2, kVec>(a, st);
     case 4: return launch_fx_g<4, kVec>(a, st);
     case 8: return launch_fx_g<8, kVec>(a, st);
     case 16: return launch_fx_g<16, kVec>(a, st);
@@ -171,7 +169,7 @@ int fx_group_size(int n, long long N, bool vec)
 {
     if (const char *e = getenv("VES_FX_LANES")) {  // tuning
         const int v = atoi(e);
-        if (v >= 0 && v <= 128 && (v & (v - 1)) == 0) return v;
+        if (v == 0 || (v >= 4 && v <= 128 && (v & (v - 1)) == 0)) return v;
     }
     if (N > 6000) return 0;
     return n <= 8 ? 8 : n <= 24 ? 16 : n <= 32 ? 32 : n <= 48 ? 64 : 128;
@@ -209,7 +207,7 @@ void load_fx_kernels()
     load_kernel(fx_lane_kernel<true>);
     load_kernel(fx_lane_kernel<false>);
     load_kernel(fx_shifts_kernel);
-    load_fx_g<1>(); load_fx_g<2>(); load_fx_g<4>(); load_fx_g<8>(); load_fx_g<16>(); load_fx_g<32>(); load_fx_g<64>();
+    load_fx_g<4>(); load_fx_g<8>(); load_fx_g<16>(); load_fx_g<32>(); load_fx_g<64>();
     load_fx_g<128>();
 }
 

@@ -226,30 +226,64 @@ __device__ __forceinline__ void fx_pair(cx64 &x1, cx64 &x2, const FxCoef &q)
     x2.i = fx_dot3(q.c, b.i, q.nsr, a.i, q.si, a.r);
 }
 
-// Wilkinson's shift of the trailing 2 x 2 block [a b; c d] (any phases) in
-// FP64, in the units of H: t = d - bc / (x + y), x = (a - d) / 2,
-// y = sqrt(x^2 + bc) on x's side.  Entries are integers up to 2^61: nothing
-// here overflows or underflows, so no scaling is needed.
-__device__ __forceinline__ cx<double> fx_wilkinson(const cx<double> a, const cx<double> b, const cx<double> c,
-                                                   const cx<double> d)
+// Wilkinson's correction of the shift: t = d - bc / (x + y) for the trailing
+// block [a b; c d] (any phases), x = (a - d) / 2, y = sqrt(x^2 + bc) on x's
+// side; here bc / (x + y), from x, b, c in units of 2^61 of H.  In FP32: as c
+// becomes small the term does too, and an error of 2^-22 of it costs the
+// convergence nothing.  Products and sums are written out, so every kernel
+// computes the same bits.
+__device__ __forceinline__ cx<float> fx_wilkinson(const cx<float> x, const cx<float> b, const cx<float> c)
 {
-    const cx<double> bc = cmul(b, c);
-    const cx<double> x = cscal(csub(a, d), 0.5);
-    const cx<double> z = cadd(cmul(x, x), bc);
-    const double n2 = fma(z.r, z.r, z.i * z.i);
-    cx<double> y = mk(0.0, 0.0);
-    if (n2 > 0.0) {
-        const double az = n2 * rsqrt(n2);
-        const double h = 0.5 * (az + fabs(z.r));
-        const double rh = rsqrt(h), zr = h * rh, zi = 0.5 * fabs(z.i) * rh;
-        y = z.r < 0.0 ? mk(zi, zr) : mk(zr, zi);
-        if (z.i < 0.0) y.i = -y.i;
+    const cx<float> bc = mk(__fmaf_rn(b.r, c.r, -__fmul_rn(b.i, c.i)), __fmaf_rn(b.i, c.r, __fmul_rn(b.r, c.i)));
+    const cx<float> z = mk(__fadd_rn(__fmaf_rn(x.r, x.r, -__fmul_rn(x.i, x.i)), bc.r),
+                           __fadd_rn(__fmul_rn(2.f, __fmul_rn(x.r, x.i)), bc.i));
+    // sqrt(z): |z| = m |z / m|, m its larger component
+    const float m = fmaxf(fabsf(z.r), fabsf(z.i));
+    cx<float> y = mk(0.f, 0.f);
+    if (m > 0.f) {
+        const float im = __frcp_rn(m), u = __fmul_rn(z.r, im), v = __fmul_rn(z.i, im);
+        const float az = __fsqrt_rn(__fmaf_rn(u, u, __fmul_rn(v, v)));
+        const float h = __fmul_rn(0.5f, __fadd_rn(az, fabsf(u)));  // in [1/2, sqrt 2]
+        const float sm = __fsqrt_rn(m), zr = __fsqrt_rn(h), zi = __fmul_rn(__fmul_rn(0.5f, fabsf(v)), __frcp_rn(zr));
+        y = u < 0.f ? mk(__fmul_rn(zi, sm), __fmul_rn(zr, sm)) : mk(__fmul_rn(zr, sm), __fmul_rn(zi, sm));
+        if (v < 0.f) y.i = -y.i;
     }
-    if (fma(x.r, y.r, x.i * y.i) < 0.0) y = mk(-y.r, -y.i);
-    const cx<double> v = cadd(x, y);
-    const double v2 = fma(v.r, v.r, v.i * v.i);
-    if (!(v2 > 0.0)) return d;
-    return csub(d, cscal(cmulc(bc, v), 1.0 / v2));
+    if (__fmaf_rn(x.r, y.r, __fmul_rn(x.i, y.i)) < 0.f) y = mk(-y.r, -y.i);
+    const cx<float> w = mk(__fadd_rn(x.r, y.r), __fadd_rn(x.i, y.i));
+    const float k = fmaxf(fabsf(w.r), fabsf(w.i));
+    if (!(k > 0.f)) return mk(0.f, 0.f);
+    const float ik = __frcp_rn(k), wr = __fmul_rn(w.r, ik), wi = __fmul_rn(w.i, ik);
+    const float q = __fmul_rn(ik, __frcp_rn(__fmaf_rn(wr, wr, __fmul_rn(wi, wi))));
+    return mk(__fmul_rn(__fmaf_rn(bc.r, wr, __fmul_rn(bc.i, wi)), q),
+              __fmul_rn(__fmaf_rn(bc.i, wr, -__fmul_rn(bc.r, wi)), q));
+}
+
+// For a window of two the shift is the eigenvalue, and one sweep ends it if
+// the shift is exact to rounding: two Newton steps on w (w + 2x) = bc, the
+// residual in fixed point, take the FP32 value there (2^-22 -> 2^-44 -> units).
+__device__ __forceinline__ void fx_wilkinson_2x2(cx64 &w, const cx64 x2, const cx64 b, const cx64 c)
+{
+    const cfx bf = fx_split(b), cf = fx_split(c);
+    const fx nbi = fx_split(-b.i);
+    const cx64 bc = {fx_dot2<61>(bf.r, cf.r, nbi, cf.i), fx_dot2<61>(bf.r, cf.i, bf.i, cf.r)};
+#pragma unroll 1
+    for (int it = 0; it < 2; ++it) {
+        const cx64 v = {w.r + x2.r, w.i + x2.i};
+        const cfx wf = fx_split(w), vf = fx_split(v);
+        const fx nwi = fx_split(-w.i);
+        const float rr = (float)(fx_dot2<61>(wf.r, vf.r, nwi, vf.i) - bc.r);
+        const float ri = (float)(fx_dot2<61>(wf.r, vf.i, wf.i, vf.r) - bc.i);
+        const float k = 0x1p-61f, dr = __fmul_rn(__fadd_rn((float)v.r, (float)w.r), k),
+                    di = __fmul_rn(__fadd_rn((float)v.i, (float)w.i), k);
+        const float m = fmaxf(fabsf(dr), fabsf(di));
+        if (!(m > 0x1p-55f)) return;
+        const float im = __frcp_rn(m), ur = __fmul_rn(dr, im), ui = __fmul_rn(di, im);
+        const float q = __fmul_rn(im, __frcp_rn(__fmaf_rn(ur, ur, __fmul_rn(ui, ui))));
+        const float er = __fmul_rn(__fmaf_rn(rr, ur, __fmul_rn(ri, ui)), q), ei = __fmul_rn(__fmaf_rn(ri, ur, -__fmul_rn(rr, ui)), q);
+        if (!(fabsf(er) + fabsf(ei) < 0x1p60f)) return;
+        w.r -= __float2ll_rn(er);
+        w.i -= __float2ll_rn(ei);
+    }
 }
 
 // Is the subdiagonal H(K, K-1) = S(K-1) negligible?  The reference's test
@@ -258,31 +292,36 @@ __device__ __forceinline__ cx<double> fx_wilkinson(const cx<double> a, const cx<
 // moves the thresholds by a few 2^-23; anything below half a unit is
 // negligible too.  The reference keeps subdiagonals real by a diagonal phase
 // similarity: there H(K, K-1) is |s| and H(K-1, K) is turned by the phase of s.
-__device__ __forceinline__ float fx_absf(cx<double> z)
+__device__ __forceinline__ float fx_absf(cx<float> z) { return __fsqrt_rn(__fmaf_rn(z.r, z.r, __fmul_rn(z.i, z.i))); }
+// x 2^sh in FP32, truncated, without the FP64 pipe (conversions run on it);
+// 0 below 2^-126
+__device__ __forceinline__ float fx_float(const double x, const int sh)
 {
-    const float r = (float)z.r, i = (float)z.i;
-    return sqrtf(fmaf(r, r, i * i));
+    const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023 + 127 + sh;
+    const int v = (hi & 0x80000000) | (e << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(x) >> 29);
+    return e > 0 ? __int_as_float(v) : 0.f;
 }
+__device__ __forceinline__ cx<float> fx_float(const cx<double> z, const int sh) { return mk(fx_float(z.r, sh), fx_float(z.i, sh)); }
 // (s, d1, d2): S(K-1), H(K-1, K-1), H(K, K).
 template <int ST>
 __device__ __forceinline__ bool fx_negligible(const FxMat<ST> &H, const FxVec<ST> &S, const int K, const int n,
                                               const cx<double> s, const cx64 d1, const cx64 d2)
 {
-    const float sr = (float)s.r, si = (float)s.i, hk = sqrtf(fmaf(sr, sr, si * si));
+    const cx<float> sf = fx_float(s, 0);
+    const float hk = fx_absf(sf);
     if (hk <= 0.5f) return true;
     float tst = (float)(fx_abs1(d1) + fx_abs1(d2));
     if (tst == 0.f) {
-        if (K - 2 >= 1) tst += fx_absf(S.ldd(K - 2));
-        if (K + 1 <= n) tst += fx_absf(S.ldd(K));
+        if (K - 2 >= 1) tst += fx_absf(fx_float(S.ldd(K - 2), 0));
+        if (K + 1 <= n) tst += fx_absf(fx_float(S.ldd(K), 0));
     }
     if (hk > 0x1p-52f * tst) return false;
     const cx64 u = H.ld(K - 1, K);
-    const float ur = (float)u.r, ui = (float)u.i, ih = 1.f / hk, pr = sr * ih, pi = si * ih;
-    const float up = fabsf(ur * pr - ui * pi) + fabsf(ur * pi + ui * pr);
+    const float ur = (float)u.r, ui = (float)u.i, ih = __frcp_rn(hk), pr = sf.r * ih, pi = sf.i * ih;
+    const float up = fabsf(__fmaf_rn(ur, pr, -__fmul_rn(ui, pi))) + fabsf(__fmaf_rn(ur, pi, __fmul_rn(ui, pr)));
     const float kk = (float)fx_abs1(d2), df = (float)fx_abs1({d1.r - d2.r, d1.i - d2.i});
     return fminf(hk, up) * fmaxf(hk, up) <= 0x1p-52f * fminf(kk, df) * fmaxf(kk, df);
 }
-
 template <int ST>
 __device__ __forceinline__ bool fx_negligible(const FxMat<ST> &H, const FxVec<ST> &S, const int K, const int n)
 {
@@ -649,22 +688,36 @@ __device__ __forceinline__ bool fx_next_sweep(const FxGroup<G> &gr, const int n,
         if (G > 32) __syncthreads();  // the scans have read S
         if (L > 1) S.std(L - 1, mk(0.0, 0.0));  // every lane: the same value
         if (L >= I) {
-            if (sp) sp->deflated(its);
+            if constexpr (SP::kOn) sp->deflated(its);
             --I; L = 1; its = 0;
             continue;
         }
-        const cx<double> hll = fx_d(H.ld(L, L));
+        const cx64 hll = H.ld(L, L);
         a1 = S.ldd(L);
-        cx<double> t;
-        if (its == 10) t = mk(fma(0.75, cabs(a1), hll.r), hll.i);
-        else {
-            const cx<double> si = S.ldd(I - 1);
-            t = fx_d(H.ld(I, I));
-            if (its == 20) t.r = fma(0.75, cabs(si), t.r);
-            else t = fx_wilkinson(fx_d(H.ld(I - 1, I - 1)), fx_d(H.ld(I - 1, I)), si, t);
+        const cx<double> si = S.ldd(I - 1);
+        cx64 t = H.ld(I, I);
+        if (its == 10) {
+            t = hll;
+            t.r += __float2ll_rn(0.75f * fx_absf(fx_float(a1, 0)));
+        } else if (its == 20) {
+            t.r += __float2ll_rn(0.75f * fx_absf(fx_float(si, 0)));
+        } else {
+            const cx64 u = H.ld(I - 1, I), d = H.ld(I - 1, I - 1);
+            const float k = 0x1p-61f;
+            const cx<float> w = fx_wilkinson(mk((float)(d.r - t.r) * (0.5f * k), (float)(d.i - t.i) * (0.5f * k)),
+                                             mk((float)u.r * k, (float)u.i * k), fx_float(si, -61));
+            cx64 c = {__float2ll_rn(w.r * 0x1p61f), __float2ll_rn(w.i * 0x1p61f)};
+            if (L == I - 1) fx_wilkinson_2x2(c, {d.r - t.r, d.i - t.i}, u, fx_i(si));
+            t.r -= c.r;
+            t.i -= c.i;
         }
-        if (sp) sp->template pick<double>(its, I, t, cabs(S.ldd(I - 1)));
-        a0 = csub(hll, t);
+        if constexpr (SP::kOn) {
+            const cx<double> t0 = fx_d(t);
+            cx<double> td = t0;
+            sp->template pick<double>(its, I, td, (double)fx_absf(fx_float(si, 0)));
+            if (td.r != t0.r || td.i != t0.i) t = fx_i(td);
+        }
+        a0 = fx_d(cx64{hll.r - t.r, hll.i - t.i});
         ++its;
         return true;
     }
@@ -682,18 +735,33 @@ __device__ __forceinline__ bool fx_next_sweep(const FxGroup<G> &gr, const int n,
 // reach the end of the window.  With them in fixed point (an absolute
 // rounding) the transformations are as accurate, but the subdiagonals stall at
 // 2^-46 of the matrix.  Every other entry is only rotated.
+//
+// The FP64 steps of a rotation are spread over the lanes of a quad: an FP64
+// instruction holds a quarter of an SM for 62 cycles however many lanes need
+// it, and the chain of them is what a group waits for.  Lanes 0 and 1 of a quad
+// work on the real and imaginary part of the pair's first number (and of what
+// becomes the next first number), lanes 2 and 3 on the second; the other lanes
+// of the group repeat them.  The operations on each value are those of fx_rot
+// and of fx_qr_lane.
 template <int G, bool kVec, int ST>
 __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z, const FxVec<ST> &S,
                                       const bool run, const int max_its, int &sweeps, int &status)
 {
+    static_assert(G >= 4, "the scalar steps are spread over four lanes");
+    const int role = gr.gl & 3;
+    const bool im = role & 1, second = role >= 2;
+    const unsigned mk4 = gr.mask;
+    const auto from = [&](double v, int lane) { return __shfl_sync(mk4, v, lane, 4); };
+    const double one = 4611686018427387904.0;  // 2^62
     int I = n, L = 1, its = 0;
     bool done = !run || n <= 1;
     for (;;) {
-        cx<double> a0, a1, sub;  // the pair of the next rotation; H(K+1, K)
-        const bool sweep = !done && fx_next_sweep<G>(gr, n, H, S, max_its, I, L, its, status, a0, a1);
+        cx<double> z, a1;
+        const bool sweep = !done && fx_next_sweep<G>(gr, n, H, S, max_its, I, L, its, status, z, a1);
         done = !sweep;
-        sub = a1;
         sweeps += sweep;
+        double sub = im ? a1.i : a1.r;  // lanes 0, 1: H(K+1, K)
+        if (second) z = a1;             // the lane's number of the pair
         int Kmin, Kmax;
         if (G < 32) {
             if (!__any_sync(FULL, sweep)) break;
@@ -709,20 +777,42 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
         const int jmax = kVec ? n : I, jmin = kVec ? 1 : L;
         for (int K = Kmin; K <= Kmax; ++K) {
             if (sweep && K >= L && K < I) {
-                cx<double> r;
-                const FxRot R = fx_rot(a0, a1, r);
-                const FxCoef C(R), CC = C.columns();
-                const cx64 ssub = fx_i(sub);
-                const cx<double> hkk = fx_d(H.ld(K, K));
+                const cx64 hk = H.ld(K, K);
                 const cx<double> nxt = K + 1 < I ? S.ldd(K + 1) : mk(0.0, 0.0);  // H(K+2, K+1)
-                const cx<double> ks = conj(R.ds);
-                // H(K+1, K) after the row operation
-                const cx<double> x1 = cnmac(cscal(sub, R.dc), ks, hkk);
-                gr.sync();  // every lane has read H(K, K) and S
-                if (gr.gl == 0) {
-                    if (K > L) S.std(K - 1, r);
-                    if (K + 1 < I) S.std(K + 1, cscal(nxt, R.dc));
+                const double hc = (double)(im ? hk.i : hk.r);
+                const i64 isub = __double2ll_rn(sub);
+                // fx_rot
+                const double m2 = fma(z.r, z.r, z.i * z.i);
+                const double f = from(m2, 0), g = from(m2, 2);
+                const double n2 = f + g, w = f * n2;
+                const bool deg = !(w > 1e-280);
+                const double p = rsqrt(deg ? fmax(g, 1e-280) : w);
+                const double x1r = from(z.r, 2), x1i = from(z.i, 2);
+                const double a = deg ? 1.0 : from(z.r, 0), b = deg ? 0.0 : from(z.i, 0);
+                double v = fma(im ? b : a, x1r, (im ? -a : b) * x1i);  // s / p
+                if (second) v = im ? (deg ? g : n2) : f;
+                v *= p;  // Re s, Im s, c, n2 p
+                if (deg) {
+                    if (role == 2) v = g > 1e-280 ? 0.0 : 1.0;
+                    if (!second && !(g > 1e-280)) v = 0.0;
                 }
+                const double np = from(v, 3), dc = from(v, 2);
+                const cx<double> ks = mk(from(v, 0), -from(v, 1));  // conj(s)
+                const i64 iv = __double2ll_rn(v * one);
+                const FxCoef C(__shfl_sync(mk4, iv, 2, 4), __shfl_sync(mk4, iv, 0, 4), __shfl_sync(mk4, iv, 1, 4)),
+                    CC = C.columns();
+                const double rc = (im ? b : a) * np;  // lanes 0, 1: r
+                // lanes 0, 1: x1 = c sub - conj(s) h_kk, H(K+1, K) after the row operation;
+                // lanes 2, 3: the bulge conj(s) H(K+2, K+1)
+                const double hr = from(hc, 0), hi = from(hc, 1);
+                double t = second ? (im ? ks.r : -ks.i) * nxt.i : sub * dc;
+                t = fma(second ? (im ? ks.i : ks.r) : (im ? -ks.i : -ks.r), second ? nxt.r : hr, t);
+                if (!second) t = fma(im ? -ks.r : ks.i, hi, t);
+                const i64 ix1 = __double2ll_rn(t);
+                const cx64 sx1 = {__shfl_sync(mk4, ix1, 0, 4), __shfl_sync(mk4, ix1, 1, 4)};
+                const cx64 ssub = {__shfl_sync(mk4, isub, 0, 4), __shfl_sync(mk4, isub, 1, 4)};
+                gr.sync();  // every lane has read H(K, K) and S
+                if (K > L && gr.gl < 2) reinterpret_cast<double *>(S.at(K - 1))[gr.gl] = rc;
                 // rows K, K+1 of columns K..jmax; H(K+1, K) is the FP64 subdiagonal
                 for (int j = K + gr.gl; j <= jmax; j += G) {
                     cx64 y1 = H.ld(K, j), y2 = H.ld(K + 1, j);
@@ -732,13 +822,22 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
                     if (j > K) H.st(K + 1, j, y2);
                 }
                 gr.sync();
-                // columns K, K+1 of H (rows up to K+1), then of Z
-                const cx<double> x2 = fx_d(H.ld(K + 1, K + 1));
-                const cx64 sx1 = fx_i(x1);
-                a0 = cmac(cscal(x1, R.dc), ks, x2);
-                a1 = cmul(ks, nxt);  // the bulge H(K+2, K)
-                sub = cscal(nxt, R.dc);
+                // a0 = c x1 + conj(s) h_k+1,k+1; sub = c H(K+2, K+1)
+                const cx64 h2 = H.ld(K + 1, K + 1);
+                const double xc = (double)(im ? h2.i : h2.r);
+                const double xr = from(xc, 0), xi = from(xc, 1);
+                double u = (second ? (im ? nxt.i : nxt.r) : t) * dc;
+                const double nsub = __shfl_xor_sync(mk4, u, 2, 4);  // lanes 0, 1: from lanes 2, 3
+                if (!second) {
+                    u = fma(im ? ks.i : ks.r, xr, u);
+                    u = fma(im ? ks.r : -ks.i, xi, u);
+                    t = u;
+                }
+                sub = nsub;
+                const double other = __shfl_xor_sync(mk4, t, 1, 4);
+                z = im ? mk(other, t) : mk(t, other);
                 gr.sync();  // every lane has read H(K+1, K+1)
+                // columns K, K+1 of H (rows up to K+1), then of Z
                 const int nc = K + 2 - jmin;
                 for (int q = gr.gl; q < nc + (kVec ? n : 0); q += G) {
                     const bool h = !kVec || q < nc;
@@ -751,7 +850,7 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
                     if (q != 0) *p1 = make_longlong2(y1.r, y1.i);
                     *p2 = make_longlong2(y2.r, y2.i);
                 }
-                if (K == I - 1 && gr.gl == 0) S.std(I - 1, a0);
+                if (K == I - 1 && gr.gl < 2) reinterpret_cast<double *>(S.at(I - 1))[gr.gl] = t;
                 gr.sync();
             }
             if (G < 32) __syncwarp();
@@ -913,7 +1012,6 @@ __device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, cons
                     const cx<double> ks = conj(R.ds);
                     const cx<double> x1 = cnmac(cscal(sub, R.dc), ks, fx_d(h0));  // H(K+1, K) after the row operation
                     if (K > L) S.std(K - 1, r);
-                    if (K + 1 < I) S.std(K + 1, cscal(nxt, R.dc));
                     a0 = cmac(cscal(x1, R.dc), ks, fx_d(y));
                     a1 = cmul(ks, nxt);  // the bulge H(K+2, K)
                     sub = cscal(nxt, R.dc);
@@ -1151,6 +1249,7 @@ __device__ __forceinline__ bool fx_solve(const FxGroup<G> &gr, const int n, cons
             o.rE[(k - 1) * o.sv] = e.r;
             o.iE[(k - 1) * o.sv] = e.i;
         }
+    gr.sync();  // the diagonal is read before it is converted below
     if (kVec) {
         FxIndex ix(gr.gl, n);
         for (int e = gr.gl; e < n * n; e += G, ix.next(G, n)) {
