@@ -4,6 +4,7 @@
 #include "ves_internal.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 
 namespace ves {
@@ -133,17 +134,20 @@ int fx_sms()
 template <int G> size_t fx_smem(int n, bool vec) { return (size_t)FxShape<G>::mats * fx_slot(n, G, vec) * sizeof(longlong2); }
 constexpr size_t kMaxSmem = 227 * 1024;
 
+// Blocks that fit an SM: 228 KB of shared memory (1 KB of it per block is the
+// system's) and 64 K registers (168 a thread for one warp, at most 128 for more).
+int fx_blocks_per_sm(int G, size_t smem)
+{
+    const int regs = G > 32 ? G * 128 : 32 * 168;
+    return std::max(1, (int)std::min<size_t>(228 * 1024 / (smem + 1024), (size_t)65536 / regs));
+}
+
 template <int G, bool kVec> cudaError_t launch_fx_g(const FxArgs &a, cudaStream_t st)
 {
     const size_t smem = fx_smem<G>(a.g.n, kVec);
     if (smem > kMaxSmem) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(fx_kernel<G, kVec>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 1;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fx_kernel<G, kVec>, FxShape<G>::threads, smem);
-    if (e != cudaSuccess) return e;
     const long long need = (a.g.N + FxShape<G>::mats - 1) / FxShape<G>::mats;
-    const long long blocks = std::min<long long>(need, (long long)fx_sms() * std::max(per_sm, 1));
+    const long long blocks = std::min<long long>(need, (long long)fx_sms() * fx_blocks_per_sm(G, smem));
     fx_kernel<G, kVec><<<(unsigned)std::max<long long>(blocks, 1), FxShape<G>::threads, smem, st>>>(a);
     return cudaGetLastError();
 }
@@ -163,16 +167,42 @@ template <bool kVec> cudaError_t launch_fx_v(const FxArgs &a, int G, cudaStream_
 }  // namespace
 
 // Lanes per matrix: 0 = the lane kernel, whose 32 matrices share every FP64
-// instruction, once a batch is large enough to fill it; below, a group of
-// lanes per matrix in shared memory, more of them for fewer matrices.
+// instruction but take long for one wave; otherwise a group of G lanes per
+// matrix in shared memory, faster per matrix with more lanes but with fewer
+// matrices resident.  The rule takes the smallest estimated time:
+//   group  waves * 0.33 ms (n/8)^1.85 (1 + n / (3 G)), and for G > 32, whose
+//          warps repeat the FP64 steps, 3% per warp on the SM
+//   lane   1.05 ms (n/8)^2.66 (1 + N n / 1.2e6) for one wave of 2,432 warps
+// Measured on GB300, ms (lane; G = 4, 8, 16, 32): n=16, N=64 6.35; 2.41 1.70
+// 1.35 1.19.  N=2,048 6.84; 2.57 1.85 1.68 2.47.  N=8,192 6.94; 7.43 5.65
+// 5.69 9.40.  N=16,384 8.05; 12.3 9.5 10.2 18.5.  n=32 (G = 16, 32, 64), N=64
+// 41.5; 6.05 4.83 4.28, N=8,192 54.7; 53.8 47.7 65.2.  n=64 (G = 64, 128),
+// N=512 299; 68.2 64.1.  Without vectors about half the lane kernel's time and
+// 0.9 of the group's.  Over 60 (n, N) from 4 to 64 and 64 to 65,536 the choice
+// is on average 2% from the best of all.
 int fx_group_size(int n, long long N, bool vec)
 {
     if (const char *e = getenv("VES_FX_LANES")) {  // tuning
         const int v = atoi(e);
         if (v == 0 || (v >= 4 && v <= 128 && (v & (v - 1)) == 0)) return v;
     }
-    if (N > 6000) return 0;
-    return n <= 8 ? 8 : n <= 24 ? 16 : n <= 32 ? 32 : n <= 48 ? 64 : 128;
+    const double sms = fx_sms(), x = n / 8.0;
+    int best = 0;
+    double t = (vec ? 1.05 : 0.52) * pow(x, 2.66) * (1.0 + (double)N * n / (vec ? 1.2e6 : 2e6));
+    for (int G = 4; G <= 128; G *= 2) {
+        if (G > 32 ? G > 2 * n : G > 4 * n) break;
+        const int mats = G < 32 ? 32 / G : 1;
+        const size_t smem = (size_t)mats * fx_slot(n, G, vec) * sizeof(longlong2);
+        if (smem > kMaxSmem) continue;
+        const double fit = fx_blocks_per_sm(G, smem), waves = ceil((double)N / (sms * fit * mats));
+        double tg = waves * (vec ? 0.33 : 0.30) * pow(x, 1.85) * (1.0 + n / ((vec ? 3.0 : 5.0) * G));
+        if (G > 32) tg *= 1.0 + 0.03 * std::min(fit, ceil((double)N / (sms * mats))) * G / 32;
+        if (tg < t) {
+            t = tg;
+            best = G;
+        }
+    }
+    return best;
 }
 
 cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, cudaStream_t st)
@@ -201,6 +231,8 @@ template <int G> static void load_fx_g()
 {
     load_kernel(fx_kernel<G, true>);
     load_kernel(fx_kernel<G, false>);
+    cudaFuncSetAttribute(fx_kernel<G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    cudaFuncSetAttribute(fx_kernel<G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
 }
 void load_fx_kernels()
 {

@@ -795,16 +795,11 @@ cudaError_t launch_fp64_list(FusedArgs a, cudaStream_t st)
     if (a.g.N <= 0) return cudaSuccess;
     a.list_split = 0;
     if (a.list && !a.rS && a.g.n <= 64) {
-        // per call (per device, thread safe; microseconds next to the kernel)
-        cudaError_t e = cudaFuncSetAttribute(fp64_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)fp64_warp_smem(64));
-        if (e != cudaSuccess) return e;
-        int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fp64_warp_kernel, 32, fp64_warp_smem(a.g.n));
-        const long long slots = (long long)device_sms() * std::max(per_sm, 1);
-        a.list_split = std::min<long long>(a.g.N, slots);
+        // one matrix per warp slot: 228 KB of shared memory, at most 16 a SM (64 K registers)
+        const long long per_sm = std::max<long long>(1, std::min<long long>(16, 228 * 1024 / (fp64_warp_smem(a.g.n) + 1024)));
+        a.list_split = std::min<long long>(a.g.N, device_sms() * per_sm);
         fp64_warp_kernel<<<(unsigned)a.list_split, 32, fp64_warp_smem(a.g.n), st>>>(a);
-        e = cudaGetLastError();
+        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
     return launch_fused_fp64(a, st);
@@ -972,6 +967,7 @@ void load_fused_kernels()
     load_kernel(fused_fp64_kernel<false>);
     load_kernel(fused_fp64_kernel<true>);
     load_kernel(fp64_warp_kernel);
+    cudaFuncSetAttribute(fp64_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp64_warp_smem(64));
     load_kernel(polish32_warp_kernel);
     load_kernel(zgehrd_kernel);
     load_kernel(zunghr_kernel);
