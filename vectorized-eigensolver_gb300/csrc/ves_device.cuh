@@ -640,18 +640,24 @@ __device__ __forceinline__ unsigned group_mask(int lane)
     return G == 32 ? FULL : (((1u << G) - 1u) << (lane & ~(G - 1)));
 }
 
-// zgehd2 on a G-lane group's matrix (n <= G): H = Q^H A Q, the same
+// zgehd2 on a G-lane group's matrix (n <= NJ G): H = Q^H A Q, the same
 // reflector conventions and per-element operation order as zgehrd_lane;
 // reflector vectors below the subdiagonal, tau(i) in sTau[i - 1].  gl is the
 // lane's index in its group, mask the group's lanes.
-template <int G>
+template <int G, int NJ = 1>
 __device__ __forceinline__ void hess_group(const int n, const SmemMat &H, float2 *sTau, const int gl, const unsigned mask)
 {
-    const int j = gl + 1;
     for (int i = 1; i <= n - 1; ++i) {
         const int mm = n - i;
-        const cx<float> xk = (j >= i + 2 && j <= n) ? H.ld(j, i) : mk(0.f, 0.f);
-        const float xnorm2 = group_sum<G>(fmaf(xk.i, xk.i, xk.r * xk.r), mask);
+        cx<float> xk[NJ];
+        float x2 = 0.f;
+#pragma unroll
+        for (int t = 0; t < NJ; ++t) {
+            const int j = gl + 1 + t * G;
+            xk[t] = (j >= i + 2 && j <= n) ? H.ld(j, i) : mk(0.f, 0.f);
+            x2 = t ? fmaf(xk[t].i, xk[t].i, fmaf(xk[t].r, xk[t].r, x2)) : fmaf(xk[t].i, xk[t].i, xk[t].r * xk[t].r);
+        }
+        const float xnorm2 = group_sum<G>(x2, mask);
         const cx<float> alpha = H.ld(i + 1, i);
         const bool trivial = (xnorm2 == 0.f) && (alpha.i == 0.f);
         const float beta = trivial ? alpha.r : -copysignf(fsqrt<float>(fmaf(alpha.r, alpha.r, fmaf(alpha.i, alpha.i, xnorm2))), alpha.r);
@@ -662,11 +668,15 @@ __device__ __forceinline__ void hess_group(const int n, const SmemMat &H, float2
             scale = cinv(mk(alpha.r - beta, alpha.i));
         }
         __syncwarp(mask);  // every lane has read alpha and its x element
-        if (j >= i + 2 && j <= n) H.st(j, i, cmul(xk, scale));
+#pragma unroll
+        for (int t = 0; t < NJ; ++t) {
+            const int j = gl + 1 + t * G;
+            if (j >= i + 2 && j <= n) H.st(j, i, cmul(xk[t], scale));
+        }
         if (gl == 0) sTau[i - 1] = make_float2(t.r, t.i);
         __syncwarp(mask);
         // right: row j of A(1:n, i+1:n) -= tau (A v)_j v^H
-        if (j <= n) {
+        for (int j = gl + 1; j <= n; j += G) {
             cx<float> sacc = H.ld(j, i + 1);
             for (int q = 2; q <= mm; ++q) sacc = cmac(sacc, H.ld(j, i + q), H.ld(i + q, i));
             const cx<float> ts = cmul(t, sacc);
@@ -675,7 +685,8 @@ __device__ __forceinline__ void hess_group(const int n, const SmemMat &H, float2
         }
         __syncwarp(mask);
         // left: column j of A(i+1:n, i+1:n) -= conj(tau) v (v^H A)_j
-        if (j >= i + 1 && j <= n) {
+        for (int j = gl + 1; j <= n; j += G) {
+            if (j < i + 1) continue;
             const cx<float> tcj = conj(t);
             cx<float> sacc = H.ld(i + 1, j);
             for (int q = 2; q <= mm; ++q) sacc = cjmac(sacc, H.ld(i + q, i), H.ld(i + q, j));

@@ -240,23 +240,25 @@ __global__ void __launch_bounds__(kSchurThreads) schur32_kernel(const MixedArgs 
 // the T-eigenvectors X go to the per-matrix buffer layout read by
 // refine_kernel.
 // ---------------------------------------------------------------------------
-constexpr int kWarpSchurThreads = 128;  // 4 warps per block
+// a lane owns NJ rows and columns: j, j + G, ... (n <= NJ G); one warp per block
+// for NJ > 1, whose matrices fill the shared memory a few at a time
+template <int NJ> struct WarpSchur { static constexpr int threads = NJ > 1 ? 32 : 128; };
 
 // per-matrix buffer layout: T, Z, X (n*n float2 each, column-major), a work
 // vector whose first entry holds ||A||_F^2, then Ah and Al (n*n each)
 __host__ __device__ __forceinline__ long long mat_elems(int n) { return 5LL * n * n + n; }
 
-__host__ __device__ __forceinline__ size_t warp_schur_smem(int n, int G)
+__host__ __device__ __forceinline__ size_t warp_schur_smem(int n, int G, int threads)
 {
-    return (size_t)(kWarpSchurThreads / G) * (2 * n * (n + 1) + n) * sizeof(float2);
+    return (size_t)(threads / G) * (2 * n * (n + 1) + n) * sizeof(float2);
 }
 
-template <int G>
-__global__ void __launch_bounds__(kWarpSchurThreads) schur32_warp_kernel(const MixedArgs a, float2 *buf, int *flags)
+template <int G, int NJ = 1>
+__global__ void __launch_bounds__(WarpSchur<NJ>::threads) schur32_warp_kernel(const MixedArgs a, float2 *buf, int *flags)
 {
     extern __shared__ float2 wsm[];
+    constexpr int kThreads = WarpSchur<NJ>::threads;
     const int n = a.g.n, tc = a.g.tc;
-    const long long N = a.g.N;
     const int gl = threadIdx.x & (G - 1), wib = threadIdx.x / G;  // lane in group, group in block
     const unsigned gmask = group_mask<G>(threadIdx.x & 31);
     const int lda = n + 1;
@@ -264,9 +266,8 @@ __global__ void __launch_bounds__(kWarpSchurThreads) schur32_warp_kernel(const M
     float2 *sZ = sH + n * lda, *sTau = sZ + n * lda;
     const SmemMat H{sH, lda}, Z{sZ, lda};
     const long long nn = (long long)n * n;
-    const long long gw = (long long)blockIdx.x * (kWarpSchurThreads / G) + wib;
-    const long long nw = (long long)gridDim.x * (kWarpSchurThreads / G);
-    const int j = gl + 1;  // the row / column this lane owns
+    const long long gw = (long long)blockIdx.x * (kThreads / G) + wib;
+    const long long nw = (long long)gridDim.x * (kThreads / G);
     const float ulp = lim<float>::eps();
     const float smlnum = lim<float>::tiny() * ((float)n / ulp);
 
@@ -291,31 +292,43 @@ __global__ void __launch_bounds__(kWarpSchurThreads) schur32_warp_kernel(const M
         int status = 0, sweeps = 0;
         __syncwarp(gmask);
         if (!fb) {
-            hess_group<G>(n, H, sTau, gl, gmask);
+            hess_group<G, NJ>(n, H, sTau, gl, gmask);
             // ---- zung2r: Z = Q from the reflectors, last reflector first
             for (int i = n - 1; i >= 1; --i) {
                 const cx<float> t = mk(sTau[i - 1].x, sTau[i - 1].y);
                 const int c = i + 1;
-                if (j >= c + 1 && j <= n) {
-                    cx<float> sacc = Z.ld(c, j);
-                    for (int k = c + 1; k <= n; ++k) sacc = cjmac(sacc, H.ld(k, i), Z.ld(k, j));
-                    const cx<float> ts = cmul(t, sacc);
-                    Z.st(c, j, csub(Z.ld(c, j), ts));
-                    for (int k = c + 1; k <= n; ++k) Z.st(k, j, cnmac(Z.ld(k, j), H.ld(k, i), ts));
+#pragma unroll
+                for (int t_ = 0; t_ < NJ; ++t_) {
+                    const int j = gl + 1 + t_ * G;
+                    if (j >= c + 1 && j <= n) {
+                        cx<float> sacc = Z.ld(c, j);
+                        for (int k = c + 1; k <= n; ++k) sacc = cjmac(sacc, H.ld(k, i), Z.ld(k, j));
+                        const cx<float> ts = cmul(t, sacc);
+                        Z.st(c, j, csub(Z.ld(c, j), ts));
+                        for (int k = c + 1; k <= n; ++k) Z.st(k, j, cnmac(Z.ld(k, j), H.ld(k, i), ts));
+                    }
                 }
                 __syncwarp(gmask);
-                if (j >= c + 1 && j <= n) Z.st(j, c, cmul(H.ld(j, i), mk(-t.r, -t.i)));
-                if (j == c) Z.st(c, c, mk(1.f - t.r, -t.i));
-                if (j >= 2 && j <= c - 1) Z.st(j, c, mk(0.f, 0.f));
+#pragma unroll
+                for (int t_ = 0; t_ < NJ; ++t_) {
+                    const int j = gl + 1 + t_ * G;
+                    if (j >= c + 1 && j <= n) Z.st(j, c, cmul(H.ld(j, i), mk(-t.r, -t.i)));
+                    if (j == c) Z.st(c, c, mk(1.f - t.r, -t.i));
+                    if (j >= 2 && j <= c - 1) Z.st(j, c, mk(0.f, 0.f));
+                }
                 __syncwarp(gmask);
             }
-            if (j <= n) {
-                Z.st(j, 1, mk(j == 1 ? 1.f : 0.f, 0.f));
-                if (j > 1) Z.st(1, j, mk(0.f, 0.f));
+#pragma unroll
+            for (int t_ = 0; t_ < NJ; ++t_) {
+                const int j = gl + 1 + t_ * G;
+                if (j <= n) {
+                    Z.st(j, 1, mk(j == 1 ? 1.f : 0.f, 0.f));
+                    if (j > 1) Z.st(1, j, mk(0.f, 0.f));
+                }
+                // clear below the subdiagonal: column j, rows j+2..n
+                if (j <= n)
+                    for (int k = j + 2; k <= n; ++k) H.st(k, j, mk(0.f, 0.f));
             }
-            // clear below the subdiagonal: column j, rows j+2..n
-            if (j <= n)
-                for (int k = j + 2; k <= n; ++k) H.st(k, j, mk(0.f, 0.f));
             __syncwarp(gmask);
             // ---- make the subdiagonal real
             for (int i = 2; i <= n; ++i) {
@@ -325,11 +338,19 @@ __global__ void __launch_bounds__(kWarpSchurThreads) schur32_warp_kernel(const M
                     sc = cscal(conj(sc), frcp<float>(cabs(sc)));
                     __syncwarp(gmask);
                     if (gl == 0) H.st(i, i - 1, mk(cabs(h), 0.f));
-                    if (j >= i && j <= n) H.st(i, j, cmul(H.ld(i, j), sc));
+#pragma unroll
+                    for (int t_ = 0; t_ < NJ; ++t_) {
+                        const int j = gl + 1 + t_ * G;
+                        if (j >= i && j <= n) H.st(i, j, cmul(H.ld(i, j), sc));
+                    }
                     __syncwarp(gmask);
                     const int re = (i + 1) < n ? (i + 1) : n;
-                    if (j <= re) H.st(j, i, cmulc(H.ld(j, i), sc));
-                    if (j <= n) Z.st(j, i, cmulc(Z.ld(j, i), sc));
+#pragma unroll
+                    for (int t_ = 0; t_ < NJ; ++t_) {
+                        const int j = gl + 1 + t_ * G;
+                        if (j <= re) H.st(j, i, cmulc(H.ld(j, i), sc));
+                        if (j <= n) Z.st(j, i, cmulc(Z.ld(j, i), sc));
+                    }
                 }
                 __syncwarp(gmask);
             }
@@ -355,28 +376,36 @@ __global__ void __launch_bounds__(kWarpSchurThreads) schur32_warp_kernel(const M
                     zlarfg2<float>(a0, a1, t1);
                     const cx<float> w1 = a1, cw = conj(w1), c1 = conj(t1);
                     const float t2 = fmaf(t1.r, w1.r, -(t1.i * w1.i));
-                    if (j >= K && j <= n) {  // rows K, K+1, column j
-                        cx<float> h1 = H.ld(K, j), h2 = H.ld(K + 1, j);
-                        rot_pair(h1, h2, c1, t2, w1);
-                        H.st(K, j, h1);
-                        H.st(K + 1, j, h2);
+#pragma unroll
+                    for (int t_ = 0; t_ < NJ; ++t_) {
+                        const int j = gl + 1 + t_ * G;
+                        if (j >= K && j <= n) {  // rows K, K+1, column j
+                            cx<float> h1 = H.ld(K, j), h2 = H.ld(K + 1, j);
+                            rot_pair(h1, h2, c1, t2, w1);
+                            H.st(K, j, h1);
+                            H.st(K + 1, j, h2);
+                        }
                     }
                     __syncwarp(gmask);
                     // the reflector's entries in column K-1, stored once every lane has
                     // read them (the row update above does not touch that column)
                     if (K > L && gl == 0) { H.st(K, K - 1, a0); H.st(K + 1, K - 1, mk(0.f, 0.f)); }
                     const int je = (K + 2) < I ? (K + 2) : I;
-                    if (j <= je) {  // columns K, K+1, row j
-                        cx<float> h1 = H.ld(j, K), h2 = H.ld(j, K + 1);
-                        rot_pair(h1, h2, t1, t2, cw);
-                        H.st(j, K, h1);
-                        H.st(j, K + 1, h2);
-                    }
-                    if (j <= n) {  // Schur vectors, row j
-                        cx<float> z1 = Z.ld(j, K), z2 = Z.ld(j, K + 1);
-                        rot_pair(z1, z2, t1, t2, cw);
-                        Z.st(j, K, z1);
-                        Z.st(j, K + 1, z2);
+#pragma unroll
+                    for (int t_ = 0; t_ < NJ; ++t_) {
+                        const int j = gl + 1 + t_ * G;
+                        if (j <= je) {  // columns K, K+1, row j
+                            cx<float> h1 = H.ld(j, K), h2 = H.ld(j, K + 1);
+                            rot_pair(h1, h2, t1, t2, cw);
+                            H.st(j, K, h1);
+                            H.st(j, K + 1, h2);
+                        }
+                        if (j <= n) {  // Schur vectors, row j
+                            cx<float> z1 = Z.ld(j, K), z2 = Z.ld(j, K + 1);
+                            rot_pair(z1, z2, t1, t2, cw);
+                            Z.st(j, K, z1);
+                            Z.st(j, K + 1, z2);
+                        }
                     }
                     __syncwarp(gmask);
                 }
@@ -387,9 +416,13 @@ __global__ void __launch_bounds__(kWarpSchurThreads) schur32_warp_kernel(const M
                     const cx<float> z = conj(cscal(h, frcp<float>(d)));
                     __syncwarp(gmask);
                     if (gl == 0) H.st(I, I - 1, mk(d, 0.f));
-                    if (j >= I + 1 && j <= n) H.st(I, j, cmul(H.ld(I, j), z));
-                    if (j <= I - 1) H.st(j, I, cmulc(H.ld(j, I), z));
-                    if (j <= n) Z.st(j, I, cmulc(Z.ld(j, I), z));
+#pragma unroll
+                    for (int t_ = 0; t_ < NJ; ++t_) {
+                        const int j = gl + 1 + t_ * G;
+                        if (j >= I + 1 && j <= n) H.st(I, j, cmul(H.ld(I, j), z));
+                        if (j <= I - 1) H.st(j, I, cmulc(H.ld(j, I), z));
+                        if (j <= n) Z.st(j, I, cmulc(Z.ld(j, I), z));
+                    }
                 }
                 __syncwarp(gmask);
             }
@@ -405,13 +438,17 @@ __global__ void __launch_bounds__(kWarpSchurThreads) schur32_warp_kernel(const M
             }
             __syncwarp(gmask);
             // T-eigenvectors: lane j solves column j into sZ (Z is saved)
-            if (j <= n) {
-                const SmemCol xc{sZ + (j - 1) * lda};
-                const cx<float> tkk = H.ld(j, j);
-                const float smin = fmaxf(ulp * cabs1(tkk), smlnum);
-                const float sc = j > 1 ? trevc_solve<float>(j, H, xc, smin, tkk) : 1.f;
-                xc.st(j, mk(sc, 0.f));
-                for (int i = j + 1; i <= n; ++i) xc.st(i, mk(0.f, 0.f));
+#pragma unroll
+            for (int t_ = 0; t_ < NJ; ++t_) {
+                const int j = gl + 1 + t_ * G;
+                if (j <= n) {
+                    const SmemCol xc{sZ + (j - 1) * lda};
+                    const cx<float> tkk = H.ld(j, j);
+                    const float smin = fmaxf(ulp * cabs1(tkk), smlnum);
+                    const float sc = j > 1 ? trevc_solve<float>(j, H, xc, smin, tkk) : 1.f;
+                    xc.st(j, mk(sc, 0.f));
+                    for (int i = j + 1; i <= n; ++i) xc.st(i, mk(0.f, 0.f));
+                }
             }
             __syncwarp(gmask);
             for (int e = gl; e < nn; e += G) out[2 * nn + e] = sZ[(e % n) + (e / n) * lda];
@@ -1097,20 +1134,30 @@ namespace {
 // the warp kernel at n = 17..32 (n=20 3.64 / 3.73, n=24 1.77 / 2.16, n=32
 // 0.58 / 0.95 M/s against 3.78, 2.42, 1.10).  Default now: G = 32 for
 // 17 <= n <= 32.
+// Small batches, and n > 32 (two rows and columns per lane): a lane kernel's wave
+// takes 0.5 ms at n=9, 3 ms at n=16, 175 ms at n=64 however few matrices there
+// are, and above n=32 it is the slower one at every size.  ms, lane -> chosen:
+// 512 matrices n=9 0.523 -> 0.251 (G = 16), n=16 (group, G = 8) 0.610 -> 0.476
+// (G = 32); 8,192 n=9 0.634 -> 0.415 (group, G = 8); n=48 512 73.6 -> 4.88, 8,192
+// 147 -> 43.3; n=64 512 176 -> 12.4, 8,192 365 -> 110; n=40 32,768 192 -> 78.
+// At 32,768 n=9 the lane kernel is ahead again (1.24 against 1.28).
+// The choice goes by the whole batch, so chunks of it take the same kernel.
 // VES_MIXED_SCHUR overrides (tests and tuning): lane; warp (G = 16 for
-// n <= 16, G = 32 for n <= 32); warp16; warp32.
-int schur_group(int n)
+// n <= 16, G = 32 above); warp16; warp32; warp64 (G = 32 for any n).
+int schur_group(int n, long long N)
 {
     const char *e = getenv("VES_MIXED_SCHUR");  // read per launch: a getenv is cheap next to a solve
     if (e && !strcmp(e, "lane")) return 0;
-    if (e && !strcmp(e, "warp")) return n <= 16 ? 16 : (n <= 32 ? 32 : 0);
+    if (e && !strcmp(e, "warp")) return n <= 16 ? 16 : 32;
     if (e && !strcmp(e, "warp16")) return n <= 16 ? 16 : 0;
     if (e && !strcmp(e, "warp32")) return n <= 32 ? 32 : 0;
+    if (e && !strcmp(e, "warp64")) return 32;
     if (e && !strcmp(e, "group4")) return n <= 16 ? 4 : 0;
     if (e && !strcmp(e, "group8")) return n <= 16 ? 8 : 0;
-    if (n >= 11 && n <= 14) return 4;
-    if (n >= 15 && n <= 16) return 8;
-    return (n >= 17 && n <= 32) ? 32 : 0;
+    if (n >= 17) return 32;
+    if (N <= 4096) return n <= 6 ? 8 : n <= 12 ? 16 : 32;
+    if (N <= 16384) return 8;
+    return n <= 10 ? 0 : n <= 14 ? 4 : 8;
 }
 
 template <int G>
@@ -1131,22 +1178,22 @@ long long group_schur_blocks(int n, long long N, int blocks_per_sm)
     return std::max<long long>(1, std::min<long long>(need, (long long)sms * per_sm));
 }
 
-template <int G>
-long long warp_schur_blocks(int n, long long N, int blocks_per_sm)
+template <int G, int NJ = 1>
+cudaError_t launch_warp_schur(const MixedArgs &a, float2 *buf, int *flags, long long N, int blocks_per_sm,
+                              cudaStream_t st)
 {
-    // per call (per device, thread safe; microseconds next to the kernel)
-    cudaFuncSetAttribute(schur32_warp_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)warp_schur_smem(G, G));
-    const int sms = device_sms();
+    constexpr int threads = WarpSchur<NJ>::threads;
+    const size_t smem = warp_schur_smem(a.g.n, G, threads);
     int per_sm = blocks_per_sm;
     if (per_sm <= 0) {
         per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, schur32_warp_kernel<G>, kWarpSchurThreads,
-                                                      warp_schur_smem(n, G));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, schur32_warp_kernel<G, NJ>, threads, smem);
         if (per_sm < 1) per_sm = 1;
     }
-    const long long need = (N + kWarpSchurThreads / G - 1) / (kWarpSchurThreads / G);
-    return std::max<long long>(1, std::min<long long>(need, (long long)sms * per_sm));
+    const long long need = (N + threads / G - 1) / (threads / G);
+    const long long blocks = std::max<long long>(1, std::min<long long>(need, (long long)device_sms() * per_sm));
+    schur32_warp_kernel<G, NJ><<<(unsigned)blocks, threads, smem, st>>>(a, buf, flags);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -1172,7 +1219,7 @@ cudaError_t launch_schur(const MixedArgs &a, int blocks_per_sm, cudaStream_t st)
     const int n = a.g.n;
     const long long cnt = a.m_end - a.m_begin;
     const MixedBufs b = mixed_bufs(a);
-    const int G = schur_group(n);
+    const int G = schur_group(n, a.g.N);
     if (G == 4)
         schur32_group_kernel<4><<<(unsigned)group_schur_blocks<4>(n, cnt, blocks_per_sm), kGroupSchurThreads,
                                   group_schur_smem(n, 4), st>>>(a, b.buf, b.flags);
@@ -1180,11 +1227,10 @@ cudaError_t launch_schur(const MixedArgs &a, int blocks_per_sm, cudaStream_t st)
         schur32_group_kernel<8><<<(unsigned)group_schur_blocks<8>(n, cnt, blocks_per_sm), kGroupSchurThreads,
                                   group_schur_smem(n, 8), st>>>(a, b.buf, b.flags);
     else if (G == 16)
-        schur32_warp_kernel<16><<<(unsigned)warp_schur_blocks<16>(n, cnt, blocks_per_sm), kWarpSchurThreads,
-                                  warp_schur_smem(n, 16), st>>>(a, b.buf, b.flags);
+        return launch_warp_schur<16>(a, b.buf, b.flags, cnt, blocks_per_sm, st);
     else if (G == 32)
-        schur32_warp_kernel<32><<<(unsigned)warp_schur_blocks<32>(n, cnt, blocks_per_sm), kWarpSchurThreads,
-                                  warp_schur_smem(n, 32), st>>>(a, b.buf, b.flags);
+        return n <= 32 ? launch_warp_schur<32>(a, b.buf, b.flags, cnt, blocks_per_sm, st)
+                       : launch_warp_schur<32, 2>(a, b.buf, b.flags, cnt, 0, st);
     else
         schur32_kernel<<<(unsigned)schur_blocks(cnt, blocks_per_sm), kSchurThreads, 0, st>>>(a, b.buf, b.flags);
     return cudaGetLastError();
@@ -1203,11 +1249,13 @@ cudaError_t launch_refine(const MixedArgs &a, cudaStream_t st)
         if (v >= 1 && v <= 32) tiles = std::min<long long>(tiles, (long long)device_sms() * v);
     }
     const unsigned rb = (unsigned)std::max<long long>(1, tiles);
-    if (schur_group(n)) {  // per-matrix buffer layout
+    if (schur_group(n, a.g.N)) {  // per-matrix buffer layout
         if (n <= 16)
             refine_kernel<16, true><<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
-        else
+        else if (n <= 32)
             refine_kernel<32, true><<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
+        else
+            refine_kernel<64, true><<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
     } else if (n <= 16) {
         refine16_lane_kernel<<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
     } else if (n <= 32) {
@@ -1223,7 +1271,7 @@ cudaError_t launch_dupcheck(const MixedArgs &a, cudaStream_t st)
 {
     const MixedBufs b = mixed_bufs(a);
     const unsigned blocks = (unsigned)((a.m_end - a.m_begin + 127) / 128);
-    if (schur_group(a.g.n))
+    if (schur_group(a.g.n, a.g.N))
         dupcheck_kernel<true><<<blocks, 128, 0, st>>>(a, b.buf, b.flags);
     else
         dupcheck_kernel<false><<<blocks, 128, 0, st>>>(a, b.buf, b.flags);
@@ -1271,7 +1319,7 @@ cudaError_t launch_mixed_overlap(const MixedArgs &a0, cudaStream_t st, cudaStrea
     // n=16 5.10 -> 5.87 M/s, n=24 1.63 -> 1.72 M/s, n=32 0.726 -> 0.846 M/s);
     // VES_MIXED_OVERLAP_BLOCKS_PER_SM overrides
     // (the group kernel: as many as shared memory holds)
-    const int G = schur_group(a.g.n);
+    const int G = schur_group(a.g.n, a.g.N);
     int bps = a.blocks_per_sm > 0 ? a.blocks_per_sm : (G == 4 || G == 8 ? 0 : (G ? 6 : 4));
     if (a.blocks_per_sm <= 0)
         if (const char *ev = getenv("VES_MIXED_OVERLAP_BLOCKS_PER_SM")) {
@@ -1332,6 +1380,11 @@ void load_mixed_kernels()
     load_kernel(schur32_warp_kernel<32>);
     load_kernel(refine_kernel<32, true>);
     load_kernel(schur32_warp_kernel<16>);
+    load_kernel(schur32_warp_kernel<32, 2>);
+    load_kernel(refine_kernel<64, true>);
+    cudaFuncSetAttribute(schur32_warp_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_schur_smem(16, 16, 128));
+    cudaFuncSetAttribute(schur32_warp_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_schur_smem(32, 32, 128));
+    cudaFuncSetAttribute(schur32_warp_kernel<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_schur_smem(64, 32, 32));
     load_kernel(refine_kernel<16, true>);
     load_kernel(schur32_group_kernel<8>);
     load_kernel(schur32_group_kernel<4>);
