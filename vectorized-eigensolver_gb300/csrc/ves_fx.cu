@@ -53,29 +53,30 @@ __global__ void __launch_bounds__(FxShape<G>::threads) fx_kernel(const FxArgs a)
     }
 }
 
-// One matrix per lane, 32 in lockstep, H, Z and U in the warp's workspace
-// ([element][lane], as in the FP64 lane kernel): the FP64 steps of a rotation
-// serve 32 matrices per instruction.
+// One matrix per lane, or per G lanes, the warp's 32 / G matrices in lockstep,
+// H, Z and U in the warp's workspace ([element][matrix]): the FP64 steps of a
+// rotation serve all of them.  kShifts: with predicted shifts (G = 1), whose
+// storage follows U in the slot.
 constexpr int kLaneThreads = 128;
-// kShifts: with predicted shifts, whose storage follows U in the slot.
-template <bool kVec, bool kShifts>
+template <int G, bool kVec, bool kShifts>
 __device__ __forceinline__ void fx_lanes(const FxArgs &a)
 {
-    __shared__ longlong2 chs[kLaneThreads * kFxChunk];
-    __shared__ i64 chi[kLaneThreads * kFxChunk];
-    const FxGroup<1> gr;
-    const int n = a.g.n, tc = a.g.tc, lane = threadIdx.x & 31;
-    const int ch0 = (threadIdx.x >> 5) * 32 * kFxChunk + lane;
+    constexpr int kChunk = FxChunkOf<G>::k, M = 32 / G;
+    __shared__ longlong2 chs[kLaneThreads * kChunk];
+    __shared__ i64 chi[kLaneThreads * kChunk];
+    const FxLanes<G> gr;
+    const int n = a.g.n, tc = a.g.tc, lane = threadIdx.x & 31, mat = lane % M;
+    const int ch0 = (threadIdx.x >> 5) * 32 * kChunk + lane;
     const FxChunk ch{chs + ch0, chi + ch0};
     const long long slot = (long long)blockIdx.x * (kLaneThreads / 32) + (threadIdx.x >> 5);
     const long long nslots = (long long)gridDim.x * (kLaneThreads / 32);
     const long long nn = (long long)n * n, nu = (kVec ? 2 : 1) * nn;
-    longlong2 *base = static_cast<longlong2 *>(a.ws) + slot * (kShifts ? shift_slot_elems(n) : nu + n) * 32 + lane;
-    const FxMat<32> H{base, n, n}, Z{base + (kVec ? nn * 32 : 0), n, n};
-    const FxVec<32> U{base + nu * 32};
+    longlong2 *base = static_cast<longlong2 *>(a.ws) + slot * (kShifts ? shift_slot_elems(n) : nu + n) * M + mat;
+    const FxMat<M> H{base, n, n}, Z{base + (kVec ? nn * M : 0), n, n};
+    const FxVec<M> U{base + nu * M};
     const long long Nw = a.list ? (long long)*a.list_count : a.g.N;
-    for (long long base_w = slot * 32; base_w < Nw; base_w += nslots * 32) {
-        const long long w = base_w + lane;
+    for (long long base_w = slot * M; base_w < Nw; base_w += nslots * M) {
+        const long long w = base_w + mat;
         const bool valid = w < Nw;
         const long long m = !valid ? 0 : a.list ? (long long)a.list[w] : a.m_begin + w;
         const long long mo = (m / tc) * (long long)tc * n * n + m % tc, vo = (m / tc) * (long long)tc * n + m % tc;
@@ -104,10 +105,10 @@ __device__ __forceinline__ void fx_lanes(const FxArgs &a)
             if (sh.sp.fallbacks) status |= ST_SHIFT_FALLBACK;
             if (ok && a.fallbacks) a.fallbacks[m] = sh.sp.fallbacks;
         } else {
-            ok = fx_solve<1, kVec>(gr, n, H, Z, U, valid, a.rA + mo, a.iA + mo, tc, o, a.max_its, a.vnorm, sweeps,
+            ok = fx_solve<G, kVec>(gr, n, H, Z, U, valid, a.rA + mo, a.iA + mo, tc, o, a.max_its, a.vnorm, sweeps,
                                    status, ch);
         }
-        if (valid) {
+        if (valid && gr.gl == 0) {
             if (ok) {
                 if (a.status) a.status[m] = status | a.status_or;
                 if (a.sweeps) a.sweeps[m] = sweeps;
@@ -117,11 +118,11 @@ __device__ __forceinline__ void fx_lanes(const FxArgs &a)
         }
     }
 }
-template <bool kVec> __global__ void __launch_bounds__(kLaneThreads, 4) fx_lane_kernel(const FxArgs a)
+template <int G, bool kVec> __global__ void __launch_bounds__(kLaneThreads, 4) fx_lane_kernel(const FxArgs a)
 {
-    fx_lanes<kVec, false>(a);
+    fx_lanes<G, kVec, false>(a);
 }
-__global__ void __launch_bounds__(kLaneThreads, 4) fx_shifts_kernel(const FxArgs a) { fx_lanes<true, true>(a); }
+__global__ void __launch_bounds__(kLaneThreads, 4) fx_shifts_kernel(const FxArgs a) { fx_lanes<1, true, true>(a); }
 
 int fx_sms()
 {
@@ -166,29 +167,48 @@ template <bool kVec> cudaError_t launch_fx_v(const FxArgs &a, int G, cudaStream_
 
 }  // namespace
 
-// Lanes per matrix: 0 = the lane kernel, whose 32 matrices share every FP64
-// instruction but take long for one wave; otherwise a group of G lanes per
-// matrix in shared memory, faster per matrix with more lanes but with fewer
-// matrices resident.  The rule takes the smallest estimated time:
-//   group  waves * 0.33 ms (n/8)^1.85 (1 + n / (3 G)), and for G > 32, whose
+// Which kernel, and how many lanes per matrix.  The lane kernel's warps hold
+// 32 / G matrices in the workspace (G = 1, 2, 4, 8) and share the FP64 steps;
+// the group kernel keeps a matrix in shared memory (G = 4 .. 128).  More lanes
+// finish a matrix sooner; fewer waste less.  The rule takes the smallest
+// estimated time, x = n / 8:
+//   lanes  (0.07 + 1.05 x^2.66) ms r (1 + c w) for a wave of w * 2,432 warps, r =
+//          a + (1 - a) / G, a = 1.9 / n^0.62 the share of a rotation that all
+//          lanes repeat, c = 1.5, 1.2, 1.3, 0.8 for G = 1, 2, 4, 8
+//   group  waves * 0.33 ms x^1.85 (1 + n / (3 G)), and for G > 32, whose
 //          warps repeat the FP64 steps, 3% per warp on the SM
-//   lane   1.05 ms (n/8)^2.66 (1 + N n / 1.2e6) for one wave of 2,432 warps
-// Measured on GB300, ms (lane; G = 4, 8, 16, 32): n=16, N=64 6.35; 2.41 1.70
-// 1.35 1.19.  N=2,048 6.84; 2.57 1.85 1.68 2.47.  N=8,192 6.94; 7.43 5.65
-// 5.69 9.40.  N=16,384 8.05; 12.3 9.5 10.2 18.5.  n=32 (G = 16, 32, 64), N=64
-// 41.5; 6.05 4.83 4.28, N=8,192 54.7; 53.8 47.7 65.2.  n=64 (G = 64, 128),
-// N=512 299; 68.2 64.1.  Without vectors about half the lane kernel's time and
-// 0.9 of the group's.  Over 60 (n, N) from 4 to 64 and 64 to 65,536 the choice
-// is on average 2% from the best of all.
-int fx_group_size(int n, long long N, bool vec)
+// Measured on GB300, ms.  Lanes G = 1, 2, 4, 8: n=16, N=96 6.35 5.35 3.86 3.02,
+// N=16,384 8.05 6.97 7.21 11.8, N=65,536 14.3 20.3 33.2 49.1; n=32, N=4,096 48 36.0
+// 23.6 19.3, N=16,384 59.5 48.9 40.5 59.9; n=64, N=96 292 207 123 80, N=4,096
+// 360 278 174 135.  Group G = 4, 8, 16, 32: n=16, N=64 2.41 1.70 1.35 1.19,
+// N=2,048 2.57 1.85 1.68 2.47, N=8,192 7.43 5.65 5.69 9.40; G = 16, 32, 64: n=32,
+// N=64 6.05 4.83 4.28, N=8,192 53.8 47.7 65.2; G = 64, 128: n=64, N=512 68.2 64.1.
+// Without vectors half the lane kernel's time and 0.9 of the group's.
+struct FxChoice {
+    bool lanes;
+    int G;
+};
+FxChoice fx_choose(int n, long long N, bool vec)
 {
-    if (const char *e = getenv("VES_FX_LANES")) {  // tuning
-        const int v = atoi(e);
-        if (v == 0 || (v >= 4 && v <= 128 && (v & (v - 1)) == 0)) return v;
+    if (const char *e = getenv("VES_FX_LANES")) {  // tuning: 1, 2, 4, 8 lanes ("l4"), or a group of 4 .. 128 ("g16")
+        const int v = atoi(e + (*e != 0));
+        if (e[0] == 'l' && (v == 1 || v == 2 || v == 4 || v == 8)) return {true, v};
+        if (e[0] == 'g' && v >= 4 && v <= 128 && (v & (v - 1)) == 0) return {false, v};
     }
     const double sms = fx_sms(), x = n / 8.0;
-    int best = 0;
-    double t = (vec ? 1.05 : 0.52) * pow(x, 2.66) * (1.0 + (double)N * n / (vec ? 1.2e6 : 2e6));
+    FxChoice best{true, 1};
+    double t = 1e300;
+    const double lat = (vec ? 0.07 : 0.08) + (vec ? 1.05 : 0.52) * pow(x, 2.66), a = std::min(1.0, (vec ? 1.9 : 3.0) / pow(n, 0.62));
+    const double c[4] = {vec ? 1.5 : 1.0, 1.2, 1.3, 0.8};
+    for (int k = 0; k < 4; ++k) {
+        const int G = 1 << k;
+        const double w = (double)N * G / 32 / (sms * 16), full = floor(w);
+        const double tl = lat * (a + (1 - a) / G) * (full * (1 + c[k]) + (w > full ? 1 + c[k] * (w - full) : 0));
+        if (tl < t) {
+            t = tl;
+            best = {true, G};
+        }
+    }
     for (int G = 4; G <= 128; G *= 2) {
         if (G > 32 ? G > 2 * n : G > 4 * n) break;
         const int mats = G < 32 ? 32 / G : 1;
@@ -199,16 +219,28 @@ int fx_group_size(int n, long long N, bool vec)
         if (G > 32) tg *= 1.0 + 0.03 * std::min(fit, ceil((double)N / (sms * mats))) * G / 32;
         if (tg < t) {
             t = tg;
-            best = G;
+            best = {false, G};
         }
     }
     return best;
 }
 
-cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, cudaStream_t st)
+template <int G> static void launch_fx_lanes_g(const FxArgs &a, bool vec, cudaStream_t st)
 {
-    if (vec) fx_lane_kernel<true><<<a.lane_blocks, kLaneThreads, 0, st>>>(a);
-    else fx_lane_kernel<false><<<a.lane_blocks, kLaneThreads, 0, st>>>(a);
+    // G times the warps in the same workspace, at most the four blocks that fit an SM
+    const long long per_block = kLaneThreads / G;
+    long long blocks = std::min<long long>((a.g.N + per_block - 1) / per_block, (long long)a.lane_blocks * G);
+    if (G > 1) blocks = std::min<long long>(blocks, std::max(a.lane_blocks, fx_sms() * 4));
+    if (vec) fx_lane_kernel<G, true><<<(unsigned)blocks, kLaneThreads, 0, st>>>(a);
+    else fx_lane_kernel<G, false><<<(unsigned)blocks, kLaneThreads, 0, st>>>(a);
+}
+
+cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, int G, cudaStream_t st)
+{
+    if (G == 2) launch_fx_lanes_g<2>(a, vec, st);
+    else if (G == 4) launch_fx_lanes_g<4>(a, vec, st);
+    else if (G == 8) launch_fx_lanes_g<8>(a, vec, st);
+    else launch_fx_lanes_g<1>(a, vec, st);
     return cudaGetLastError();
 }
 
@@ -222,9 +254,9 @@ cudaError_t launch_fx(const FxArgs &a, bool vec, cudaStream_t st)
 {
     if (a.g.N <= 0) return cudaSuccess;
     if (!fx_order(a.g.n)) return cudaErrorInvalidValue;
-    const int G = fx_group_size(a.g.n, a.g.N, vec);
-    if (G == 0) return launch_fx_lanes(a, vec, st);
-    return vec ? launch_fx_v<true>(a, G, st) : launch_fx_v<false>(a, G, st);
+    const FxChoice c = fx_choose(a.g.n, a.g.N, vec);
+    if (c.lanes) return launch_fx_lanes(a, vec, c.G, st);
+    return vec ? launch_fx_v<true>(a, c.G, st) : launch_fx_v<false>(a, c.G, st);
 }
 
 template <int G> static void load_fx_g()
@@ -236,8 +268,14 @@ template <int G> static void load_fx_g()
 }
 void load_fx_kernels()
 {
-    load_kernel(fx_lane_kernel<true>);
-    load_kernel(fx_lane_kernel<false>);
+    load_kernel(fx_lane_kernel<1, true>);
+    load_kernel(fx_lane_kernel<1, false>);
+    load_kernel(fx_lane_kernel<2, true>);
+    load_kernel(fx_lane_kernel<2, false>);
+    load_kernel(fx_lane_kernel<4, true>);
+    load_kernel(fx_lane_kernel<4, false>);
+    load_kernel(fx_lane_kernel<8, true>);
+    load_kernel(fx_lane_kernel<8, false>);
     load_kernel(fx_shifts_kernel);
     load_fx_g<4>(); load_fx_g<8>(); load_fx_g<16>(); load_fx_g<32>(); load_fx_g<64>();
     load_fx_g<128>();

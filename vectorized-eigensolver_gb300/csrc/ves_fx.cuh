@@ -374,6 +374,41 @@ template <int G> struct FxGroup {
     }
 };
 
+// G lanes that own one matrix in a warp's workspace: the warp holds 32 / G
+// matrices, lane l works on matrix l % (32 / G), so that the lanes with one
+// index of their groups touch neighbouring matrices.
+// Its reductions and syncs are those of the whole warp: all 32 lanes call them.
+template <int G> struct FxLanes {
+    static constexpr int RG = G, M = 32 / G;
+    int gl, rl;
+    __device__ __forceinline__ FxLanes() : gl((threadIdx.x & 31) / M), rl(gl) {}
+    __device__ __forceinline__ void sync() const { __syncwarp(); }
+    template <class T, class F> __device__ __forceinline__ T fold(T v, F f) const
+    {
+#pragma unroll
+        for (int o = M; o < 32; o <<= 1) v = f(v, __shfl_xor_sync(FULL, v, o));
+        return v;
+    }
+    __device__ __forceinline__ bool all(bool p) const
+    {
+        return fold((int)p, [](int a, int b) { return a & b; });
+    }
+    __device__ __forceinline__ i64 sum(i64 v) const
+    {
+        return fold(v, [](i64 a, i64 b) { return a + b; });
+    }
+    __device__ __forceinline__ i64 orr(i64 v) const
+    {
+        return fold(v, [](i64 a, i64 b) { return a | b; });
+    }
+    __device__ __forceinline__ int maxi(int v) const
+    {
+        return fold(v, [](int a, int b) { return max(a, b); });
+    }
+};
+
+template <> struct FxLanes<1> : FxGroup<1> {};
+
 __host__ __device__ __forceinline__ int fx_lda(int n) { return n | 1; }
 // 16-byte elements of a matrix's slot in shared memory: H, Z (vectors only),
 // and n entries for the reflectors' first elements and the column scales;
@@ -403,8 +438,8 @@ struct FxOut {
 
 // Load A (element e of the column-major matrix at e * s) into H as integers.
 // Returns false for a matrix that is left to the FP64 kernels; unit = 2^(e-61).
-template <int G, int ST>
-__device__ __forceinline__ bool fx_load(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const bool valid,
+template <int G, class GR, int ST>
+__device__ __forceinline__ bool fx_load(const GR &gr, const int n, const FxMat<ST> &H, const bool valid,
                                         const double *rA, const double *iA, const long long s, double &unit)
 {
     unit = 1.0;
@@ -428,7 +463,7 @@ __device__ __forceinline__ bool fx_load(const FxGroup<G> &gr, const int n, const
     // ||A||_F^2 from above: |component| < (q + 1) 2^(emax - 1043), q its leading 21 bits
     i64 q2 = 0;
     FxIndex i1(gr.rl, n);
-    for (int e = gr.rl; e < n * n; e += FxGroup<G>::RG, i1.next(FxGroup<G>::RG, n)) {
+    for (int e = gr.rl; e < n * n; e += GR::RG, i1.next(GR::RG, n)) {
         const cx<double> v = H.ldd(i1.i, i1.j);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -455,7 +490,7 @@ __device__ __forceinline__ bool fx_load(const FxGroup<G> &gr, const int n, const
     gr.sync();
     // every row and column has an entry of at least 2^-9 of the scale
     bool ok = range;
-    for (int r = gr.rl + 1; r <= n; r += FxGroup<G>::RG) {
+    for (int r = gr.rl + 1; r <= n; r += GR::RG) {
         int mr = 0, mc = 0;
         for (int j = 1; j <= n; ++j) {
             const cx64 a = H.ld(r, j), b = H.ld(j, r);
@@ -572,10 +607,10 @@ __device__ __forceinline__ void fx_reflect_all(const int gl, longlong2 *a, const
 // Householder reduction to Hessenberg form with Hermitian reflectors
 // P = I - u u^H, ||u||^2 = 2 (the subdiagonal comes out complex).  u_k, k >=
 // i + 2, stays below the subdiagonal of column i, u_{i+1} in U(i).
-template <int G, int ST>
-__device__ __forceinline__ void fx_reduce(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxVec<ST> &U)
+template <int G, class GR, int ST>
+__device__ __forceinline__ void fx_reduce(const GR &gr, const int n, const FxMat<ST> &H, const FxVec<ST> &U)
 {
-    constexpr int RG = FxGroup<G>::RG;
+    constexpr int RG = GR::RG;
     const int rs = ST, cs = H.lda * ST;  // steps to the next row, the next column
     for (int i = 1; i <= n - 2; ++i) {
         const cx64 al = H.ld(i + 1, i);
@@ -630,8 +665,8 @@ __device__ __forceinline__ void fx_reduce(const FxGroup<G> &gr, const int n, con
 }
 
 // Z = P_1 P_2 ... P_{n-2} from the reflectors.
-template <int G, int ST>
-__device__ __forceinline__ void fx_form_q(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
+template <int G, class GR, int ST>
+__device__ __forceinline__ void fx_form_q(const GR &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
                                           const FxVec<ST> &U)
 {
     for (int c = gr.gl + 1; c <= n; c += G)
@@ -644,11 +679,11 @@ __device__ __forceinline__ void fx_form_q(const FxGroup<G> &gr, const int n, con
 }
 
 // no subdiagonal below 2^-30 of the scale
-template <int G, int ST>
-__device__ __forceinline__ bool fx_irreducible(const FxGroup<G> &gr, const int n, const FxMat<ST> &H)
+template <int G, class GR, int ST>
+__device__ __forceinline__ bool fx_irreducible(const GR &gr, const int n, const FxMat<ST> &H)
 {
     bool ok = true;
-    for (int k = gr.rl + 2; k <= n; k += FxGroup<G>::RG) ok = ok && fx_abs1(H.ld(k, k - 1)) >= (1LL << 31);
+    for (int k = gr.rl + 2; k <= n; k += GR::RG) ok = ok && fx_abs1(H.ld(k, k - 1)) >= (1LL << 31);
     return gr.all(ok);
 }
 
@@ -859,7 +894,9 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
 }
 
 // Rotations of the current chunk of a sweep, in shared memory, one set per lane.
+// (n=16, one lane per matrix, chunk 4, 8, 16: 277, 274, 260 ms per 1,048,576)
 constexpr int kFxChunk = 16;
+template <int G> struct FxChunkOf { static constexpr int k = G == 1 ? kFxChunk : 8; };
 constexpr int kFxStream = 2;  // chains streamed together
 struct FxChunk {
     longlong2 *cs;  // (c, sr) of rotation k at cs[k * 32]
@@ -882,8 +919,8 @@ struct FxChunk {
 // two rotations share stays in registers, so each entry is read and written
 // once per chunk.
 //
-// next (nullable): NB chains of the same shape, next_step apart per entry, that
-// the caller streams after these; their lines are brought into L2 meanwhile.
+// next (nullable): the chains that the caller streams after these; their lines
+// are brought into L2 meanwhile.
 // One rotation's entries ahead in registers, 16 warps keep 16 KB in flight per
 // SM, which against the latency of DRAM is 4.7 TB/s at most; with the lines
 // already in L2 the registers cover what is left.
@@ -926,34 +963,37 @@ __device__ __noinline__ void fx_stream(longlong2 *p, const int step, const int b
 #pragma unroll
     for (int b = 0; b < NB; ++b) p[b * blk] = make_longlong2(x[b].r, x[b].i);
 }
-__device__ __forceinline__ void fx_stream_all(longlong2 *p, const int step, const int blk, const int count,
-                                              const FxChunk &ch, const int ns, const bool col,
-                                              const longlong2 *next = nullptr, const int next_step = 0)
+template <int G>
+__device__ __forceinline__ void fx_stream_all(const int gl, longlong2 *p, const int step, const int blk, const int count,
+                                              const FxChunk &ch, const int ns, const bool col)
 {
-    int b = 0;
-    for (; b + kFxStream <= count; b += kFxStream) {
-        const bool more = b + 2 * kFxStream <= count;
-        fx_stream<kFxStream>(p + b * blk, step, blk, ch.cs, ch.si, ns, col, more ? p + (b + kFxStream) * blk : next,
-                             more ? step : next_step);
+    int b = G == 1 ? 0 : gl;  // chains gl, gl + G, ... of count
+    for (; b + kFxStream * G <= count + G - 1; b += kFxStream * G) {
+        const bool more = b + 2 * kFxStream * G <= count + G - 1;
+        fx_stream<kFxStream>(p + b * blk, step, G * blk, ch.cs, ch.si, ns, col, more ? p + (b + kFxStream * G) * blk : nullptr,
+                             more ? step : 0);
     }
-    for (; b < count; ++b) fx_stream<1>(p + b * blk, step, blk, ch.cs, ch.si, ns, col, nullptr, 0);
+    for (; b < count; b += G) fx_stream<1>(p + b * blk, step, blk, ch.cs, ch.si, ns, col, nullptr, 0);
 }
 
-// fx_qr for one matrix per lane, 32 in lockstep per sweep, in the warp's
-// workspace.  A sweep runs in chunks of kFxChunk rotations: first the chain of
+// fx_qr for one matrix per lane, or per G lanes of FxLanes, the warp's matrices
+// in lockstep per sweep, in its workspace.  The lanes of a matrix compute the
+// chain alike and share out the rows and columns.  A sweep runs in chunks of kFxChunk rotations: first the chain of
 // rotations, which needs of the matrix only the chunk's own columns (the left
 // rotations of the chunk are applied to column K + 1 when rotation K is due)
 // and the diagonal; then the chunk's rotations are streamed over the rows of Z,
 // the rows above and the columns to the right.  A lane whose window does not
 // contain K takes part with the identity, which leaves integers unchanged.
 // The entries see the same operations as in fx_qr.
-template <bool kVec, class SP>
-__device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, const FxMat<32> &Z, const FxVec<32> &S,
+template <int G, bool kVec, int ST, class SP>
+__device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, const FxMat<ST> &H, const FxMat<ST> &Z, const FxVec<ST> &S,
                                            const FxChunk &ch, const bool run, const int max_its, int &sweeps,
                                            int &status, SP *sp)
 {
-    const FxGroup<1> gr;
-    const int rs = 32, cs = n * 32;  // steps to the next row, the next column
+    const FxGroup<1> gr;  // a lane scans its matrix by itself
+    constexpr int kChunk = FxChunkOf<G>::k;
+    const int rs = ST, cs = n * ST;  // steps to the next row, the next column
+    const int gl = G == 1 ? 0 : group_lane;
     int I = n, L = 1, its = 0;
     bool done = !run || n <= 1;
     for (;;) {
@@ -966,8 +1006,8 @@ __device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, cons
         const int Kmin = __reduce_min_sync(FULL, sweep ? L : INT_MAX);
         const int Kmax = __reduce_max_sync(FULL, sweep ? I - 1 : 0);
         cx64 hkk = H.ld(Kmin, Kmin);
-        for (int Kc = Kmin; Kc <= Kmax; Kc += kFxChunk) {
-            const int Ke = min(Kc + kFxChunk - 1, Kmax), ns = Ke - Kc + 1;
+        for (int Kc = Kmin; Kc <= Kmax; Kc += kChunk) {
+            const int Ke = min(Kc + kChunk - 1, Kmax), ns = Ke - Kc + 1;
             for (int K = Kc; K <= Ke; ++K) {
                 const bool act = sweep && K >= L && K < I;
                 FxRot R;
@@ -993,9 +1033,11 @@ __device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, cons
                     v = pc[2 * rs];
                     w = pl[rs];
                     fx_pair(x, y, ch.get(q - Kc));
-                    fx_pair(z, x, CC);
-                    pl[0] = make_longlong2(z.r, z.i);
-                    pc[0] = make_longlong2(x.r, x.i);
+                    if (G == 1 || (q & (G - 1)) == gl) {  // the rows of a chunk are shared out
+                        fx_pair(z, x, CC);
+                        pl[0] = make_longlong2(z.r, z.i);
+                        pc[0] = make_longlong2(x.r, x.i);
+                    }
                     x = y;
                     pc += rs;
                     pl += rs;
@@ -1006,36 +1048,40 @@ __device__ __forceinline__ void fx_qr_lane(const int n, const FxMat<32> &H, cons
                 fx_pair(x, y, C);
                 fx_pair(hkk, y2, C);
                 fx_pair(hkk, x, CC);
-                pl[0] = make_longlong2(hkk.r, hkk.i);
-                pc[0] = make_longlong2(x.r, x.i);
+                if (G == 1 || (K & (G - 1)) == gl) {
+                    pl[0] = make_longlong2(hkk.r, hkk.i);
+                    pc[0] = make_longlong2(x.r, x.i);
+                }
                 if (act) {
                     const cx<double> ks = conj(R.ds);
                     const cx<double> x1 = cnmac(cscal(sub, R.dc), ks, fx_d(h0));  // H(K+1, K) after the row operation
-                    if (K > L) S.std(K - 1, r);
+                    if (K > L && gl == 0) S.std(K - 1, r);
                     a0 = cmac(cscal(x1, R.dc), ks, fx_d(y));
                     a1 = cmul(ks, nxt);  // the bulge H(K+2, K)
                     sub = cscal(nxt, R.dc);
                     cx64 z1 = fx_i(x1);
                     fx_pair(z1, y, CC);
-                    if (K == I - 1) S.std(I - 1, a0);
+                    if (K == I - 1 && gl == 0) S.std(I - 1, a0);
                 }
                 hkk = y;
-                H.st(K + 1, K + 1, y);
+                if (gl == 0) H.st(K + 1, K + 1, y);
             }
+            if (G > 1) __syncwarp();
             // rows above the chunk
             const int r0 = kVec ? 1 : Kmin;
-            if (Kc > r0) fx_stream_all(H.at(r0, Kc), cs, rs, Kc - r0, ch, ns, true);
-            if (kVec) fx_stream_all(Z.at(1, Kc), cs, rs, n, ch, ns, true);
+            if (Kc > r0) fx_stream_all<G>(gl, H.at(r0, Kc), cs, rs, Kc - r0, ch, ns, true);
+            if (kVec) fx_stream_all<G>(gl, Z.at(1, Kc), cs, rs, n, ch, ns, true);
             const int je = kVec ? n : Kmax + 1;
-            if (je > Ke + 1) fx_stream_all(H.at(Kc, Ke + 2), rs, cs, je - Ke - 1, ch, ns, false);
+            if (je > Ke + 1) fx_stream_all<G>(gl, H.at(Kc, Ke + 2), rs, cs, je - Ke - 1, ch, ns, false);
+            if (G > 1) __syncwarp();
         }
     }
 }
 
 // T-eigenvectors (ztrevc back substitution) on H converted to FP64, x of
 // column k in row k of H's lower triangle; then V = Z X in Z, in FP64.
-template <int G, int ST>
-__device__ __forceinline__ void fx_vectors(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
+template <int G, class GR, int ST>
+__device__ __forceinline__ void fx_vectors(const GR &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
                                            const FxVec<ST> &U)
 {
     const double ulp = lim<double>::eps();
@@ -1220,8 +1266,8 @@ struct FxShifts {
 // The whole solve of one matrix per group, with H, Z (vectors only) and U (n
 // entries) its storage.  Returns false (group-uniform) for a valid matrix
 // that is left to the FP64 kernels; nothing is written then.
-template <int G, bool kVec, int ST, class SH = FxNoShifts>
-__device__ __forceinline__ bool fx_solve(const FxGroup<G> &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
+template <int G, bool kVec, class GR, int ST, class SH = FxNoShifts>
+__device__ __forceinline__ bool fx_solve(const GR &gr, const int n, const FxMat<ST> &H, const FxMat<ST> &Z,
                                          const FxVec<ST> &U, const bool valid, const double *rA, const double *iA,
                                          const long long s, const FxOut &o, const int max_its, const int vnorm,
                                          int &sweeps, int &status, const FxChunk ch = {}, SH *shifts = nullptr)
@@ -1229,7 +1275,8 @@ __device__ __forceinline__ bool fx_solve(const FxGroup<G> &gr, const int n, cons
     double unit;
     bool ok = fx_load<G>(gr, n, H, valid, rA, iA, s, unit);
     fx_reduce<G>(gr, n, H, U);
-    ok = ok && fx_irreducible<G>(gr, n, H);
+    const bool irreducible = fx_irreducible<G>(gr, n, H);  // every lane takes part, whatever ok is
+    ok = ok && irreducible;
     typename SH::Picker *sp = nullptr;
     if constexpr (SH::kOn) {
         const FxVec<32> Sub{shifts->scratch + 5 * n * 32};
@@ -1240,7 +1287,7 @@ __device__ __forceinline__ bool fx_solve(const FxGroup<G> &gr, const int n, cons
     // subdiagonals in FP64 from here on
     for (int k = gr.gl + 1; k < n; k += G) U.std(k, fx_d(H.ld(k + 1, k)));
     gr.sync();
-    if constexpr (ST == 32) fx_qr_lane<kVec>(n, H, Z, U, ch, ok, max_its, sweeps, status, sp);
+    if constexpr (ST > 1) fx_qr_lane<G, kVec>(gr.gl, n, H, Z, U, ch, ok, max_its, sweeps, status, sp);
     else fx_qr<G, kVec>(gr, n, H, Z, U, ok, max_its, sweeps, status);
     gr.sync();
     if (ok)

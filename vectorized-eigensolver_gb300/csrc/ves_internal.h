@@ -124,7 +124,9 @@ __host__ __device__ inline long long shift_slot_elems(int n)
     return 2 * nn + n + (nn + 1) / 2 + n + (n + 1) / 2 + (n < 6 ? 6 * n : 0);
 }
 cudaError_t launch_fx(const FxArgs &a, bool vec, cudaStream_t st);
-cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, cudaStream_t st);  // one matrix per lane, on a.lane_blocks blocks
+// The lane kernel, G = 1, 2, 4 or 8 lanes per matrix, in the workspace of
+// a.lane_blocks blocks of it with G = 1.
+cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, int G, cudaStream_t st);
 
 cudaError_t launch_fx_shifts(const FxArgs &a, cudaStream_t st);  // the same with predicted shifts
 

@@ -717,17 +717,17 @@ constexpr int kStageThreads = 128;
 inline unsigned stage_blocks(const Geom &g) { return (unsigned)((g.N + kStageThreads - 1) / kStageThreads); }
 
 // Blocks (4 warps) per SM of the persistent FP64 grid when the caller leaves
-// it to the library; VES_FUSED_BLOCKS_PER_SM overrides.  Measured on GB300
-// (eigensolves/s, 2 -> 3 -> 4 -> 5 blocks): n=8 8.88 9.07 9.19 9.30 M/s,
-// n=16 1.588 1.651 1.656 1.637 M/s, n=24 0.520 0.565 0.549 0.546 M/s,
-// n=32 0.230 0.248 0.251 0.232 M/s, n=48 0.063 0.060 0.068 0.068 M/s.
-int fused_default_bps(int n)
+// it to the library; VES_FUSED_BLOCKS_PER_SM overrides.  The fixed-point lane
+// kernel on GB300 (eigensolves/s, 3 -> 4 blocks): n=16 4.05 4.03 M/s, n=24 1.46
+// 1.54 M/s, n=32 0.585 0.656 M/s, n=48 0.149 0.146 M/s; five blocks (96
+// registers a thread) are slower at every order.
+int fused_default_bps()
 {
     if (const char *e = getenv("VES_FUSED_BLOCKS_PER_SM")) {
         const int v = atoi(e);
         if (v >= 1 && v <= 16) return v;
     }
-    return (n >= 21 && n <= 28) ? 3 : 4;
+    return 4;
 }
 
 int device_sms()
@@ -745,7 +745,7 @@ size_t fused_workspace_bytes(int n, long long N, int blocks_per_sm, int *out_blo
     const int sms = device_sms();
     const long long groups = (N + 31) / 32;
     const int wpb = kFusedThreads / 32;
-    const int bps = blocks_per_sm > 0 ? blocks_per_sm : fused_default_bps(n);
+    const int bps = blocks_per_sm > 0 ? blocks_per_sm : fused_default_bps();
     long long blocks = std::min<long long>((groups + wpb - 1) / wpb, (long long)sms * bps);
     if (blocks < 1) blocks = 1;
     const size_t per_slot = (size_t)fused_slot_elems(n, learned) * 32 * sizeof(double2);
@@ -868,7 +868,7 @@ cudaError_t launch_plain_blocks(const FusedArgs &a, long long m0, long long coun
         fused_fp64_kernel<false><<<blocks, kFusedThreads, 0, st>>>(r);
         return cudaGetLastError();
     }
-    if ((e = launch_fx_lanes(f, true, st)) != cudaSuccess) return e;
+    if ((e = launch_fx_lanes(f, true, 1, st)) != cudaSuccess) return e;
     r.list = flist;
     r.list_count = fcount;
     fused_fp64_kernel<false><<<blocks, kFusedThreads, 0, st>>>(r);

@@ -33,7 +33,8 @@ constexpr int kSolveThreads = 128;
 
 struct Item {
     int n;
-    int count;     // matrices in this group (1..32)
+    int count;     // matrices in this group: up to 32, or with kWide lanes per matrix up to 32 / kWide
+    int wide;      // kWide lanes per matrix
     long long at;  // first position in the n-sorted index array
 };
 
@@ -104,11 +105,21 @@ __global__ void histogram_kernel(const int *dims, long long count, int maxd, int
         if (h[b]) atomicAdd(&hist[b], h[b]);
 }
 
-// bin starts, cursors, and the work-item list (one thread; 64 bins)
+// bin starts, cursors, and the work-item list (one thread; 64 bins).
+// A warp takes 1.05 ms (n/8)^2.66 for up to 32 matrices of order n, one per
+// lane, alone on the chip and 2.5 times that on a full one.  Where one item
+// would outlast the batch's whole work spread over all warps, the order gets
+// kWide lanes per matrix: 8 lanes take 0.23 (n=64) to 0.41 (n=16) of the time, for
+// 1.9 to 3.3 times the work.  20,000 matrices of orders 4 .. 64: 348 ms with
+// one lane each, bound by the items of n=64.
+constexpr int kWide = 8;
 __global__ void plan_kernel(const int *hist, long long *bin_start, long long *cursor, Item *items, int *nitems,
-                            int order)
+                            int order, long long nslots)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    float work = 0.f;
+    for (int b = kFxMinDim; b <= kMaxVarDim; ++b) work += hist[b] / 32.f * __powf(b, 2.66f);
+    const float longest = 2.5f * work / (float)nslots;
     long long s = 0;
     for (int b = 0; b <= kMaxVarDim; ++b) {
         bin_start[b] = s;
@@ -118,10 +129,13 @@ __global__ void plan_kernel(const int *hist, long long *bin_start, long long *cu
     int it = 0;
     for (int k = 0; k < kMaxVarDim; ++k) {
         const int b = order == 0 ? kMaxVarDim - k : k + 1;  // 0: largest n first
-        for (long long at = bin_start[b]; at < bin_start[b] + hist[b]; at += 32) {
+        const int wide = fx_order(b) && __powf(b, 2.66f) > longest;
+        const int per = wide ? 32 / kWide : 32;
+        for (long long at = bin_start[b]; at < bin_start[b] + hist[b]; at += per) {
             Item x;
             x.n = b;
-            x.count = (int)min(32LL, bin_start[b] + hist[b] - at);
+            x.wide = wide;
+            x.count = (int)min((long long)per, bin_start[b] + hist[b] - at);
             x.at = at;
             items[it++] = x;
         }
@@ -159,11 +173,10 @@ struct VarArgs {
     int vnorm;
 };
 
-__global__ void __launch_bounds__(kSolveThreads) varsize_solve_kernel(const VarArgs a)
+__global__ void __launch_bounds__(kSolveThreads, 4) varsize_solve_kernel(const VarArgs a)
 {
     __shared__ longlong2 chs[kSolveThreads * kFxChunk];
     __shared__ i64 chi[kSolveThreads * kFxChunk];
-    const FxGroup<1> gr;
     const int lane = threadIdx.x & 31;
     const int ch0 = (threadIdx.x >> 5) * 32 * kFxChunk + lane;
     const FxChunk ch{chs + ch0, chi + ch0};
@@ -178,29 +191,38 @@ __global__ void __launch_bounds__(kSolveThreads) varsize_solve_kernel(const VarA
         if (it >= total) break;
         const Item item = a.items[it];
         const int n = item.n;
-        const MatIlv<double> H{base, n};
-        const MatIlv<double> Z{base + (long long)n * n * 32, n};
-        const VecIlv<double> W{base + 2LL * n * n * 32};
-        bool valid = lane < item.count;
-        const long long m = valid ? a.sorted[item.at + lane] : 0;
-        const long long ao = valid ? a.aoff[m] : 0, eo = valid ? a.eoff[m] : 0;
         int status = 0, sweeps = 0;
+        // lanes of an item: matrix lane % per, the lanes of one matrix per apart
+        const int per = item.wide ? 32 / kWide : 32, mat = lane & (per - 1);
+        bool valid = mat < item.count;
+        const long long m = valid ? a.sorted[item.at + mat] : 0;
+        const long long ao = valid ? a.aoff[m] : 0, eo = valid ? a.eoff[m] : 0;
         if (fx_order(n)) {
-            longlong2 *const fb = reinterpret_cast<longlong2 *>(base);
-            const FxMat<32> FH{fb, n, n}, FZ{fb + (long long)n * n * 32, n, n};
-            const FxVec<32> FU{fb + 2LL * n * n * 32};
             const FxOut o{a.rE + eo, a.iE + eo, a.rV + ao, a.iV + ao, nullptr, nullptr, 1, 1};
-            const bool ok = fx_solve<1, true>(gr, n, FH, FZ, FU, valid, a.rA + ao, a.iA + ao, 1, o, a.max_its, a.vnorm,
-                                              sweeps, status, ch);
-            if (ok) {
+            longlong2 *const w = reinterpret_cast<longlong2 *>(base) - lane + mat;
+            bool ok;
+            if (item.wide) {
+                constexpr int M = 32 / kWide;
+                ok = fx_solve<kWide, true>(FxLanes<kWide>(), n, FxMat<M>{w, n, n}, FxMat<M>{w + n * n * M, n, n},
+                                           FxVec<M>{w + 2 * n * n * M}, valid, a.rA + ao, a.iA + ao, 1, o, a.max_its,
+                                           a.vnorm, sweeps, status, ch);
+            } else {
+                ok = fx_solve<1, true>(FxLanes<1>(), n, FxMat<32>{w, n, n}, FxMat<32>{w + n * n * 32, n, n},
+                                       FxVec<32>{w + 2 * n * n * 32}, valid, a.rA + ao, a.iA + ao, 1, o, a.max_its,
+                                       a.vnorm, sweeps, status, ch);
+            }
+            if (ok && lane < per) {
                 if (a.status) a.status[m] = status;
                 if (a.sweeps) a.sweeps[m] = sweeps;
             }
             // what the fixed-point form leaves is solved in FP64 by the same warp
-            valid = valid && !ok;
+            valid = valid && !ok && lane < per;
             if (!__any_sync(FULL, valid)) continue;
             status = sweeps = 0;
         }
+        const MatIlv<double> H{base, n};
+        const MatIlv<double> Z{base + (long long)n * n * 32, n};
+        const VecIlv<double> W{base + 2LL * n * n * 32};
         if (valid) {
             const MatSoA<double> A{const_cast<double *>(a.rA) + ao, const_cast<double *>(a.iA) + ao, 1, n};
             bool bad = false;
@@ -255,7 +277,7 @@ VarPlan var_plan(long long count, int max_dim, int blocks_per_sm)
     if (sms <= 0) sms = 1;
     VarPlan p{};
     p.nblocks = (count + kScanBlock - 1) / kScanBlock;
-    const long long max_items = count / 32 + kMaxVarDim + 1;
+    const long long max_items = count / (32 / kWide) + kMaxVarDim + 1;
     const long long solve_blocks = std::max<long long>(1, std::min<long long>((max_items + 3) / 4,
                                                                                (long long)sms * blocks_per_sm));
     p.nslots = solve_blocks * (kSolveThreads / 32);
@@ -309,7 +331,7 @@ cudaError_t launch_varsize(long long count, int max_dim, const int *dims, const 
     scan_apply_kernel<<<(unsigned)p.nblocks, kScanBlock, 0, st>>>(aoff, eoff, bsa, bse, count);
     const unsigned hb = (unsigned)std::min<long long>((count + 255) / 256, 4096);
     histogram_kernel<<<hb, 256, 0, st>>>(dims, count, max_dim, hist);
-    plan_kernel<<<1, 32, 0, st>>>(hist, bstart, cursor, items, nitems, order);
+    plan_kernel<<<1, 32, 0, st>>>(hist, bstart, cursor, items, nitems, order, p.nslots);
     scatter_kernel<<<hb, 256, 0, st>>>(dims, count, max_dim, cursor, sorted, status);
     VarArgs a{};
     a.rA = rA; a.iA = iA; a.rE = rE; a.iE = iE; a.rV = rV; a.iV = iV;
