@@ -779,6 +779,7 @@ int ves_eigensolve(int dim, int block_cnt, int thread_cnt, const double *rA, con
     m.tol = o.refine_tol;
     m.fb_list = list;
     m.fb_count = count;
+    m.plain_count = ves::fx_order(dim) ? fcount : nullptr;  // (other orders have no such list)
     m.blocks_per_sm = o.blocks_per_sm;
     m.work = o.work_counts;
     // refinement steps with a float-float residual: 2 (default) or 1; VES_MIXED_FF_STEPS overrides (tuning)
@@ -811,7 +812,7 @@ int ves_eigensolve(int dim, int block_cnt, int thread_cnt, const double *rA, con
     a.list = list;
     a.list_count = count;
     a.status_or = VES_STATUS_REFINE_FALLBACK;
-    return native(cuda_ok(ves::launch_plain(a, flist, fcount, st), "fallback kernel launch"));
+    return native(cuda_ok(ves::launch_plain(a, flist, fcount, st, true), "fallback kernel launch"));
 }
 
 size_t ves_polyroots_workspace_size(int degree, int block_cnt, int thread_cnt)

@@ -73,6 +73,7 @@ struct MixedArgs {
     double tol;     // ||r|| <= tol ||A||_F ||v||
     int *fb_list;   // matrices handed to the FP64 solver
     int *fb_count;
+    int *plain_count;  // the FP64 solver's own list counter (nullable), set to zero by the last kernel here
     int blocks_per_sm;  // FP32 Schur kernel grid: blocks per SM; 0 = default
     // matrices [m_begin, m_end) of the batch (a multiple of 32 where a chunk
     // ends inside the batch); launch_mixed sets the whole batch when m_end == 0
@@ -158,8 +159,8 @@ cudaError_t launch_backsubs(Geom g, const double *rT, const double *iT, double *
 // The plain FP64 solve: fx_order(n) in fixed point, then the matrices that it
 // leaves to the FP64 kernels; other n in the FP64 kernels.  `a` as for
 // launch_fused_fp64 (a.list: those matrices only); flist holds a.g.N ints
-// (unused for other n), fcount one int.
-cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st);
+// (unused for other n), fcount one int, which is set to zero here unless `zeroed`.
+cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st, bool zeroed = false);
 // The shift-seeded solve (a.rS) the same way, one matrix per lane.
 cudaError_t launch_shifts(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st);
 // launch_plain for matrices [m0, m0 + count) (n <= 64) with the lane kernels on a

@@ -819,11 +819,11 @@ static FxArgs fx_args(const FusedArgs &a, int *flist, int *fcount)
     return f;
 }
 
-cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st)
+cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st, bool zeroed)
 {
     if (a.g.N <= 0) return cudaSuccess;
     if (!fx_order(a.g.n)) return a.list ? launch_fp64_list(a, st) : launch_fused_fp64(a, st);
-    cudaError_t e = cudaMemsetAsync(fcount, 0, sizeof(int), st);
+    cudaError_t e = zeroed ? cudaSuccess : cudaMemsetAsync(fcount, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     FxArgs f = fx_args(a, flist, fcount);
     fused_workspace_bytes(a.g.n, a.g.N, a.blocks_per_sm, &f.lane_blocks, nullptr);

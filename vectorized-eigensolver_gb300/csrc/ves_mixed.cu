@@ -8,7 +8,7 @@
 // FP64 work shrinks to the residuals r = A v - lambda v (4 n^2 FMAs per pair
 // and step).
 //
-// Two kernels:
+// Its kernels:
 //  schur32  one matrix per lane (the lockstep routines of ves_device.cuh in
 //           float): T, Z and the T-eigenvectors X of each matrix are left in an
 //           HBM buffer laid out [group of 32][element][lane].  Matrices whose
@@ -16,7 +16,8 @@
 //           sweep cap, are put on the FP64 list here.
 //  refine   one EIGENPAIR per lane: the lanes of one matrix read the same A, T,
 //           Z, X elements (one broadcast transaction each) and every FP64
-//           instruction works on 32 pairs.
+//           instruction works on 32 pairs; or, after a Schur kernel that leaves
+//           its results per matrix, one matrix per block (refine_mat_kernel).
 //
 // Refinement of pair k (Newton on (A - lambda I) v = 0 with the component of v
 // along the k-th Schur vector held fixed; Dongarra, Moler & Wilkinson,
@@ -38,9 +39,11 @@
 // is not accepted after `max_steps` corrections sends its matrix to the FP64
 // solver (the caller's second launch over the list).
 #include "ves_device.cuh"
+#include "ves_fx.cuh"
 #include "ves_internal.h"
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 
@@ -104,12 +107,16 @@ __device__ __forceinline__ void ff_mac(float &s, float &e, const float a, const 
 
 // One entry of an eigenvector iterate: float-float (head h, tail t with
 // |t| <= ulp(h) / 2) while the residuals are float-float, FP64 (d) from the
-// first FP64 residual on.  The two forms share the 16 bytes, so the per-lane
-// vector costs what an FP64 one does.
+// first FP64 residual on, or 64-bit fixed point (x, refine_mat_kernel).  The
+// forms share the 16 bytes, so a vector costs what an FP64 one does.
 union VEntry {
     cx<double> d;
+    int4 x;
     struct { cx<float> h, t; } f;
 };
+
+__device__ __forceinline__ double pow2d(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }
 
 // (h, t) += s in float-float: TwoSum of the heads, the tail and the rounding
 // error summed, then renormalised (Fast2Sum, valid as |sum| >= |tail|).
@@ -1030,6 +1037,484 @@ __global__ void __launch_bounds__(kRefineThreads, 16) refine16_lane_kernel(const
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) refine_tile<16, false>(a, buf, flags, tile);
 }
 
+// ---------------------------------------------------------------------------
+// refine_mat_kernel<TR>: the refinement for the per-matrix layout, one matrix
+// per block, all of its pairs together: V (n x n) and the residuals are matrices
+// in shared memory, so that R = A V - V Lambda, Z^H R and Z dX are matrix
+// products.  A warp's lanes form a 4 x 8 grid over a tile of 4 TR rows and 8
+// columns, TR rows a lane; the tiles are dealt over the block's warps.  The
+// triangular solve and the tests of pair k are thread k's.
+//
+// Why: with a pair per lane (refine_kernel, refine_by_matrix below says where it is
+// still used) a lane's vectors lie in local memory, 25% of whose loads hit L1 at
+// n=16, and the accepting residual in FP64 fills 58% of the time of the FP64 pipe.
+// That kernel with the residual on the integer pipe, or with four rows per load of
+// a vector, gained nothing: it waits for local memory.  Here, 524,288 matrices
+// n=16, 30.2 -> 27.2 ms: 36,000 instructions a matrix, a third of them the two
+// float-float residuals, issued in 56% of the cycles of 14 warps per SM (with the
+// loops unrolled 2 to 4 times 44%: the phases of the warps then miss the
+// instruction cache).  65,536 matrices n=32: 28.3 -> 20.4 ms.
+//
+// Accepting residual: 64-bit fixed point.  A and lambda are held in units of
+// 2^(eA - 60), 2^eA >= ||A||_F, and v in units of 2^(f - 60), 2^f >= ||v||, each
+// as a signed high and a balanced signed low word.  Of a product the low-by-low
+// part (below 2^-58 of the scales, of random sign) is dropped, sums are exact;
+// FP64 rounds every partial sum, of size |lambda| |v_i|, to 2^-53 of it.  A
+// complex multiply-add takes twelve IMAD.WIDE (12 / 26 clocks per lane and SM)
+// where FP64 takes 4 / 1.8.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ i64 fx_join(int h, int l) { return ((i64)h << 32) + l; }
+__device__ __forceinline__ void fx_words(i64 x, int &h, int &l)
+{
+    l = (int)x;
+    h = (int)((x - l) >> 32);
+    if (l == INT_MIN) l = INT_MIN + 1;  // its negative is used too
+}
+// real and imaginary part of z s, s a power of two: {high, low, high, low}
+__device__ __forceinline__ int4 fx_entry(const cx<double> z, const double s)
+{
+    int4 w;
+    fx_words(__double2ll_rn(z.r * s), w.x, w.y);
+    fx_words(__double2ll_rn(z.i * s), w.z, w.w);
+    return w;
+}
+__device__ __forceinline__ int4 fx_add(const int4 x, const i64 r, const i64 i)
+{
+    int4 w;
+    fx_words(fx_join(x.x, x.y) + r, w.x, w.y);
+    fx_words(fx_join(x.z, x.w) + i, w.z, w.w);
+    return w;
+}
+
+// Complex sum of products: high halves (weight 2^64) and cross halves (weight
+// 2^32).  A row of A and a column of V have 2-norms of at most 2^28 in their high
+// words, so 16 columns add at most 2 sqrt(32) 2^28 2^31 < 2^63 to the cross halves:
+// carry() at least every 16 columns.
+struct FxSum {
+    i64 hr, xr, hi, xi;
+    __device__ __forceinline__ void mac(const int4 a, const int4 v)
+    {
+        const int nh = -v.z, nl = -v.w;
+        hr = wide(a.x, v.x, wide(a.z, nh, hr));
+        xr = wide(a.x, v.y, wide(a.y, v.x, wide(a.z, nl, wide(a.w, nh, xr))));
+        hi = wide(a.x, v.z, wide(a.z, v.x, hi));
+        xi = wide(a.x, v.w, wide(a.y, v.z, wide(a.z, v.y, wide(a.w, v.x, xi))));
+    }
+    __device__ __forceinline__ void carry()
+    {
+        hr += xr >> 32; xr &= 0xffffffffLL;
+        hi += xi >> 32; xi &= 0xffffffffLL;
+    }
+    // a sum (carried) in units of 2^(eA + f), to FP32: to 2^-76 where it is below 2^-14
+    static __device__ __forceinline__ float value(i64 h, i64 x)
+    {
+        const bool small = h < (1LL << 42) && h > -(1LL << 42);
+        return __ll2float_rn(small ? (h << 20) + (x >> 12) : h) * (small ? 0x1p-76f : 0x1p-56f);
+    }
+};
+
+// shared memory of refine_mat_kernel: 32 bytes per pair; V; rows of A, which share
+// their place with dX; R, T and Z
+__host__ __device__ __forceinline__ int refine_ld(int n) { return n | 1; }
+__host__ __device__ __forceinline__ int refine_a_units(int n, int TR)
+{
+    const int rows = 4 * TR * n, dx = (refine_ld(n) * n + 1) / 2;
+    return rows > dx ? rows : dx;
+}
+__host__ __device__ __forceinline__ size_t refine_smem(int n, int TR)
+{
+    const int e = refine_ld(n) * n;
+    return 16 * (size_t)(2 * n + e + refine_a_units(n, TR)) + 8 * (size_t)(3 * e);
+}
+
+// s[t] = sum_j L(r_t, j) R(j, c), or with kAdj sum_j conj(L(j, r_t)) R(j, c), for rows
+// r_t = r0 + 4 t (the last row again beyond it); R at its column c
+template <int TR, bool kAdj>
+__device__ __forceinline__ void mat_rows(const int n, const int ld, const float2 *L, const float2 *Rc, const int r0,
+                                         cx<float> (&s)[TR])
+{
+    const float2 *p[TR];
+#pragma unroll
+    for (int t = 0; t < TR; ++t) {
+        const int r = min(r0 + 4 * t, n - 1);
+        p[t] = L + (kAdj ? r * ld : r);
+        s[t] = mk(0.f, 0.f);
+    }
+#pragma unroll 2
+    for (int j = 0; j < n; ++j) {
+        const float2 b = Rc[j];
+#pragma unroll
+        for (int t = 0; t < TR; ++t) {
+            const float2 l = p[t][kAdj ? j : j * ld];
+            s[t] = kAdj ? cjmac(s[t], mk(l.x, l.y), mk(b.x, b.y)) : cmac(s[t], mk(l.x, l.y), mk(b.x, b.y));
+        }
+    }
+}
+
+// a / b (cdiv) without a branch
+__device__ __forceinline__ cx<float> cdiv_select(const cx<float> a, const cx<float> b)
+{
+    const bool w = fabsf(b.r) <= fabsf(b.i);
+    const float p = w ? b.i : b.r, q = w ? b.r : b.i;
+    const float ratio = __fdividef(q, p), rden = frcp<float>(p * fmaf(ratio, ratio, 1.f));
+    const float re = fmaf(w ? a.r : a.i, ratio, w ? a.i : a.r), im = fmaf(w ? a.i : -a.r, ratio, w ? -a.r : a.i);
+    return mk(re * rden, im * rden);
+}
+
+template <int TR>
+__global__ void __launch_bounds__(256) refine_mat_kernel(const MixedArgs a, const float2 *buf, int *flags)
+{
+    constexpr int RB = 4 * TR;  // rows of a tile
+    extern __shared__ int4 rsm[];
+    const long long m = a.m_begin + blockIdx.x;
+    if (flags[m] != 0) return;
+    const int n = a.g.n, tc = a.g.tc, tid = threadIdx.x, nt = blockDim.x, ld = refine_ld(n), nn = n * n;
+    const int lane = tid & 31, warp = tid >> 5, W = nt >> 5;
+    const int lr = lane & 3, lc = lane >> 2, ncb = (n + 7) >> 3, nrb = (n + RB - 1) / RB;
+    int4 *const sL = rsm;  // -lambda: float-float {head, tail}, or fixed point
+    double *const sO = reinterpret_cast<double *>(sL + n);  // factor from a fixed-point vector to the output
+    int *const sU = reinterpret_cast<int *>(sO + n);  // a pair's vector scale f; whether its correction is added
+    float *const sS = reinterpret_cast<float *>(sU + n);  // 2^-f
+    int4 *const sV = sL + 2 * n, *const sA = sV + ld * n;
+    float2 *const sD = reinterpret_cast<float2 *>(sA);
+    float2 *const sR = reinterpret_cast<float2 *>(sA + refine_a_units(n, TR));
+    float2 *const sT = sR + ld * n, *const sZ = sT + ld * n;
+    VEntry *const V = reinterpret_cast<VEntry *>(sV);
+    const float2 *const bT = buf + m * mat_elems(n), *const bX = bT + 2 * nn, *const bA = bT + 3 * nn + n;
+    const float nA2 = bT[3 * nn].x;
+    const float nb = fmaf(nA2, 1.002f, 1e-37f);  // >= ||A||_F^2, also where squares underflowed
+    const int eA = (ilogbf(nb) + 2) >> 1;
+    const long long mo = soa_off_m(m, nn, tc);
+
+    for (int e = tid; e < nn; e += nt) {
+        const int c = e / n, o = e + c * (ld - n);
+        sT[o] = bT[e];
+        sZ[o] = bT[nn + e];
+        sD[o] = bX[e];
+    }
+    __syncthreads();
+    // V = Z X, X upper triangular with zeros below
+    for (int t = warp; t < nrb * ncb; t += W) {
+        const int r0 = (t % nrb) * RB + lr, c = (t / nrb) * 8 + lc, cc = min(c, n - 1);
+        cx<float> s[TR];
+        mat_rows<TR, false>(n, ld, sZ, sD + cc * ld, r0, s);
+#pragma unroll
+        for (int u = 0; u < TR; ++u)
+            if (r0 + 4 * u < n && c < n) {
+                V[r0 + 4 * u + c * ld].f.h = s[u];
+                V[r0 + 4 * u + c * ld].f.t = mk(0.f, 0.f);
+            }
+    }
+    // thread k < n: pair k
+    bool act = tid < n, fail = false;
+    const int k = act ? tid : 0;
+    cx<double> lam = up(mk(sT[k + k * ld].x, sT[k + k * ld].y));
+    const float xkk = sD[k + k * ld].x;
+    int f = 0;  // v's scale once it is in fixed point
+    const double tol2 = a.tol * a.tol;
+    // eigenvalue acceptance: the Newton correction from a certified residual
+    // estimates the eigenvalue's remaining error; it must be <= 4 tol ||A||_F
+    const float etol2 = (float)(16.0 * tol2);
+    int n_res64 = 0, n_corr = 0, n_ff = 0;  // work counters: accepting / float-float residuals, FP32 corrections
+    const int ff_steps = a.max_steps >= 2 ? a.ff_steps : 1;  // steps whose residual is float-float (see refine_tile)
+    for (int step = 0; step <= a.max_steps; ++step) {
+        if (!__syncthreads_or(act)) break;
+        const bool ff = step < ff_steps;
+        float vn2 = 0.f;  // ||v||^2 in units of 2^2f
+        if (ff) {
+            if (act) {
+                ++n_ff;
+                const cx<float> lh = down(lam), ll = down(csub(lam, up(lh)));
+                sL[k] = make_int4(__float_as_int(-lh.r), __float_as_int(-lh.i), __float_as_int(-ll.r),
+                                  __float_as_int(-ll.i));
+            }
+        } else {
+            if (step == ff_steps) {  // V into fixed point
+                if (act) {
+                    double n2 = 0.0;
+                    for (int i = 0; i < n; ++i) {
+                        const cx<float> h = V[i + k * ld].f.h;
+                        n2 = fma((double)h.i, (double)h.i, fma((double)h.r, (double)h.r, n2));
+                    }
+                    fail = !(n2 > 0x1p-240 && n2 < 0x1p240);  // or not finite
+                    act = !fail;
+                    f = act ? (ilogb(n2) + 3) >> 1 : 0;  // ||v|| <= 2^(f - 1/2)
+                    sU[k] = f;
+                    sS[k] = pow2f(-f);
+                }
+                __syncthreads();
+                for (int e = tid; e < nn; e += nt) {
+                    const int c = e / n, o = e + c * (ld - n);
+                    const cx<float> h = V[o].f.h, t = V[o].f.t;
+                    V[o].x = fx_entry(cadd(up(h), up(t)), pow2d(60 - sU[c]));
+                }
+                __syncthreads();
+            }
+            if (act) {
+                ++n_res64;
+                for (int i = 0; i < n; ++i) {
+                    const float hr = (float)V[i + k * ld].x.x * 0x1p-28f, hi = (float)V[i + k * ld].x.z * 0x1p-28f;
+                    vn2 = fmaf(hi, hi, fmaf(hr, hr, vn2));
+                }
+                // an iterate that left the range of eigenvalues, or of its scale, is the FP64 solver's
+                const double lmax = pow2d(eA + 1);
+                if (!(fabs(lam.r) <= lmax && fabs(lam.i) <= lmax && vn2 <= 1.f)) {
+                    fail = true;
+                    act = false;
+                }
+                sL[k] = act ? fx_entry(mk(-lam.r, -lam.i), pow2d(60 - eA)) : make_int4(0, 0, 0, 0);
+            }
+        }
+        // ---- R = A V - V Lambda, a block of rows of A at a time
+        for (int rb = 0; rb < nrb; ++rb) {
+            const int rows = min(RB, n - rb * RB);
+            for (int e = tid; e < rows * n; e += nt) {
+                const int j = e / rows, i = e - j * rows, g = rb * RB + i + j * n;
+                if (ff) {
+                    const float2 h = bA[g], l = bA[nn + g];
+                    sA[j * RB + i] = make_int4(__float_as_int(h.x), __float_as_int(h.y), __float_as_int(l.x),
+                                               __float_as_int(l.y));
+                } else {
+                    const long long o = mo + (long long)g * tc;
+                    sA[j * RB + i] = fx_entry(mk(a.rA[o], a.iA[o]), pow2d(60 - eA));
+                }
+            }
+            __syncthreads();
+            for (int cb = warp; cb < ncb; cb += W) {
+                const int c = cb * 8 + lc, cc = min(c, n - 1);
+                const VEntry *const v = V + cc * ld;
+                const int4 L = sL[cc];
+                int ri[TR];  // the lane's rows in the block
+#pragma unroll
+                for (int t = 0; t < TR; ++t) ri[t] = min(lr + 4 * t, rows - 1);
+                float or_[TR], oi[TR];
+                if (ff) {
+                    const float lhr = __int_as_float(L.x), lhi = __int_as_float(L.y);
+                    const float llr = __int_as_float(L.z), lli = __int_as_float(L.w);
+                    float sr[TR], er[TR], si[TR], ei[TR];
+#pragma unroll
+                    for (int t = 0; t < TR; ++t) {
+                        const cx<float> vi = v[rb * RB + ri[t]].f.h, wi = v[rb * RB + ri[t]].f.t;
+                        sr[t] = er[t] = si[t] = ei[t] = 0.f;
+                        ff_mac(sr[t], er[t], lhr, vi.r);
+                        ff_mac(sr[t], er[t], -lhi, vi.i);
+                        ff_mac(si[t], ei[t], lhr, vi.i);
+                        ff_mac(si[t], ei[t], lhi, vi.r);
+                        er[t] = fmaf(-lhi, wi.i, fmaf(lhr, wi.r, fmaf(-lli, vi.i, fmaf(llr, vi.r, er[t]))));
+                        ei[t] = fmaf(lhi, wi.r, fmaf(lhr, wi.i, fmaf(lli, vi.r, fmaf(llr, vi.i, ei[t]))));
+                    }
+#pragma unroll 1
+                    for (int j = 0; j < n; ++j) {
+                        const cx<float> vj = v[j].f.h, wj = v[j].f.t;
+#pragma unroll
+                        for (int t = 0; t < TR; ++t) {
+                            const int4 q = sA[j * RB + ri[t]];
+                            const float ahr = __int_as_float(q.x), ahi = __int_as_float(q.y);
+                            const float alr = __int_as_float(q.z), ali = __int_as_float(q.w);
+                            ff_mac(sr[t], er[t], ahr, vj.r);
+                            ff_mac(sr[t], er[t], -ahi, vj.i);
+                            ff_mac(si[t], ei[t], ahr, vj.i);
+                            ff_mac(si[t], ei[t], ahi, vj.r);
+                            er[t] = fmaf(-ali, vj.i, fmaf(alr, vj.r, er[t]));
+                            ei[t] = fmaf(ali, vj.r, fmaf(alr, vj.i, ei[t]));
+                            er[t] = fmaf(-ahi, wj.i, fmaf(ahr, wj.r, er[t]));
+                            ei[t] = fmaf(ahi, wj.r, fmaf(ahr, wj.i, ei[t]));
+                        }
+                    }
+#pragma unroll
+                    for (int t = 0; t < TR; ++t) {
+                        or_[t] = __fadd_rn(sr[t], er[t]);
+                        oi[t] = __fadd_rn(si[t], ei[t]);
+                    }
+                } else {
+                    FxSum s[TR];
+#pragma unroll
+                    for (int t = 0; t < TR; ++t) {
+                        s[t] = FxSum{0, 0, 0, 0};
+                        s[t].mac(L, v[rb * RB + ri[t]].x);
+                        s[t].carry();
+                    }
+                    for (int j0 = 0; j0 < n; j0 += 16) {
+                        const int j1 = min(j0 + 16, n);
+#pragma unroll 1
+                        for (int j = j0; j < j1; ++j) {
+                            const int4 vj = v[j].x;
+#pragma unroll
+                            for (int t = 0; t < TR; ++t) s[t].mac(sA[j * RB + ri[t]], vj);
+                        }
+#pragma unroll
+                        for (int t = 0; t < TR; ++t) s[t].carry();
+                    }
+#pragma unroll
+                    for (int t = 0; t < TR; ++t) {
+                        or_[t] = FxSum::value(s[t].hr, s[t].xr);
+                        oi[t] = FxSum::value(s[t].hi, s[t].xi);
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < TR; ++t)
+                    if (lr + 4 * t < rows && c < n) sR[rb * RB + lr + 4 * t + c * ld] = make_float2(or_[t], oi[t]);
+            }
+            __syncthreads();
+        }
+        bool certified = false;
+        if (act) {
+            if (!ff) {
+                float rn2 = 0.f;  // in units of 2^(2 eA + 2 f - 80)
+                for (int i = 0; i < n; ++i) {
+                    const float2 r = sR[i + k * ld];
+                    const float br = r.x * 0x1p40f, bi = r.y * 0x1p40f;
+                    rn2 = fmaf(bi, bi, fmaf(br, br, rn2));
+                }
+                // (FP32 sums of squares, good to 2^-17: the margin keeps them from accepting more than FP64 would)
+                certified = (double)rn2 * 1.0001 <= tol2 * (double)nA2 * pow2d(80 - 2 * eA) * (double)vn2;
+            }
+            if (!certified && step == a.max_steps) { fail = true; act = false; }
+        }
+        // ---- FP32 correction through the Schur form: r' = Z^H r
+        for (int t = warp; t < nrb * ncb; t += W) {
+            const int r0 = (t % nrb) * RB + lr, c = (t / nrb) * 8 + lc, cc = min(c, n - 1);
+            cx<float> s[TR];
+            mat_rows<TR, true>(n, ld, sZ, sR + cc * ld, r0, s);
+#pragma unroll
+            for (int u = 0; u < TR; ++u)
+                if (r0 + 4 * u < n && c < n) sD[r0 + 4 * u + c * ld] = make_float2(s[u].r, s[u].i);
+        }
+        __syncthreads();
+        bool upd = act;
+        cx<float> dl = mk(0.f, 0.f);
+        if (act) {
+            ++n_corr;
+            float2 *const x = sD + k * ld;
+            const float sa = ff ? 1.f : pow2f(eA), sv = ff ? 1.f : pow2f(f);
+            const cx<float> l32 = down(lam);
+            const float smin = fmax(lim<float>::eps() * cabs1(l32), lim<float>::tiny() * (float(n) / lim<float>::eps()));
+#pragma unroll 1
+            for (int i0 = n - 1; i0 >= 0; i0 -= 4) {  // rows i0, i0 - 1, ..: the columns right of them first
+                cx<float> s[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const float2 d = x[max(i0 - t, 0)];
+                    s[t] = mk(-d.x * sa * sv, -d.y * sa * sv);
+                }
+#pragma unroll 1
+                for (int j = i0 + 1; j < n; ++j) {
+                    const float2 d = x[j];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const float2 q = sT[max(i0 - t, 0) + j * ld];
+                        s[t] = cnmac(s[t], mk(q.x, q.y), mk(d.x, d.y));
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (i0 >= t) x[i0 - t] = make_float2(s[t].r, s[t].i);
+#pragma unroll 1
+                for (int i = i0; i >= max(i0 - 3, 0); --i) {
+                    cx<float> y = mk(x[i].x, x[i].y);
+#pragma unroll 1
+                    for (int j = i0; j > i; --j) {
+                        const float2 q = sT[i + j * ld], d = x[j];
+                        y = cnmac(y, mk(q.x, q.y), mk(d.x, d.y));
+                    }
+                    if (i == k) dl = cscal(mk(-y.r, -y.i), 1.f / xkk);  // dlambda x_k = r'_k + sum_{j>k} T_kj dx_j = -s
+                    if (i < k) {
+                        const float2 q = bX[i + k * n];
+                        y = cmac(y, dl, mk(q.x, q.y));
+                    }
+                    const float2 q = sT[i + i * ld];
+                    cx<float> d = csub(mk(q.x, q.y), l32);
+                    if (cabs1(d) < smin) d = mk(smin, 0.f);
+                    y = i == k ? mk(0.f, 0.f) : cdiv_select(y, d);
+                    x[i] = make_float2(y.r, y.i);
+                }
+            }
+            if (certified) {
+                // a small residual bounds the eigenvalue error only through its
+                // condition number: accept when the next correction to lambda is
+                // below 4 tol ||A||_F, else take the step and verify again
+                if (dl.r * dl.r + dl.i * dl.i <= etol2 * nA2) act = upd = false;
+                else if (step == a.max_steps) { fail = true; act = upd = false; }
+            }
+            if (upd) lam = cadd(lam, up(dl));
+        }
+        if (tid < n) sU[k] = upd;
+        __syncthreads();
+        // ---- v += Z dx
+        for (int t = warp; t < nrb * ncb; t += W) {
+            const int r0 = (t % nrb) * RB + lr, c = (t / nrb) * 8 + lc, cc = min(c, n - 1);
+            if (!__any_sync(FULL, sU[cc])) continue;
+            cx<float> s[TR];
+            mat_rows<TR, false>(n, ld, sZ, sD + cc * ld, r0, s);
+            if (c < n && sU[c]) {
+                const float u = sS[c];
+#pragma unroll
+                for (int q = 0; q < TR; ++q)
+                    if (r0 + 4 * q < n) {
+                        VEntry &v = V[r0 + 4 * q + c * ld];
+                        if (ff) {
+                            ff_add(v.f.h.r, v.f.t.r, s[q].r);
+                            ff_add(v.f.h.i, v.f.t.i, s[q].i);
+                        } else {
+                            // (a correction as large as v: ||v|| leaves its scale and the pair fails)
+                            const float br = fminf(fmaxf(s[q].r * u, -1.f), 1.f), bi = fminf(fmaxf(s[q].i * u, -1.f), 1.f);
+                            v.x = fx_add(v.x, __float2ll_rn(br * 0x1p60f), __float2ll_rn(bi * 0x1p60f));
+                        }
+                    }
+            }
+        }
+    }
+    if (a.work) {
+        const int r64 = __reduce_add_sync(FULL, n_res64), c32 = __reduce_add_sync(FULL, n_corr);
+        const int rff = __reduce_add_sync(FULL, n_ff);
+        if (lane == 0) {
+            if (r64) atomicAdd(a.work + WORK_RES64, (unsigned long long)r64);
+            if (c32) atomicAdd(a.work + WORK_CORR32, (unsigned long long)c32);
+            if (rff) atomicAdd(a.work + WORK_RESFF, (unsigned long long)rff);
+        }
+    }
+    if (__syncthreads_or(fail)) {
+        if (tid == 0) to_fp64_list(a, flags, m);
+        return;
+    }
+    if (tid < n) {
+        // (norms on the integer pipe as well: FP64 sums over n threads took 2.5 of 66 ms at n=16)
+        double o = pow2d(f - 60);
+        if (a.vnorm == 1) {
+            i64 mx = 0;
+            for (int i = 0; i < n; ++i) {
+                const int4 x = V[i + k * ld].x;
+                mx = max(mx, llabs(fx_join(x.x, x.y)) + llabs(fx_join(x.z, x.w)));
+            }
+            if (mx > 0) o = 1.0 / (double)mx;
+        } else if (a.vnorm == 2) {
+            i64 h = 0, c = 0;  // squares of the high words (weight 2^64), high by low words (2^33)
+            for (int i0 = 0; i0 < n; i0 += 16) {
+                for (int i = i0; i < min(i0 + 16, n); ++i) {
+                    const int4 x = V[i + k * ld].x;
+                    h = wide(x.x, x.x, wide(x.z, x.z, h));
+                    c = wide(x.x, x.y, wide(x.z, x.w, c));
+                }
+                h += c >> 31; c &= 0x7fffffffLL;
+            }
+            const i64 s2 = (h << 6) + (c >> 25);  // units of 2^58
+            if (s2 > 0) o = 0x1p-29 / sqrt((double)s2);
+        }
+        sO[k] = o;
+        const long long vo = soa_off_m(m, n, tc);
+        const VecSoA<double> E{a.rE + vo, a.iE + vo, tc};
+        E.st(k + 1, lam);
+    }
+    __syncthreads();
+    for (int e = tid; e < nn; e += nt) {
+        const int c = e / n;
+        const int4 x = V[e + c * (ld - n)].x;
+        const long long o = mo + (long long)e * tc;
+        a.rV[o] = (double)fx_join(x.x, x.y) * sO[c];
+        a.iV[o] = (double)fx_join(x.z, x.w) * sO[c];
+    }
+}
+
 // Distinctness of the refined eigenvalues of each matrix.  Newton from two
 // FP32 starting points can land on the same eigenpair when the FP32 Schur
 // form does not resolve a cluster: both pairs pass their residual and
@@ -1045,6 +1530,7 @@ __global__ void __launch_bounds__(128) dupcheck_kernel(const MixedArgs a, const 
 {
     const int n = a.g.n, tc = a.g.tc;
     const long long m = a.m_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.plain_count) *a.plain_count = 0;
     if (m >= a.m_end || flags[m] != 0 || n < 2) return;
     const long long nn = (long long)n * n;
     const float2 *pT = buf + (kPerMatrix ? m * mat_elems(n) : (m / 32) * group_elems(n) * 32 + (m % 32));
@@ -1236,7 +1722,31 @@ cudaError_t launch_schur(const MixedArgs &a, int blocks_per_sm, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// FP64 refinement of the eigenpairs of matrices [a.m_begin, a.m_end)
+// Which refinement follows a per-matrix Schur kernel: refine_mat_kernel, a matrix
+// per block, or refine_kernel, a pair per lane.  Whole FP32+refine solves, pair ->
+// matrix, ms: n=16 x 524,288 65.6 -> 63.6, n=24 x 131,072 55.3 -> 54.0, n=32 x
+// 65,536 61.0 -> 53.2, n=48 x 16,384 84.0 -> 71.6, n=64 x 8,192 109 -> 89.9; small
+// batches leave the lanes of the pair kernel waiting: n=12 x 4,000 0.48 -> 0.43, n=16 x
+// 64 0.46 -> 0.36, n=21 x 1,000 0.88 -> 0.61, n=57 x 300 7.3 -> 4.2.  Where the tiles
+// fit the order badly the pair kernel is ahead in large batches: n=12 x 300,000 19.2
+// against 20.3, n=17 x 100,000 19.1 against 22.7, n=20 x 131,072 35.4 against 37.7; at
+// n=9 x 16,384 0.78 against 0.82.
+bool refine_by_matrix(int n, long long N) { return n >= 24 || n == 15 || n == 16 || N <= 4096; }
+
+// One block per matrix, of 1 to 8 warps: shared memory (15 KB at n=16, 50 KB at
+// n=32, 200 KB at n=64) then holds about 16 warps per SM.
+template <int TR> cudaError_t launch_refine_mat(const MixedArgs &a, const MixedBufs &b, cudaStream_t st)
+{
+    const int n = a.g.n, W = n <= 16 ? 1 : n <= 28 ? 2 : n <= 40 ? 4 : 8;
+    const size_t smem = refine_smem(n, TR);
+    const cudaError_t e = cudaFuncSetAttribute(refine_mat_kernel<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)refine_smem(64, 4));
+    if (e != cudaSuccess) return e;
+    refine_mat_kernel<TR><<<(unsigned)(a.m_end - a.m_begin), 32 * W, smem, st>>>(a, b.buf, b.flags);
+    return cudaGetLastError();
+}
+
+// refinement of the eigenpairs of matrices [a.m_begin, a.m_end)
 cudaError_t launch_refine(const MixedArgs &a, cudaStream_t st)
 {
     const int n = a.g.n;
@@ -1249,13 +1759,17 @@ cudaError_t launch_refine(const MixedArgs &a, cudaStream_t st)
         if (v >= 1 && v <= 32) tiles = std::min<long long>(tiles, (long long)device_sms() * v);
     }
     const unsigned rb = (unsigned)std::max<long long>(1, tiles);
-    if (schur_group(n, a.g.N)) {  // per-matrix buffer layout
+    const bool per_matrix = schur_group(n, a.g.N) != 0;  // layout of the Schur buffer
+    if (per_matrix && refine_by_matrix(n, a.g.N)) {
+        const int TR = (n + 4 * ((n + 15) / 16) - 1) / (4 * ((n + 15) / 16));  // rows in the fewest tiles
+        return TR <= 2 ? launch_refine_mat<2>(a, b, st) : TR == 3 ? launch_refine_mat<3>(a, b, st)
+                                                                  : launch_refine_mat<4>(a, b, st);
+    }
+    if (per_matrix) {
         if (n <= 16)
             refine_kernel<16, true><<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
-        else if (n <= 32)
-            refine_kernel<32, true><<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
         else
-            refine_kernel<64, true><<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
+            refine_kernel<32, true><<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
     } else if (n <= 16) {
         refine16_lane_kernel<<<rb, kRefineThreads, 0, st>>>(a, b.buf, b.flags);
     } else if (n <= 32) {
@@ -1378,14 +1892,16 @@ void load_mixed_kernels()
     load_kernel(refine_kernel<32, false>);
     load_kernel(refine_kernel<64, false>);
     load_kernel(schur32_warp_kernel<32>);
-    load_kernel(refine_kernel<32, true>);
     load_kernel(schur32_warp_kernel<16>);
     load_kernel(schur32_warp_kernel<32, 2>);
-    load_kernel(refine_kernel<64, true>);
     cudaFuncSetAttribute(schur32_warp_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_schur_smem(16, 16, 128));
     cudaFuncSetAttribute(schur32_warp_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_schur_smem(32, 32, 128));
     cudaFuncSetAttribute(schur32_warp_kernel<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_schur_smem(64, 32, 32));
     load_kernel(refine_kernel<16, true>);
+    load_kernel(refine_kernel<32, true>);
+    load_kernel(refine_mat_kernel<2>);
+    load_kernel(refine_mat_kernel<3>);
+    load_kernel(refine_mat_kernel<4>);
     load_kernel(schur32_group_kernel<8>);
     load_kernel(schur32_group_kernel<4>);
     load_kernel(dupcheck_kernel<false>);
