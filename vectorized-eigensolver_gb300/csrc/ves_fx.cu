@@ -183,7 +183,9 @@ template <bool kVec> cudaError_t launch_fx_v(const FxArgs &a, int G, cudaStream_
 // 360 278 174 135.  Group G = 4, 8, 16, 32: n=16, N=64 2.41 1.70 1.35 1.19,
 // N=2,048 2.57 1.85 1.68 2.47, N=8,192 7.43 5.65 5.69 9.40; G = 16, 32, 64: n=32,
 // N=64 6.05 4.83 4.28, N=8,192 53.8 47.7 65.2; G = 64, 128: n=64, N=512 68.2 64.1.
-// Without vectors half the lane kernel's time and 0.9 of the group's.
+// Without vectors 0.9 of the group's time, and lanes (0.066 + 0.43 x^2.66) ms times
+// the larger of r (a = 3 / n^0.62) and {1, 0.57, 0.2, 0.15} + 1.64 w: n=24, N=10,000
+// G = 1, 2, 4, 8: 9.98 8.00 8.05 11.2; N=30,720 14.0 15.1 23.3 39.3.
 struct FxChoice {
     bool lanes;
     int G;
@@ -198,12 +200,14 @@ FxChoice fx_choose(int n, long long N, bool vec)
     const double sms = fx_sms(), x = n / 8.0;
     FxChoice best{true, 1};
     double t = 1e300;
-    const double lat = (vec ? 0.07 : 0.08) + (vec ? 1.05 : 0.52) * pow(x, 2.66), a = std::min(1.0, (vec ? 1.9 : 3.0) / pow(n, 0.62));
-    const double c[4] = {vec ? 1.5 : 1.0, 1.2, 1.3, 0.8};
+    const double lat = vec ? 0.07 + 1.05 * pow(x, 2.66) : 0.066 + 0.43 * pow(x, 2.66);
+    const double a = std::min(1.0, (vec ? 1.9 : 3.0) / pow(n, 0.62));
+    const double c[4] = {1.5, 1.2, 1.3, 0.8}, r[4] = {1, 0.57, 0.2, 0.15};
     for (int k = 0; k < 4; ++k) {
         const int G = 1 << k;
-        const double w = (double)N * G / 32 / (sms * 16), full = floor(w);
-        const double tl = lat * (a + (1 - a) / G) * (full * (1 + c[k]) + (w > full ? 1 + c[k] * (w - full) : 0));
+        const double w = (double)N * G / 32 / (sms * 16), full = floor(w), alone = a + (1 - a) / G;
+        const double tl = lat * (vec ? alone * (full * (1 + c[k]) + (w > full ? 1 + c[k] * (w - full) : 0))
+                                     : std::max(alone, r[k] + 1.64 * w));
         if (tl < t) {
             t = tl;
             best = {true, G};
