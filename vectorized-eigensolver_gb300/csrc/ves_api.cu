@@ -750,7 +750,7 @@ int ves_eigensolve(int dim, int block_cnt, int thread_cnt, const double *rA, con
             f.out_list = flist; f.out_count = fcount;
             f.ws = ws;
             f.lane_blocks = ves::eigvals_blocks(dim, g.N, o.blocks_per_sm);
-            if (!cuda_ok(cudaMemsetAsync(fcount, 0, sizeof(int), st), "list counter reset") ||
+            if (!cuda_ok(cudaMemsetAsync(fcount, 0, 2 * sizeof(int), st), "list counter reset") ||
                 !cuda_ok(ves::launch_fx(f, false, st), "eigenvalues kernel launch"))
                 return VES_ERR_CUDA;
         } else {

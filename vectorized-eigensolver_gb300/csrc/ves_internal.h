@@ -73,7 +73,7 @@ struct MixedArgs {
     double tol;     // ||r|| <= tol ||A||_F ||v||
     int *fb_list;   // matrices handed to the FP64 solver
     int *fb_count;
-    int *plain_count;  // the FP64 solver's own list counter (nullable), set to zero by the last kernel here
+    int *plain_count;  // the FP64 solver's own two counters (nullable), set to zero by the last kernel here
     int blocks_per_sm;  // FP32 Schur kernel grid: blocks per SM; 0 = default
     // matrices [m_begin, m_end) of the batch (a multiple of 32 where a chunk
     // ends inside the batch); launch_mixed sets the whole batch when m_end == 0
@@ -106,7 +106,7 @@ struct FxArgs {
     int max_its, vnorm;
     const int *list, *list_count;  // nullable: the matrices to solve
     int status_or;                 // bits added to every solved matrix's status
-    int *out_list, *out_count;
+    int *out_list, *out_count;  // out_count: the list's length, then the lane kernel's count of groups taken
     void *ws;         // lane kernel: workspace of lane_blocks x 4 warp slots (fused_workspace_bytes)
     int lane_blocks;
     long long m_begin;  // without a list: the first of the g.N matrices
@@ -132,7 +132,7 @@ cudaError_t launch_fx_lanes(const FxArgs &a, bool vec, int G, cudaStream_t st);
 cudaError_t launch_fx_shifts(const FxArgs &a, cudaStream_t st);  // the same with predicted shifts
 
 // Fused zgehrd -> zunghr -> zlahqr -> ztrevc, FP64.
-// blocks_per_sm = 0 takes the library default (VES_FUSED_BLOCKS_PER_SM, else 4; 3 for 21 <= n <= 28).
+// blocks_per_sm = 0 takes the library default (VES_FUSED_BLOCKS_PER_SM, else 4).
 // learned = the shift-seeded kernel, whose slots also hold an FP32 copy of H
 // and the n predictions.
 size_t fused_workspace_bytes(int n, long long N, int blocks_per_sm, int *out_blocks, int *out_threads,
@@ -159,7 +159,7 @@ cudaError_t launch_backsubs(Geom g, const double *rT, const double *iT, double *
 // The plain FP64 solve: fx_order(n) in fixed point, then the matrices that it
 // leaves to the FP64 kernels; other n in the FP64 kernels.  `a` as for
 // launch_fused_fp64 (a.list: those matrices only); flist holds a.g.N ints
-// (unused for other n), fcount one int, which is set to zero here unless `zeroed`.
+// (unused for other n), fcount two ints, which are set to zero here unless `zeroed`.
 cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st, bool zeroed = false);
 // The shift-seeded solve (a.rS) the same way, one matrix per lane.
 cudaError_t launch_shifts(const FusedArgs &a, int *flist, int *fcount, cudaStream_t st);

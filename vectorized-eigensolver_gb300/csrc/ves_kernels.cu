@@ -1,4 +1,6 @@
-// ves_kernels.cu -- sm_103a kernels of the batched eigensolver.
+// ves_kernels.cu -- FP64 kernels of the batched eigensolver, and the plain solve:
+// orders 3 .. 64 in fixed point (ves_fx.cu) first, then these kernels over the
+// list of the matrices which that form leaves; other orders here alone.
 //
 // fused_fp64_kernel: the whole path of the reference's eigensolver()
 // (utils.cpp:578-698: test_zgehrd -> copy -> test_zunghr -> zlahqr_new ->
@@ -823,7 +825,7 @@ cudaError_t launch_plain(const FusedArgs &a, int *flist, int *fcount, cudaStream
 {
     if (a.g.N <= 0) return cudaSuccess;
     if (!fx_order(a.g.n)) return a.list ? launch_fp64_list(a, st) : launch_fused_fp64(a, st);
-    cudaError_t e = zeroed ? cudaSuccess : cudaMemsetAsync(fcount, 0, sizeof(int), st);
+    cudaError_t e = zeroed ? cudaSuccess : cudaMemsetAsync(fcount, 0, 2 * sizeof(int), st);
     if (e != cudaSuccess) return e;
     FxArgs f = fx_args(a, flist, fcount);
     fused_workspace_bytes(a.g.n, a.g.N, a.blocks_per_sm, &f.lane_blocks, nullptr);
@@ -838,7 +840,7 @@ cudaError_t launch_shifts(const FusedArgs &a, int *flist, int *fcount, cudaStrea
 {
     if (a.g.N <= 0) return cudaSuccess;
     if (!fx_order(a.g.n)) return launch_fused_fp64(a, st);
-    cudaError_t e = cudaMemsetAsync(fcount, 0, sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(fcount, 0, 2 * sizeof(int), st);
     if (e != cudaSuccess) return e;
     FxArgs f = fx_args(a, flist, fcount);
     f.rS = a.rS; f.iS = a.iS;
@@ -857,7 +859,7 @@ cudaError_t launch_shifts(const FusedArgs &a, int *flist, int *fcount, cudaStrea
 cudaError_t launch_plain_blocks(const FusedArgs &a, long long m0, long long count, int blocks, int *flist, int *fcount,
                                 cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(fcount, 0, sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(fcount, 0, 2 * sizeof(int), st);
     if (e != cudaSuccess) return e;
     FxArgs f = fx_args(a, flist, fcount);
     f.g.N = count;

@@ -1530,7 +1530,7 @@ __global__ void __launch_bounds__(128) dupcheck_kernel(const MixedArgs a, const 
 {
     const int n = a.g.n, tc = a.g.tc;
     const long long m = a.m_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.plain_count) *a.plain_count = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.plain_count) a.plain_count[0] = a.plain_count[1] = 0;
     if (m >= a.m_end || flags[m] != 0 || n < 2) return;
     const long long nn = (long long)n * n;
     const float2 *pT = buf + (kPerMatrix ? m * mat_elems(n) : (m / 32) * group_elems(n) * 32 + (m % 32));

@@ -11,11 +11,13 @@
 //   1. offsets      two-level exclusive scans of dims^2 and dims
 //   2. bin          histogram of n, exclusive scan over bins, scatter of
 //                   matrix indices into n-sorted order
-//   3. work items   groups of up to 32 equal-n matrices, largest n first
-//                   (longest-processing-time order) or natural order
+//   3. work items   groups of up to 32 (or 4) equal-n matrices, largest n
+//                   first (longest-processing-time order) or natural order
 //   4. solve        persistent warps take items from an atomic counter; the
-//                   32 lanes of an item run the lockstep FP64 path of the
-//                   fixed-size solver (same routines), one matrix per lane
+//                   32 lanes of an item run the lockstep path of the
+//                   fixed-size solver (same routines: fixed point from order 3
+//                   on, FP64 otherwise and for what the fixed-point form
+//                   leaves), one matrix per lane, or per 8 lanes
 // The lockstep routines need all lanes of a warp at the same n; binning is
 // what lets a mixed batch keep them full.
 #include "ves_fx.cuh"
@@ -111,7 +113,7 @@ __global__ void histogram_kernel(const int *dims, long long count, int maxd, int
 // would outlast the batch's whole work spread over all warps, the order gets
 // kWide lanes per matrix: 8 lanes take 0.23 (n=64) to 0.41 (n=16) of the time, for
 // 1.9 to 3.3 times the work.  20,000 matrices of orders 4 .. 64: 348 ms with
-// one lane each, bound by the items of n=64.
+// one lane each, bound by the items of n=64; 151 ms with this rule.
 constexpr int kWide = 8;
 __global__ void plan_kernel(const int *hist, long long *bin_start, long long *cursor, Item *items, int *nitems,
                             int order, long long nslots)
