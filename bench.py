@@ -20,12 +20,15 @@ e2e     the same metric through the reference-facing drop-in eigensolver()
         with pinned HOST buffers: host->device copy of A, solve, device->host
         copy of eigenvalues, eigenvectors and the Schur form (which the
         reference API writes back into A) inside the timed region.
-roofline  the solver is FP64-pipe bound: achieved = algorithmic FP64 flops
-        per launch (24 n^3 + 20 s n^3 per matrix, s = device-counted QR
-        sweeps per eigenvalue) / launch time, against the FP64 FMA rate
-        measured on this GPU in this run (MEASURED_PEAKS.json carries no FP64
-        figure).  The HBM view (32 n^2 + 16 n bytes per matrix) is reported
-        beside it.
+roofline  the solver applies its unitary transformations in 64-bit fixed point
+        on the integer pipe: achieved = IMAD.WIDE operations per launch (36 for
+        a rotated pair of entries, 12 for a complex multiply-add: 36 n^3 +
+        36 s n^3 per matrix, s = device-counted QR sweeps per eigenvalue) /
+        launch time, against 26 per clock and SM at the maximum SM clock.
+        `fp64` beside it is the same work as 24 n^3 + 20 s n^3 flops against
+        the FP64 FMA rate measured on this GPU in this run: the rate that FP64
+        arithmetic could reach at most, so it may exceed 1.  The HBM view
+        (32 n^2 + 16 n bytes per matrix) is reported too.
 cpu_baseline  the oracle's C restatement of the reference CPU path (OpenMP,
         all host cores) on a bounded prefix of the same batch.
 forms   the other forms, each on its own batch, each verified (residuals on the
@@ -46,7 +49,8 @@ forms   the other forms, each on its own batch, each verified (residuals on the
                      persistent solve against one launch per order.
         Each form entry carries its own roofline from its algorithmic work
         (device-counted where it is data dependent: QR sweeps, Newton
-        corrections and residuals of the refinement, polish steps): FP64
+        corrections and residuals of the refinement, polish steps): the fixed-
+        point transformations and residuals as IMAD.WIDE operations, FP64
         flops against the FP64 FMA rate probed in this run, FP32 flops
         against the FP32 FMA rate probed in this run, BF16 tensor flops
         against MEASURED_PEAKS.json's bf16_tflops, and 32 n^2 + 16 n bytes per
@@ -97,13 +101,24 @@ def r4(x):
     return float("%.4g" % x) if isinstance(x, float) else x
 
 
-def roofline(seconds, fp64=0.0, fp32=0.0, bf16=0.0, hbm=0.0):
-    """Roofline of one step from its ALGORITHMIC work: FP64 / FP32 / BF16 flops
-    and HBM bytes.  Per unit, frac = (work / step time) / measured peak; the
+# IMAD.WIDE (32 x 32 + 64 bit) operations per clock and SM, measured on a GB300
+# with a chain-free loop of them
+IMAD_PER_CLK_SM = 26.0
+
+
+def imad_ops(n, sweeps_total, matrices):
+    """IMAD.WIDE operations of fp64_flops' work in fixed point: 12 per complex
+    multiply-add (8 flops) of the reflectors, 36 per rotated pair (20 flops)."""
+    return 36.0 * n ** 3 * matrices + 36.0 * n * n * sweeps_total
+
+
+def roofline(seconds, fp64=0.0, fp32=0.0, bf16=0.0, hbm=0.0, imad=0.0):
+    """Roofline of one step from its ALGORITHMIC work: FP64 / FP32 / BF16 flops,
+    IMAD.WIDE operations and HBM bytes.  Per unit, frac = (work / step time) / measured peak; the
     bound is the unit whose work takes longest at its peak, and the top-level
     frac is that lower bound on the step time divided by the step time."""
     units = {"fp64": (fp64, "TFLOP/s", 1e12), "fp32": (fp32, "TFLOP/s", 1e12), "bf16": (bf16, "TFLOP/s", 1e12),
-             "hbm": (hbm, "GB/s", 1e9)}
+             "hbm": (hbm, "GB/s", 1e9), "imad": (imad, "T IMAD.WIDE/s", 1e12)}
     fracs = {}
     for u, (work, _, _) in units.items():
         if work > 0 and PEAKS.get(u):
@@ -347,19 +362,19 @@ def measure_form(name, n, N, seed, tc, precision, warmup, steps):
     if precision:
         # FP32: the reference path on the matrices that stayed in FP32, the Newton
         # corrections (Z^H r 8n^2, bordered back substitution 4n^2, Z dx 8n^2) and
-        # the first residuals (8n^2, in float-float on the FP32 pipe); FP64: the
-        # accepting residuals (8n^2 + 16n with the norms) and the fallback solves
+        # the first residuals (8n^2, in float-float on the FP32 pipe); integer pipe:
+        # the accepting residuals (n^2 complex multiply-adds) and the fallback solves
         f32 = fp64_flops(n, float(swd[~fbm].sum()), N - fb) + corr32 * 20.0 * n * n + resff * 8.0 * n * n
-        f64 = fp64_flops(n, float(swd[fbm].sum()), fb) + res64 * (8.0 * n * n + 16.0 * n)
+        imad = imad_ops(n, float(swd[fbm].sum()), fb) + res64 * 12.0 * n * n
     else:
-        f32, f64 = 0.0, fp64_flops(n, float(swd.sum()), N)
-    rl = roofline(ms * 1e-3, fp64=f64, fp32=f32, hbm=hbm_bytes(n, N))
+        f32, imad = 0.0, imad_ops(n, float(swd.sum()), N)
+    rl = roofline(ms * 1e-3, imad=imad, fp32=f32, hbm=hbm_bytes(n, N))
     passed = ver["max_residual"] <= RES_TOL and ver["nonfinite"] == 0 and other == 0
     out = {"form": name, "n": n, "N": N, "value": r4(N / (ms * 1e-3)), "ms": r4(ms), "roofline": rl,
            "s": r4(float(swd.mean()) / n), "max_res": r4(ver["max_residual"]), "passed": passed}
     detail = {"form": name, "n": n, "n_matrices": N, "seed": seed, "steps": steps, "warmup": warmup,
               "median_residual": ver["median_residual"], "nonfinite": ver["nonfinite"], "status_other": other,
-              "flops_fp64": f64, "flops_fp32": f32}
+              "imad_wide": imad, "flops_fp32": f32}
     if precision:
         out["fb"] = fb
         detail.update(fp64_fallback_matrices=fb, fp64_residuals=res64, fp32_corrections=corr32,
@@ -505,11 +520,12 @@ def measure_learned(n, N, train_count, steps, tc=512):
     kin = 3 + 2 * 3 * F + 2 * n
     # + the Newton step on each prediction: Hyman's recurrence for r in FP64 (4 n^2),
     # for r' in FP32 (4 n^2, with the FP32 work below)
-    f64 = fp64_flops(n, float(sw.double().sum()), N) + (N * 4.0 * n ** 3 if cfg["polish"] > 0 else 0.0)
+    imad = imad_ops(n, float(sw.double().sum()), N)
+    f64 = N * 4.0 * n ** 3 if cfg["polish"] > 0 else 0.0
     f32 = (polish_steps * (8.0 * n * n + 10.0 * n) + (N * 40.0 / 3.0 * n ** 3 if n <= 32 else 0.0) + N * 2.0 * h * 2 * n
            + (N * 4.0 * n ** 3 if cfg["polish"] > 0 else 0.0))
     fbf16 = N * 2.0 * (kin * h + (L - 1) * h * h)
-    rl = roofline(ms_learned * 1e-3, fp64=f64, fp32=f32, bf16=fbf16, hbm=hbm_bytes(n, N))
+    rl = roofline(ms_learned * 1e-3, imad=imad, fp64=f64, fp32=f32, bf16=fbf16, hbm=hbm_bytes(n, N))
     passed = ver["max_residual"] <= RES_TOL and ver["nonfinite"] == 0 and err <= 1e-12 and other == 0
     out = {"form": "learned shift", "n": n, "N": N, "value": r4(N / (ms_learned * 1e-3)), "ms": r4(ms_learned),
            "vs_plain": r4(ms_plain / ms_learned), "roofline": rl, "s": r4(float(sw.double().mean()) / n),
@@ -520,7 +536,7 @@ def measure_learned(n, N, train_count, steps, tc=512):
               "train": {"matrices": train_count, "epochs": epochs, "seconds": train_s, "loss_first": losses[0],
                         "loss_last": losses[-1], "network": cfg["net"]},
               "shift_polish": cfg["polish"], "shift_gate": cfg["gate"], "polish_steps": polish_steps,
-              "flops_fp64": f64, "flops_fp32": f32, "flops_bf16": fbf16,
+              "imad_wide": imad, "flops_fp64": f64, "flops_fp32": f32, "flops_bf16": fbf16,
               "nonfinite": ver["nonfinite"], "max_eig_err_rel": err}
     del net, rA, iA, rV, iV, ws, lws, pws, A
     torch.cuda.empty_cache()
@@ -561,7 +577,7 @@ def measure_varsize(count, steps, seed=2, max_dim=64):
     ves.eigensolve_varsize(count, max_dim, dims, re, im, er, ei, vr, vi, sweeps=sw, options=o)
     torch.cuda.synchronize()
     nd = torch.from_numpy(sizes.astype(np.float64)).cuda()
-    flops = float((24.0 * nd ** 3 + 20.0 * sw.double() * nd ** 2).sum())
+    imad = float((36.0 * nd ** 3 + 36.0 * sw.double() * nd ** 2).sum())
     # residuals per order bucket (packed column-major per matrix)
     off = np.concatenate([[0], np.cumsum(sizes.astype(np.int64) ** 2)])
     eoff = np.concatenate([[0], np.cumsum(sizes.astype(np.int64))])
@@ -597,14 +613,14 @@ def measure_varsize(count, steps, seed=2, max_dim=64):
             ves.eigensolve(n, 1, k, rs, is_, eb, eb2, vb, vb2, workspace=w, stream=stream)
 
     ms_per_order = timed(per_order, max(1, steps // 2))
-    rl = roofline(ms * 1e-3, fp64=flops, hbm=float((32.0 * nd * nd + 16.0 * nd).sum()))
+    rl = roofline(ms * 1e-3, imad=imad, hbm=float((32.0 * nd * nd + 16.0 * nd).sum()))
     out = {"form": "mixed-size batch", "n": "4..%d" % max_dim, "N": count, "value": r4(count / (ms * 1e-3)),
            "ms": r4(ms), "vs_per_order": r4(ms_per_order / ms), "roofline": rl,
            "s": r4(float(sw.double().sum()) / float(nd.sum())), "max_res": r4(worst),
            "passed": worst <= RES_TOL and bad == 0}
     detail = {"form": "mixed-size batch", "n_matrices": count, "orders": "uniform in [4, %d]" % max_dim,
               "families": "Gaussian / non-normal (cond(V)=1e4) / clustered (4 centres, radius 1e-6)",
-              "api": "ves_eigensolve_varsize captured in a CUDA graph, replayed", "flops_fp64": flops,
+              "api": "ves_eigensolve_varsize captured in a CUDA graph, replayed", "imad_wide": imad,
               "per_order_launches_value": count / (ms_per_order * 1e-3), "status_nonzero": bad}
     del g, bufs, per_n, re, im, vr, vi, er, ei, w
     torch.cuda.empty_cache()
@@ -662,7 +678,9 @@ def run_gpu_arm(args, d):
     except Exception:
         pass
     PEAKS.update(fp64=peak_fp64, fp32=ves.fp32_fma_rate(stream),
-                 bf16=peaks_file.get("bf16_tflops", 1900.0) * 1e12, hbm=peaks_file.get("hbm_gbs", 6800.0) * 1e9)
+                 bf16=peaks_file.get("bf16_tflops", 1900.0) * 1e12, hbm=peaks_file.get("hbm_gbs", 6800.0) * 1e9,
+                 imad=IMAD_PER_CLK_SM * torch.cuda.get_device_properties(d.local).multi_processor_count
+                 * peaks_file.get("sm_max_mhz", 2070.0) * 1e6)
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize()
@@ -691,7 +709,8 @@ def run_gpu_arm(args, d):
     ok = ver["max_residual"] <= RES_TOL and ver["nonfinite"] == 0 and bad_status == 0
 
     launch_s = ms * 1e-3 / args.steps
-    achieved = N * flops_per_matrix(n, s_mean) / launch_s
+    flops = N * flops_per_matrix(n, s_mean) / launch_s
+    achieved = imad_ops(n, s_mean * n * N, N) / launch_s
     hbm_b = hbm_bytes(n, N)
     hbm_peak = PEAKS["hbm"] / 1e9
     traffic = read_traffic()
@@ -758,11 +777,13 @@ def run_gpu_arm(args, d):
                    "n": n, "n_matrices": N_job, "thread_cnt": tc,
                    "form": "plain FP64", "l2": "inputs (4.3 GB) larger than L2; no flush",
                    "sweeps_per_eigenvalue": s_mean},
-        "roofline": {"bound": "fp64", "achieved": achieved / 1e12, "peak": peak_fp64 / 1e12, "unit": "TFLOP/s",
-                     "frac": achieved / peak_fp64, "traffic": traffic,
-                     "peak_source": "FP64 FMA rate measured in this run (ves_fp64_fma_rate); "
-                                    "MEASURED_PEAKS.json has no FP64 figure",
+        "roofline": {"bound": "imad", "achieved": achieved / 1e12, "peak": PEAKS["imad"] / 1e12,
+                     "unit": "T IMAD.WIDE/s", "frac": achieved / PEAKS["imad"], "traffic": traffic,
+                     "peak_source": "26 IMAD.WIDE per clock and SM, measured once on a GB300, at the maximum SM clock",
                      "flops_per_matrix": flops_per_matrix(n, s_mean),
+                     "fp64": {"achieved": flops / 1e12, "peak": peak_fp64 / 1e12, "unit": "TFLOP/s",
+                              "frac": flops / peak_fp64,
+                              "peak_source": "FP64 FMA rate measured in this run (ves_fp64_fma_rate)"},
                      "hbm": {"achieved_gbs": hbm_b / launch_s / 1e9, "peak_gbs": hbm_peak,
                              "frac": hbm_b / launch_s / 1e9 / hbm_peak, "bytes_per_matrix": 32 * n * n + 16 * n,
                              "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)"}},
@@ -772,7 +793,8 @@ def run_gpu_arm(args, d):
         "cpu_baseline": cpu,
         "e2e": e2e,
         "clocks": ck,
-        "gpu_launches": args.steps,
+        # per step: the fixed-point solve, and the two kernels over the matrices it leaves to FP64
+        "gpu_launches": 3 * args.steps,
         "verify": dict(ver, status_nonzero=bad_status, passed=ok),
         "forms": forms,
     }
@@ -788,8 +810,8 @@ def run_gpu_arm(args, d):
 
 
 def read_traffic():
-    """DRAM bytes per launch of the fused kernel from the committed ncu summary, or None."""
-    p = os.path.join(ROOT, "profiles", "fused_fp64_gauss16.md")
+    """DRAM bytes per launch of the plain solve from the committed ncu summary, or None."""
+    p = os.path.join(ROOT, "profiles", "fx_lane_gauss16.md")
     try:
         for ln in open(p):
             if ln.startswith("traffic_bytes_per_launch:"):

@@ -126,7 +126,9 @@ typedef struct ves_options {
     int want_vectors;  /* 1 (default): eigenvalues and eigenvectors; 0: eigenvalues only (FP64; the QR
                         * runs on the active block only, no Q and no Schur vectors -- the same
                         * eigenvalues, about a third of the QR work; rV/iV may be NULL) */
-    int blocks_per_sm; /* launch shape of the persistent kernels (4 warps per block); 0 = library default */
+    int blocks_per_sm; /* launch shape of the persistent kernels that keep their matrices in the workspace (4 warps
+                        * per block); 0 = library default.  Kernels that keep them in shared memory size
+                        * themselves. */
     int varsize_order; /* mixed-size batches: 0 (default) largest order first, 1 smallest first */
     int shift_sweeps;  /* ves_eigensolve_shifts: sweeps per eigenvalue that use a predicted shift; default 1 */
     float shift_gate;  /* ves_eigensolve_shifts: an eigenvalue uses the predictions only while its subdiagonal
@@ -146,7 +148,7 @@ typedef struct ves_options {
 
 /* Indices into ves_options.work_counts. */
 enum {
-    VES_WORK_RES64 = 0,   /* FP32_REFINE: FP64 residuals r = A v - lambda v (one per pair and Newton step) */
+    VES_WORK_RES64 = 0,   /* FP32_REFINE: FP64 or fixed-point residuals r = A v - lambda v (those that accept a pair) */
     VES_WORK_CORR32 = 1,  /* FP32_REFINE: FP32 Newton corrections through the Schur form */
     VES_WORK_RESFF = 2,   /* FP32_REFINE: first residuals in float-float (one per refined pair) */
     VES_WORK_POLISH = 3,  /* ves_eigensolve_shifts: FP32 Newton steps on det(H - sI), over all predictions */
@@ -159,10 +161,15 @@ void ves_default_options(ves_options *opt);
 size_t ves_eigensolve_workspace_size(int dim, int block_cnt, int thread_cnt, const ves_options *opt);
 
 /* Full eigen-decomposition on device data.
- * precision = VES_PREC_FP64: the reference path in FP64 (one launch).
+ * precision = VES_PREC_FP64: the reference path; for dim 3 .. 64 its unitary
+ *   transformations run in 64-bit fixed point with one scale per matrix (2^-61
+ *   ||A||_F a step, below FP64's rounding of the same sums), its scalar steps in
+ *   FP64.  Matrices that one scale does not serve (rows, columns or blocks that
+ *   differ widely in size, extreme exponents, not finite) and other orders run
+ *   in FP64 throughout.
  * precision = VES_PREC_FP32_REFINE: the reference path in complex FP32, then
  *   every eigenpair refined by Newton steps whose residual is computed in
- *   FP64, until ||A v - lambda v|| <= refine_tol ||A||_F ||v|| and the next
+ *   FP64 or in 64-bit fixed point, until ||A v - lambda v|| <= refine_tol ||A||_F ||v|| and the next
  *   Newton correction to lambda (its error estimate) is <= 4 refine_tol
  *   ||A||_F; a matrix that does not get there within refine_steps corrections
  *   (or whose FP32 QR hit the sweep cap, or whose data do not fit FP32) is
@@ -202,7 +209,7 @@ int ves_eigensolve(int dim, int block_cnt, int thread_cnt,
  * rV, iV), its eigenvalues at sum_{j<m} dims[j] of rE, iE.  Orders must lie in
  * [1, max_dim] with max_dim <= VES_VARSIZE_MAX_DIM; other matrices are skipped
  * and flagged VES_STATUS_BAD_DIM.  The batch is binned by order on the device
- * and solved by one persistent FP64 launch (largest orders first unless
+ * and solved by one persistent launch (the arithmetic of ves_eigensolve; largest orders first unless
  * varsize_order = 1); no host synchronisation, so the call can be captured in
  * a CUDA graph (see ves_graph_capture_varsize).  workspace must hold
  * ves_eigensolve_varsize_workspace_size() bytes (or be NULL: cached). */
