@@ -102,7 +102,7 @@ __device__ __forceinline__ void fx_lanes(const FxArgs &a)
                 sh.P.st(k, valid ? mk(a.rS[vo + (long long)(k - 1) * tc], a.iS[vo + (long long)(k - 1) * tc]) : mk(0.0, 0.0));
             ok = fx_solve<1, kVec>(gr, n, H, Z, U, valid, a.rA + mo, a.iA + mo, tc, o, a.max_its, a.vnorm, sweeps,
                                    status, ch, &sh);
-            if (sh.sp.fallbacks) status |= ST_SHIFT_FALLBACK;
+            if (ok && sh.sp.fallbacks) status |= ST_SHIFT_FALLBACK;
             if (ok && a.fallbacks) a.fallbacks[m] = sh.sp.fallbacks;
         } else {
             ok = fx_solve<G, kVec>(gr, n, H, Z, U, valid, a.rA + mo, a.iA + mo, tc, o, a.max_its, a.vnorm, sweeps,

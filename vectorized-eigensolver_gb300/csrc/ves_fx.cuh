@@ -354,6 +354,8 @@ template <int G> struct FxGroup {
         return RG == 1 ? (unsigned)p : __ballot_sync(mask, p) >> shift;
     }
     __device__ __forceinline__ bool all(bool p) const { return ballot(!p) << (32 - RG) == 0; }
+    // whether a matrix that shares this control flow has p (p is the same on all lanes of a group)
+    __device__ __forceinline__ bool any(bool p) const { return G == 1 ? __any_sync(FULL, p) : p; }
     __device__ __forceinline__ i64 sum(i64 v) const
     {
 #pragma unroll
@@ -393,6 +395,7 @@ template <int G> struct FxLanes {
     {
         return fold((int)p, [](int a, int b) { return a & b; });
     }
+    __device__ __forceinline__ bool any(bool p) const { return __any_sync(FULL, p); }
     __device__ __forceinline__ i64 sum(i64 v) const
     {
         return fold(v, [](i64 a, i64 b) { return a + b; });
@@ -604,11 +607,16 @@ __device__ __forceinline__ void fx_reflect_all(const int gl, longlong2 *a, const
     for (; v < count; v += G) fx_reflect<1, ST>(a + v * blk, step, 0, u, ST, u1.r, u1.i, m, cj);
 }
 
+constexpr i64 kFxMinSub = 1LL << 31;  // 2^-30 of the scale
+
 // Householder reduction to Hessenberg form with Hermitian reflectors
 // P = I - u u^H, ||u||^2 = 2 (the subdiagonal comes out complex).  u_k, k >=
-// i + 2, stays below the subdiagonal of column i, u_{i+1} in U(i).
+// i + 2, stays below the subdiagonal of column i, u_{i+1} in U(i).  ok turns
+// false at a subdiagonal that fx_irreducible rejects; the reduction ends where
+// no matrix is left for which it is needed (a batch of triangular or
+// block-triangular matrices would otherwise pay for it twice).
 template <int G, class GR, int ST>
-__device__ __forceinline__ void fx_reduce(const GR &gr, const int n, const FxMat<ST> &H, const FxVec<ST> &U)
+__device__ __forceinline__ void fx_reduce(const GR &gr, const int n, const FxMat<ST> &H, const FxVec<ST> &U, bool &ok)
 {
     constexpr int RG = GR::RG;
     const int rs = ST, cs = H.lda * ST;  // steps to the next row, the next column
@@ -656,6 +664,8 @@ __device__ __forceinline__ void fx_reduce(const GR &gr, const int n, const FxMat
             H.st(i + 1, i, beta);
         }
         gr.sync();
+        ok = ok && fx_abs1(beta) >= kFxMinSub;
+        if (!gr.any(ok)) return;
         const longlong2 *u = H.at(i + 2, i);
         fx_reflect_all<G, ST>(gr.gl, H.at(1, i + 1), cs, rs, n, u, u1, n - i, true);  // rows of A(:, i+1:n)
         gr.sync();
@@ -678,12 +688,12 @@ __device__ __forceinline__ void fx_form_q(const GR &gr, const int n, const FxMat
     }
 }
 
-// no subdiagonal below 2^-30 of the scale
+// no subdiagonal below kFxMinSub
 template <int G, class GR, int ST>
 __device__ __forceinline__ bool fx_irreducible(const GR &gr, const int n, const FxMat<ST> &H)
 {
     bool ok = true;
-    for (int k = gr.rl + 2; k <= n; k += GR::RG) ok = ok && fx_abs1(H.ld(k, k - 1)) >= (1LL << 31);
+    for (int k = gr.rl + 2; k <= n; k += GR::RG) ok = ok && fx_abs1(H.ld(k, k - 1)) >= kFxMinSub;
     return gr.all(ok);
 }
 
@@ -1274,9 +1284,15 @@ __device__ __forceinline__ bool fx_solve(const GR &gr, const int n, const FxMat<
 {
     double unit;
     bool ok = fx_load<G>(gr, n, H, valid, rA, iA, s, unit);
-    fx_reduce<G>(gr, n, H, U);
-    const bool irreducible = fx_irreducible<G>(gr, n, H);  // every lane takes part, whatever ok is
-    ok = ok && irreducible;
+    if (gr.any(ok)) fx_reduce<G>(gr, n, H, U, ok);
+    if (gr.any(ok)) {
+        const bool irreducible = fx_irreducible<G>(gr, n, H);  // every lane takes part, whatever ok is
+        ok = ok && irreducible;
+    }
+    if (!gr.any(ok)) {
+        gr.sync();
+        return false;
+    }
     typename SH::Picker *sp = nullptr;
     if constexpr (SH::kOn) {
         const FxVec<32> Sub{shifts->scratch + 5 * n * 32};
