@@ -175,3 +175,18 @@ def test_varsize_few_large_among_many_small(count):
         for k, i in enumerate(idx):
             assert np.array_equal(gotE[eo[i]:eo[i] + d], ref["E"][k]), (d, i)
             assert np.array_equal(gotV[vo[i]:vo[i] + d * d].reshape(d, d).T, ref["V"][k]), (d, i)
+
+
+@pytest.mark.parametrize("n,N", [(8, 5000), (16, 9000)])
+def test_long_and_short_fp64_lists_same_bits(n, N):
+    """A batch that the fixed-point form leaves to FP64 altogether: a long list
+    goes one matrix per lane, short ones one per warp, with the same bits."""
+    rng = np.random.default_rng(700 + n)
+    A = cgauss(rng, (N, n, n))
+    A[:, n // 2:, :n // 2] = 0
+    out = run_fused(A, N, vnorm=2)
+    check(A[:40], {k: v[:40] for k, v in out.items()})
+    for s in (0, N - 100):
+        part = run_fused(A[s:s + 100], 100, vnorm=2)
+        for key, want in part.items():
+            assert np.array_equal(out[key][s:s + 100], want), key

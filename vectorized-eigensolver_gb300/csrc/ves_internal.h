@@ -41,8 +41,8 @@ struct FusedArgs {
     // optional index list: solve only matrices list[0 .. *list_count) (the
     // mixed-precision form's fallback pass, matrices outside the fixed-point
     // form's range); status gets the bits of status_or.
-    // The lane kernel takes entries from list_split on, fp64_warp_kernel the
-    // ones before it (launch_fp64_list sets it).
+    // fp64_warp_kernel takes a list of at most list_split matrices, the lane
+    // kernel a longer one (launch_fp64_list sets it).
     const int *list;
     const int *list_count;
     int status_or;

@@ -81,7 +81,8 @@ __global__ void __launch_bounds__(kFusedThreads) fused_fp64_kernel(const FusedAr
     const int lane = threadIdx.x & 31;
     const long long slot = (long long)blockIdx.x * (kFusedThreads / 32) + (threadIdx.x >> 5);
     const long long nslots = (long long)gridDim.x * (kFusedThreads / 32);
-    const long long Nw = a.list ? (long long)*a.list_count - a.list_split : N;
+    // (a list of at most list_split matrices is fp64_warp_kernel's)
+    const long long Nw = a.list ? (*a.list_count > a.list_split ? (long long)*a.list_count : 0) : N;
     const long long ngroups = (Nw + 31) / 32;
     const long long per_lane = fused_slot_elems(n, kLearned);  // H, Z, work vector (+ FP32 H, predictions)
 
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(kFusedThreads) fused_fp64_kernel(const FusedAr
     for (long long g = slot; g < ngroups; g += nslots) {
         const long long idx = g * 32 + lane;
         const bool valid = idx < Nw;
-        const long long m = valid ? (a.list ? (long long)a.list[a.list_split + idx] : idx) : 0;
+        const long long m = valid ? (a.list ? (long long)a.list[idx] : idx) : 0;
         const long long mo = valid ? soa_mat_off(m, n, tc) : 0;
         const long long vo = valid ? soa_vec_off(m, n, tc) : 0;
         int status = 0, sweeps = 0;
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(32) fp64_warp_kernel(const FusedArgs a)
     double2 *sTau = fsm + 3 * n * lda, *sS = sTau + n;
     const double ulp = lim<double>::eps();
     const double smlnum = lim<double>::tiny() * ((double)n / ulp);
-    const long long count = a.list ? (long long)min(*a.list_count, (int)a.list_split) : a.g.N;
+    const long long count = a.list ? (*a.list_count <= a.list_split ? (long long)*a.list_count : 0) : a.g.N;
 
     for (long long w = blockIdx.x; w < count; w += gridDim.x) {
         const long long m = a.list ? (long long)a.list[w] : w;
@@ -792,6 +793,13 @@ cudaError_t launch_polish32(Geom g, const double *rA, const double *iA, const do
     return cudaGetLastError();
 }
 
+// The matrices on a list: one per warp for a list of up to n / 5 waves of
+// fp64_warp_kernel, which is about what a wave of the lane kernel takes however
+// few matrices it has, else one per lane.  Measured on GB300, whole solves with the
+// first wave per warp and the rest per lane -> this, ms: n=48, 500 block-triangular
+// matrices 227 -> 29.6; every tenth matrix block-triangular, n=16 x 100,000 41.1 ->
+// 36.1, n=32 x 20,000 125 -> 68.6, n=48 x 4,000 274 -> 80.1; all of them, n=16 x
+// 100,000 55.0 -> 50.0 (but n=32 x 20,000 98.8 -> 111).
 cudaError_t launch_fp64_list(FusedArgs a, cudaStream_t st)
 {
     if (a.g.N <= 0) return cudaSuccess;
@@ -799,10 +807,11 @@ cudaError_t launch_fp64_list(FusedArgs a, cudaStream_t st)
     if (a.list && !a.rS && a.g.n <= 64) {
         // one matrix per warp slot: 228 KB of shared memory, at most 16 a SM (64 K registers)
         const long long per_sm = std::max<long long>(1, std::min<long long>(16, 228 * 1024 / (fp64_warp_smem(a.g.n) + 1024)));
-        a.list_split = std::min<long long>(a.g.N, device_sms() * per_sm);
-        fp64_warp_kernel<<<(unsigned)a.list_split, 32, fp64_warp_smem(a.g.n), st>>>(a);
+        const long long slots = device_sms() * per_sm;
+        a.list_split = slots * std::max(1, a.g.n / 5);
+        fp64_warp_kernel<<<(unsigned)std::min(a.g.N, slots), 32, fp64_warp_smem(a.g.n), st>>>(a);
         const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess || a.g.N <= a.list_split) return e;
     }
     return launch_fused_fp64(a, st);
 }
