@@ -146,7 +146,6 @@ def test_mixed_larger_batches(n, N, tc):
     out = run_fused(A, tc, precision=MIX)
     assert residuals(A, out["E"], out["V"]).max() <= 1e-13
     check(A[-40:], {k: v[-40:] for k, v in out.items()})
-    # a matrix's result does not depend on the batch around it, nor on the stream overlap of large batches
     assert (out["status"] & ~ves.VES_STATUS_REFINE_FALLBACK == 0).all()
 
 
