@@ -61,13 +61,13 @@ constexpr int kLaneThreads = 128;
 template <int G, bool kVec, bool kShifts>
 __device__ __forceinline__ void fx_lanes(const FxArgs &a)
 {
-    constexpr int kChunk = FxChunkOf<G>::k, M = 32 / G;
-    __shared__ longlong2 chs[kLaneThreads * kChunk];
+    constexpr int kChunk = FxChunkOf<G>::k, kSlots = FxChunkOf<G>::slots, M = 32 / G;
+    __shared__ longlong2 chs[kLaneThreads * kSlots];
     __shared__ i64 chi[kLaneThreads * kChunk];
     const FxLanes<G> gr;
     const int n = a.g.n, tc = a.g.tc, lane = threadIdx.x & 31, mat = lane % M;
-    const int ch0 = (threadIdx.x >> 5) * 32 * kChunk + lane;
-    const FxChunk ch{chs + ch0, chi + ch0};
+    const int warp0 = (threadIdx.x >> 5) * 32;
+    const FxChunk ch{chs + warp0 * kSlots + lane, chi + warp0 * kChunk + lane};
     const long long slot = (long long)blockIdx.x * (kLaneThreads / 32) + (threadIdx.x >> 5);
     const long long nslots = (long long)gridDim.x * (kLaneThreads / 32);
     const long long nn = (long long)n * n, nu = (kVec ? 2 : 1) * nn;

@@ -701,11 +701,13 @@ __device__ __forceinline__ bool fx_irreducible(const GR &gr, const int n, const 
 // cap, which moves on) until an eigenvalue needs a sweep; false when none is
 // left.  (a0, a1): the vector of the sweep's first rotation, from Wilkinson's
 // shift or, at the 10th and 20th sweep, the reference's exceptional ones.
-// sp: predicted shifts, in the units of H.
+// sp: predicted shifts, in the units of H.  peers: with one lane's scan per lane
+// (G = 1) but several lanes per matrix, those lanes.
 template <int G, int ST, class SP = NoShiftPredictions>
 __device__ __forceinline__ bool fx_next_sweep(const FxGroup<G> &gr, const int n, const FxMat<ST> &H,
                                               const FxVec<ST> &S, const int max_its, int &I, int &L, int &its,
-                                              int &status, cx<double> &a0, cx<double> &a1, SP *sp = nullptr)
+                                              int &status, cx<double> &a0, cx<double> &a1, SP *sp = nullptr,
+                                              const unsigned peers = 0)
 {
     constexpr int RG = FxGroup<G>::RG;
     for (;;) {
@@ -731,6 +733,7 @@ __device__ __forceinline__ bool fx_next_sweep(const FxGroup<G> &gr, const int n,
         }
         L = K;
         if (G > 32) __syncthreads();  // the scans have read S
+        else if (peers) __syncwarp(peers);
         if (L > 1) S.std(L - 1, mk(0.0, 0.0));  // every lane: the same value
         if (L >= I) {
             if constexpr (SP::kOn) sp->deflated(its);
@@ -906,7 +909,12 @@ __device__ __forceinline__ void fx_qr(const FxGroup<G> &gr, const int n, const F
 // Rotations of the current chunk of a sweep, in shared memory, one set per lane.
 // (n=16, one lane per matrix, chunk 4, 8, 16: 277, 274, 260 ms per 1,048,576)
 constexpr int kFxChunk = 16;
-template <int G> struct FxChunkOf { static constexpr int k = G == 1 ? kFxChunk : 8; };
+// k: rotations of a chunk; slots: 16-byte elements per lane, those and (G > 1) the
+// lane's rows of the chunk
+template <int G> struct FxChunkOf {
+    static constexpr int k = G == 1 ? kFxChunk : 8;
+    static constexpr int slots = k + (G > 1 ? k / G : 0);
+};
 constexpr int kFxStream = 2;  // chains streamed together
 struct FxChunk {
     longlong2 *cs;  // (c, sr) of rotation k at cs[k * 32]
@@ -921,6 +929,8 @@ struct FxChunk {
         const longlong2 a = cs[k * 32];
         return FxCoef(a.x, a.y, si[k * 32]);
     }
+    // G > 1: entry of the lane's row t of the chunk in the column that the next rotation turns
+    template <int G> __device__ __forceinline__ longlong2 *row(int t) const { return cs + (FxChunkOf<G>::k + t) * 32; }
 };
 
 // Apply ns rotations (c, s at cs[k * 32], si[k * 32]) to NB chains of entries:
@@ -988,13 +998,20 @@ __device__ __forceinline__ void fx_stream_all(const int gl, longlong2 *p, const 
 
 // fx_qr for one matrix per lane, or per G lanes of FxLanes, the warp's matrices
 // in lockstep per sweep, in its workspace.  The lanes of a matrix compute the
-// chain alike and share out the rows and columns.  A sweep runs in chunks of kFxChunk rotations: first the chain of
-// rotations, which needs of the matrix only the chunk's own columns (the left
-// rotations of the chunk are applied to column K + 1 when rotation K is due)
-// and the diagonal; then the chunk's rotations are streamed over the rows of Z,
-// the rows above and the columns to the right.  A lane whose window does not
-// contain K takes part with the identity, which leaves integers unchanged.
-// The entries see the same operations as in fx_qr.
+// chain alike and share out the rows and columns.  A sweep runs in chunks of
+// FxChunkOf<G>::k rotations: first the chain of rotations, which needs of the
+// matrix only the chunk's own columns (the left rotations of the chunk are
+// applied to column K + 1 when rotation K is due) and the diagonal; then the
+// chunk's rotations are streamed over the rows of Z, the rows above and the
+// columns to the right.  A lane whose window does not contain K takes part with
+// the identity, which leaves integers unchanged.  The entries see the same
+// operations as in fx_qr.
+//
+// G > 1: every lane reads column K + 1 and S(K + 1) as they were before rotation
+// K, so nothing of them may be written before all lanes have read them.  A row's
+// owner therefore keeps its entry of column K + 1 in shared memory until rotation
+// K + 1 has turned it, column K is written after the barrier that opens rotation
+// K, and the diagonal stays in registers to the end of the chunk.
 template <int G, bool kVec, int ST, class SP>
 __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, const FxMat<ST> &H, const FxMat<ST> &Z, const FxVec<ST> &S,
                                            const FxChunk &ch, const bool run, const int max_its, int &sweeps,
@@ -1004,11 +1021,14 @@ __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, co
     constexpr int kChunk = FxChunkOf<G>::k;
     const int rs = ST, cs = n * ST;  // steps to the next row, the next column
     const int gl = G == 1 ? 0 : group_lane;
+    unsigned peers = 0;  // the lanes of this matrix
+    if (G > 1)
+        for (int t = 0; t < G; ++t) peers |= 1u << ((threadIdx.x & (32 / G - 1)) + t * (32 / G));
     int I = n, L = 1, its = 0;
     bool done = !run || n <= 1;
     for (;;) {
         cx<double> a0, a1, sub;
-        const bool sweep = !done && fx_next_sweep<1>(gr, n, H, S, max_its, I, L, its, status, a0, a1, sp);
+        const bool sweep = !done && fx_next_sweep<1>(gr, n, H, S, max_its, I, L, its, status, a0, a1, sp, peers);
         done = !sweep;
         sub = a1;
         sweeps += sweep;
@@ -1025,10 +1045,11 @@ __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, co
                 R.ds = mk(0.0, 0.0);
                 R.c = 1LL << 62;
                 R.sr = R.si = 0;
+                if (G > 1) __syncwarp();  // what this rotation writes has been read
                 // column K + 1: the chunk's left rotations so far; each row that is done takes
                 // rotation K from the right, with its entry of column K
                 longlong2 *pc = H.at(Kc, K + 1), *pl = H.at(Kc, K);
-                longlong2 v = pc[0], w = pl[0];
+                longlong2 v = pc[0], w = G == 1 ? pl[0] : v;
                 cx64 x = {v.x, v.y};
                 v = pc[rs];
                 cx<double> r, nxt = mk(0.0, 0.0);
@@ -1038,15 +1059,22 @@ __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, co
                 }
                 ch.put(K - Kc, R);
                 const FxCoef C(R), CC = C.columns();
-                for (int q = Kc; q < K; ++q) {
-                    cx64 y = {v.x, v.y}, z = {w.x, w.y};
+                for (int q = 0; q < K - Kc; ++q) {
+                    cx64 y = {v.x, v.y};
                     v = pc[2 * rs];
-                    w = pl[rs];
-                    fx_pair(x, y, ch.get(q - Kc));
-                    if (G == 1 || (q & (G - 1)) == gl) {  // the rows of a chunk are shared out
+                    fx_pair(x, y, ch.get(q));
+                    if (G == 1) {
+                        cx64 z = {w.x, w.y};
+                        w = pl[rs];
                         fx_pair(z, x, CC);
                         pl[0] = make_longlong2(z.r, z.i);
                         pc[0] = make_longlong2(x.r, x.i);
+                    } else if ((q & (G - 1)) == gl) {  // the rows of a chunk are shared out
+                        longlong2 *const row = ch.row<G>(q / G);
+                        cx64 z = {row->x, row->y};
+                        fx_pair(z, x, CC);
+                        pl[0] = make_longlong2(z.r, z.i);
+                        *row = make_longlong2(x.r, x.i);
                     }
                     x = y;
                     pc += rs;
@@ -1058,9 +1086,9 @@ __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, co
                 fx_pair(x, y, C);
                 fx_pair(hkk, y2, C);
                 fx_pair(hkk, x, CC);
-                if (G == 1 || (K & (G - 1)) == gl) {
+                if (((K - Kc) & (G - 1)) == gl) {
                     pl[0] = make_longlong2(hkk.r, hkk.i);
-                    pc[0] = make_longlong2(x.r, x.i);
+                    *(G == 1 ? pc : ch.row<G>((K - Kc) / G)) = make_longlong2(x.r, x.i);
                 }
                 if (act) {
                     const cx<double> ks = conj(R.ds);
@@ -1074,9 +1102,14 @@ __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, co
                     if (K == I - 1 && gl == 0) S.std(I - 1, a0);
                 }
                 hkk = y;
-                if (gl == 0) H.st(K + 1, K + 1, y);
+                if (G == 1) H.st(K + 1, K + 1, y);
             }
-            if (G > 1) __syncwarp();
+            if (G > 1) {
+                __syncwarp();  // column Ke + 1 has been read
+                for (int q = gl; q < ns; q += G) *H.at(Kc + q, Ke + 1) = *ch.row<G>(q / G);
+                if (gl == 0) H.st(Ke + 1, Ke + 1, hkk);
+                __syncwarp();
+            }
             // rows above the chunk
             const int r0 = kVec ? 1 : Kmin;
             if (Kc > r0) fx_stream_all<G>(gl, H.at(r0, Kc), cs, rs, Kc - r0, ch, ns, true);

@@ -177,6 +177,7 @@ struct VarArgs {
 
 __global__ void __launch_bounds__(kSolveThreads, 4) varsize_solve_kernel(const VarArgs a)
 {
+    static_assert(FxChunkOf<kWide>::slots <= kFxChunk, "one size of chunk storage for both kinds of items");
     __shared__ longlong2 chs[kSolveThreads * kFxChunk];
     __shared__ i64 chi[kSolveThreads * kFxChunk];
     const int lane = threadIdx.x & 31;
