@@ -354,8 +354,10 @@ template <int G> struct FxGroup {
         return RG == 1 ? (unsigned)p : __ballot_sync(mask, p) >> shift;
     }
     __device__ __forceinline__ bool all(bool p) const { return ballot(!p) << (32 - RG) == 0; }
-    // whether a matrix that shares this control flow has p (p is the same on all lanes of a group)
-    __device__ __forceinline__ bool any(bool p) const { return G == 1 ? __any_sync(FULL, p) : p; }
+    // whether a matrix of the warp has p (p is the same on all lanes of a group).  The
+    // groups of a warp share its votes in the QR sweeps, so they leave a solve together:
+    // all 32 lanes call this.
+    __device__ __forceinline__ bool any(bool p) const { return G < 32 ? __any_sync(FULL, p) : p; }
     __device__ __forceinline__ i64 sum(i64 v) const
     {
 #pragma unroll
