@@ -209,6 +209,7 @@ inline long long __double2ll_rn(double d) { return llrint(d); }
 inline long long __float2ll_rn(float f) { return llrintf(f); }
 inline int __float2int_rn(float f) { return (int)lrintf(f); }
 inline unsigned long long __umul64hi(unsigned long long a, unsigned long long b) { return (unsigned long long)(((unsigned __int128)a * b) >> 64); }
+inline int __clz(int x) { return x ? __builtin_clz(x) : 32; }
 inline int __clzll(long long x) { return x ? __builtin_clzll(x) : 64; }
 inline unsigned __funnelshift_l(unsigned lo, unsigned hi, unsigned s) { return s & 31 ? (hi << (s & 31)) | (lo >> (32 - (s & 31))) : hi; }
 inline int __ffs(int x) { return __builtin_ffs(x); }

@@ -51,3 +51,38 @@ def test_solves_in_fixed_point():
     for k in np.nonzero(out["ok"])[0]:
         R = A[k] @ out["V"][k] - out["V"][k] * out["E"][k]
         assert np.linalg.norm(R, axis=0).max() <= 1e-14 * np.linalg.norm(A[k])
+
+
+def bordered(rng, N, n, eps, hermitian, first=0):
+    """A weak block (entries of size eps) beside strong rows and columns: row and column
+    `first`, and before it a chain of couplings, so that no reflector mixes the two."""
+    A = eps * (rng.standard_normal((N, n, n)) + 1j * rng.standard_normal((N, n, n)))
+    strong = rng.standard_normal((N, n, n)) + 1j * rng.standard_normal((N, n, n))
+    A[:, first, first:], A[:, first:, first] = strong[:, first, first:], strong[:, first:, first]
+    A[:, :first, :], A[:, :, :first] = 0, 0
+    for k in range(first):
+        A[:, k, k:k + 2], A[:, k:k + 2, k] = strong[:, k, k:k + 2], strong[:, k:k + 2, k]
+    return (A + A.conj().transpose(0, 2, 1)) / 2 if hermitian else A
+
+
+@pytest.mark.parametrize("n,first", [(3, 0), (4, 0), (5, 1), (8, 0), (8, 2), (13, 5), (16, 0), (33, 0)])
+@pytest.mark.parametrize("hermitian", [False, True])
+@pytest.mark.parametrize("form", ["l1", "l4", "g8"])
+def test_weak_block_is_left_to_fp64(n, first, hermitian, form):
+    rng = np.random.default_rng(50 + n)
+    A = np.concatenate([bordered(rng, 1, n, 2.0 ** -k, hermitian, first) for k in range(9, 28)])
+    out = fx_host.solve(A, form)
+    assert not out["error"] and not out["ok"].any()
+
+
+@pytest.mark.parametrize("n", [3, 4, 5, 8, 16, 33, 64])
+def test_ordinary_matrices_stay_in_fixed_point(n):
+    rng = np.random.default_rng(60 + n)
+    N = 200 if n <= 16 else 12
+    A = rng.standard_normal((N, n, n)) + 1j * rng.standard_normal((N, n, n))
+    H = (A + A.conj().transpose(0, 2, 1)) / 2
+    phase = np.exp(2j * np.pi * rng.random((N, n, n)))
+    chain = np.zeros((1, n, n), complex)
+    chain[0] = np.diag(rng.uniform(-1, 1, n)) + np.diag(np.ones(n - 1), 1) + np.diag(np.ones(n - 1), -1)
+    for B in (A, H, A.real + 0j, phase, bordered(rng, N, n, 1 / 4, False), chain):
+        assert fx_host.solve(B)["ok"].all()
