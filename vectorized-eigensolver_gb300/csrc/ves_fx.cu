@@ -11,6 +11,14 @@ namespace ves {
 
 namespace {
 
+// Matrices to work on: the batch, or a list whose length lies in the launch's range.
+__device__ __forceinline__ long long fx_count(const FxArgs &a)
+{
+    if (!a.list) return a.g.N;
+    const long long c = *a.list_count;
+    return c > a.list_above && c <= a.list_upto ? c : 0;
+}
+
 template <int G> struct FxShape {
     static constexpr int threads = G > 32 ? G : 32;
     static constexpr int mats = G < 32 ? 32 / G : 1;  // matrices per block
@@ -27,7 +35,7 @@ __global__ void __launch_bounds__(FxShape<G>::threads) fx_kernel(const FxArgs a)
     const int lda = fx_lda(n);
     const FxMat<1> H{sm, lda, n}, Z{sm + (kVec ? n * lda : 0), lda, n};
     const FxVec<1> U{sm + (kVec ? 2 : 1) * n * lda};
-    const long long Nw = a.list ? (long long)*a.list_count : a.g.N;
+    const long long Nw = fx_count(a);
     for (long long base = (long long)blockIdx.x * M; base < Nw; base += (long long)gridDim.x * M) {
         const long long w = base + (G < 32 ? threadIdx.x / G : 0);
         const bool valid = w < Nw;
@@ -74,7 +82,7 @@ __device__ __forceinline__ void fx_lanes(const FxArgs &a)
     longlong2 *base = static_cast<longlong2 *>(a.ws) + slot * (kShifts ? shift_slot_elems(n) : nu + n) * M + mat;
     const FxMat<M> H{base, n, n}, Z{base + (kVec ? nn * M : 0), n, n};
     const FxVec<M> U{base + nu * M};
-    const long long Nw = a.list ? (long long)*a.list_count : a.g.N;
+    const long long Nw = fx_count(a);
     for (long long group = slot; group * M < Nw;) {
         const long long w = group * M + mat;
         const bool valid = w < Nw;
@@ -154,7 +162,8 @@ template <int G, bool kVec> cudaError_t launch_fx_g(const FxArgs &a, cudaStream_
 {
     const size_t smem = fx_smem<G>(a.g.n, kVec);
     if (smem > kMaxSmem) return cudaErrorInvalidValue;
-    const long long need = (a.g.N + FxShape<G>::mats - 1) / FxShape<G>::mats;
+    const long long work = a.list ? std::min(a.g.N, a.list_upto) : a.g.N;
+    const long long need = (work + FxShape<G>::mats - 1) / FxShape<G>::mats;
     const long long blocks = std::min<long long>(need, (long long)fx_sms() * fx_blocks_per_sm(G, smem));
     fx_kernel<G, kVec><<<(unsigned)std::max<long long>(blocks, 1), FxShape<G>::threads, smem, st>>>(a);
     return cudaGetLastError();
@@ -197,42 +206,68 @@ struct FxChoice {
     bool lanes;
     int G;
 };
-FxChoice fx_choose(int n, long long N, bool vec)
+// x^p of the fits, x = n / 8
+double fx_pow(int n, double p) { return pow(n / 8.0, p); }
+// ms of the lane kernel with G = 2^k lanes per matrix; N = 0: of a warp alone
+double fx_lane_ms(int n, long long N, int k, bool vec)
+{
+    const double lat = vec ? 0.07 + 1.05 * fx_pow(n, 2.66) : 0.066 + 0.43 * fx_pow(n, 2.66);
+    const double a = std::min(1.0, (vec ? 1.9 : 3.0) / pow(n, 0.62));
+    const double c[4] = {1.5, 1.2, 1.3, 0.8}, r[4] = {1, 0.57, 0.2, 0.15};
+    const int G = 1 << k;
+    const double w = (double)N * G / 32 / (fx_sms() * 16.0), full = floor(w), alone = a + (1 - a) / G;
+    return lat * (N == 0 ? alone
+                  : vec  ? alone * (full * (1 + c[k]) + (w > full ? 1 + c[k] * (w - full) : 0))
+                         : std::max(alone, r[k] + 1.64 * w));
+}
+// matrices of a wave of the group kernel, and ms of N matrices (G fits: fx_group_fits)
+long long fx_group_wave(int n, int G, bool vec)
+{
+    const int mats = G < 32 ? 32 / G : 1;
+    return (long long)fx_sms() * mats * fx_blocks_per_sm(G, (size_t)mats * fx_slot(n, G, vec) * sizeof(longlong2));
+}
+double fx_group_ms(int n, long long N, int G, bool vec)
+{
+    const int mats = G < 32 ? 32 / G : 1;
+    const double wave = (double)fx_group_wave(n, G, vec);
+    double t = ceil(N / wave) * (vec ? 0.33 : 0.30) * fx_pow(n, 1.85) * (1.0 + n / ((vec ? 3.0 : 5.0) * G));
+    if (G > 32) t *= 1.0 + 0.03 * std::min(wave / (fx_sms() * mats), ceil((double)N / (fx_sms() * mats))) * G / 32;
+    return t;
+}
+bool fx_group_fits(int n, int G, bool vec)
+{
+    return G <= (G > 32 ? 2 : 4) * n && (size_t)(G < 32 ? 32 / G : 1) * fx_slot(n, G, vec) * sizeof(longlong2) <= kMaxSmem;
+}
+int fx_best_group(int n, long long N, bool vec)
+{
+    int best = 0;
+    for (int G = 4; G <= 128; G *= 2)
+        if (fx_group_fits(n, G, vec) && (!best || fx_group_ms(n, N, G, vec) < fx_group_ms(n, N, best, vec))) best = G;
+    return best;
+}
+bool fx_forced(FxChoice &c)
 {
     if (const char *e = getenv("VES_FX_LANES")) {  // tuning: 1, 2, 4, 8 lanes ("l4"), or a group of 4 .. 128 ("g16")
         const int v = atoi(e + (*e != 0));
-        if (e[0] == 'l' && (v == 1 || v == 2 || v == 4 || v == 8)) return {true, v};
-        if (e[0] == 'g' && v >= 4 && v <= 128 && (v & (v - 1)) == 0) return {false, v};
+        if (e[0] == 'l' && (v == 1 || v == 2 || v == 4 || v == 8)) { c = {true, v}; return true; }
+        if (e[0] == 'g' && v >= 4 && v <= 128 && (v & (v - 1)) == 0) { c = {false, v}; return true; }
     }
-    const double sms = fx_sms(), x = n / 8.0;
+    return false;
+}
+FxChoice fx_choose(int n, long long N, bool vec)
+{
     FxChoice best{true, 1};
+    if (fx_forced(best)) return best;
     double t = 1e300;
-    const double lat = vec ? 0.07 + 1.05 * pow(x, 2.66) : 0.066 + 0.43 * pow(x, 2.66);
-    const double a = std::min(1.0, (vec ? 1.9 : 3.0) / pow(n, 0.62));
-    const double c[4] = {1.5, 1.2, 1.3, 0.8}, r[4] = {1, 0.57, 0.2, 0.15};
     for (int k = 0; k < 4; ++k) {
-        const int G = 1 << k;
-        const double w = (double)N * G / 32 / (sms * 16), full = floor(w), alone = a + (1 - a) / G;
-        const double tl = lat * (vec ? alone * (full * (1 + c[k]) + (w > full ? 1 + c[k] * (w - full) : 0))
-                                     : std::max(alone, r[k] + 1.64 * w));
+        const double tl = fx_lane_ms(n, N, k, vec);
         if (tl < t) {
             t = tl;
-            best = {true, G};
+            best = {true, 1 << k};
         }
     }
-    for (int G = 4; G <= 128; G *= 2) {
-        if (G > 32 ? G > 2 * n : G > 4 * n) break;
-        const int mats = G < 32 ? 32 / G : 1;
-        const size_t smem = (size_t)mats * fx_slot(n, G, vec) * sizeof(longlong2);
-        if (smem > kMaxSmem) continue;
-        const double fit = fx_blocks_per_sm(G, smem), waves = ceil((double)N / (sms * fit * mats));
-        double tg = waves * (vec ? 0.33 : 0.30) * pow(x, 1.85) * (1.0 + n / ((vec ? 3.0 : 5.0) * G));
-        if (G > 32) tg *= 1.0 + 0.03 * std::min(fit, ceil((double)N / (sms * mats))) * G / 32;
-        if (tg < t) {
-            t = tg;
-            best = {false, G};
-        }
-    }
+    const int G = fx_best_group(n, N, vec);
+    if (G && fx_group_ms(n, N, G, vec) < t) best = {false, G};
     return best;
 }
 
@@ -261,13 +296,40 @@ cudaError_t launch_fx_shifts(const FxArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
+static cudaError_t launch_fx_group(const FxArgs &a, bool vec, int G, cudaStream_t st)
+{
+    return vec ? launch_fx_v<true>(a, G, st) : launch_fx_v<false>(a, G, st);
+}
+
+// A list's length is known to the device only.  A lone warp of the lane kernel
+// takes as long as a full one, so up to the length whose waves of the group kernel
+// (with the G that is best for a matrix per SM) take that long, the group kernel
+// has the list, else the lane kernel; the other launch returns at once.  One matrix
+// that falls back from FP32+refine, the lane kernel alone -> this, ms added: n=16 x
+// 524,288 6.6 -> 1.0, n=32 x 65,536 42.3 -> 4.0, n=64 x 8,192 68.5 -> 16.0; a list
+// of 8,192 at n=32 51.3 -> 51.4.
 cudaError_t launch_fx(const FxArgs &a, bool vec, cudaStream_t st)
 {
     if (a.g.N <= 0) return cudaSuccess;
-    if (!fx_order(a.g.n)) return cudaErrorInvalidValue;
-    const FxChoice c = fx_choose(a.g.n, a.g.N, vec);
-    if (c.lanes) return launch_fx_lanes(a, vec, c.G, st);
-    return vec ? launch_fx_v<true>(a, c.G, st) : launch_fx_v<false>(a, c.G, st);
+    const int n = a.g.n;
+    if (!fx_order(n)) return cudaErrorInvalidValue;
+    FxChoice c = fx_choose(n, a.g.N, vec);
+    FxArgs f = a;
+    f.list_above = 0;
+    f.list_upto = a.g.N;
+    if (a.list && c.lanes && !fx_forced(c)) {
+        const int G = fx_best_group(n, fx_sms(), vec);
+        const long long wave = G ? fx_group_wave(n, G, vec) : 0;
+        const double lone = fx_lane_ms(n, 0, c.G == 1 ? 0 : c.G == 2 ? 1 : c.G == 4 ? 2 : 3, vec);
+        if (wave) f.list_upto = wave * std::max(1LL, (long long)(lone / fx_group_ms(n, wave, G, vec)));
+        if (wave) {
+            const cudaError_t e = launch_fx_group(f, vec, G, st);
+            if (e != cudaSuccess || f.list_upto >= a.g.N) return e;
+            f.list_above = f.list_upto;
+            f.list_upto = a.g.N;
+        }
+    }
+    return c.lanes ? launch_fx_lanes(f, vec, c.G, st) : launch_fx_group(f, vec, c.G, st);
 }
 
 template <int G> static void load_fx_g()

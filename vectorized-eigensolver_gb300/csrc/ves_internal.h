@@ -105,6 +105,7 @@ struct FxArgs {
     int *status, *sweeps;                 // nullable
     int max_its, vnorm;
     const int *list, *list_count;  // nullable: the matrices to solve
+    long long list_above, list_upto;  // a launch's range of list lengths: (above, upto] (launch_fx sets them)
     int status_or;                 // bits added to every solved matrix's status
     int *out_list, *out_count;  // out_count: the list's length, then the lane kernel's count of groups taken
     void *ws;         // lane kernel: workspace of lane_blocks x 4 warp slots (fused_workspace_bytes)
