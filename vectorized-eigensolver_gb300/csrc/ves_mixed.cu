@@ -1211,10 +1211,16 @@ __global__ void __launch_bounds__(256) refine_mat_kernel(const MixedArgs a, cons
     cx<double> lam = up(mk(sT[k + k * ld].x, sT[k + k * ld].y));
     const float xkk = sD[k + k * ld].x;
     int f = 0;  // v's scale once it is in fixed point
-    const double tol2 = a.tol * a.tol;
+    // The products that the fixed-point residual leaves out are random: along r they
+    // add up to 2^-59.6 sqrt(2 n) of 2^(eA + f) <= 2^2.5 ||A|| ||v|| (one standard
+    // deviation).  Six of them, 0.45% of the default tolerance at n=16, are kept from
+    // the limit, so that no pair above it is accepted: without them the largest of 16.8
+    // million accepted residuals was 5.004e-14 for a tolerance of 5e-14 (n=16 x
+    // 1,048,576; now 4.868e-14).
+    const double tolr = a.tol - fmin(0x1p-54 * (double)fsqrt<float>((float)n), 0.5 * a.tol), tol2 = tolr * tolr;
     // eigenvalue acceptance: the Newton correction from a certified residual
     // estimates the eigenvalue's remaining error; it must be <= 4 tol ||A||_F
-    const float etol2 = (float)(16.0 * tol2);
+    const float etol2 = (float)(16.0 * a.tol * a.tol);
     int n_res64 = 0, n_corr = 0, n_ff = 0;  // work counters: accepting / float-float residuals, FP32 corrections
     const int ff_steps = a.max_steps >= 2 ? a.ff_steps : 1;  // steps whose residual is float-float (see refine_tile)
     for (int step = 0; step <= a.max_steps; ++step) {
@@ -1366,7 +1372,7 @@ __global__ void __launch_bounds__(256) refine_mat_kernel(const MixedArgs a, cons
                     const float br = r.x * 0x1p40f, bi = r.y * 0x1p40f;
                     rn2 = fmaf(bi, bi, fmaf(br, br, rn2));
                 }
-                // (FP32 sums of squares, good to 2^-17: the margin keeps them from accepting more than FP64 would)
+                // (FP32 sums of squares, good to 2^-17)
                 certified = (double)rn2 * 1.0001 <= tol2 * (double)nA2 * pow2d(80 - 2 * eA) * (double)vn2;
             }
             if (!certified && step == a.max_steps) { fail = true; act = false; }
