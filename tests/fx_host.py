@@ -8,20 +8,19 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "vectorized-eigensolver_gb300", "csrc")
-_lib = None
+_libs = {}
 
 
-def lib():
-    global _lib
-    if _lib is None:
+def lib(src="fx_host.cpp"):
+    if src not in _libs:
         with tempfile.TemporaryDirectory() as d:
             so = os.path.join(d, "fx_host.so")
             # no contraction, as in the device code's written-out fma: the same bits in every form
             subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-ffp-contract=off", "-fno-strict-aliasing", "-shared", "-fPIC",
-                            "-I" + os.path.join(HERE, "host"), "-I" + CSRC, os.path.join(HERE, "host", "fx_host.cpp"), "-o", so],
+                            "-I" + os.path.join(HERE, "host"), "-I" + CSRC, os.path.join(HERE, "host", src), "-o", so],
                            check=True)
-            _lib = ctypes.CDLL(so)
-    return _lib
+            _libs[src] = ctypes.CDLL(so)
+    return _libs[src]
 
 
 def solve(A, form="l1", vec=True, order=0):

@@ -153,8 +153,13 @@ template <> struct lim<float> {
 // and every vector accessor 1 <= i <= kMaxVecIndex; an index outside is
 // counted in this translation unit's device counter and the access goes to
 // the first element instead, so the kernel runs to its end and nothing is
-// read or written out of bounds.  ves_bounds_violations() sums the counters
-// of all translation units.  In the normal build the checks compile away.
+// read or written out of bounds.  Loops that walk a matrix by pointer check
+// the last element that they reach before they start (VES_CHECK_SPAN: the
+// count of their vectors becomes 0), 0-based coordinates in shared memory go
+// through VES_CHECK_LT, and kernels with dynamic shared memory check that
+// their layout ends inside it (VES_CHECK_SMEM).  ves_bounds_violations() sums
+// the counters of all translation units.  In the normal build the checks
+// compile away.
 // ---------------------------------------------------------------------------
 #ifdef VES_BOUNDS_CHECK
 void register_bounds_counter(unsigned long long (*read)(), void (*reset)());
@@ -185,9 +190,33 @@ const BoundsCounterRegistration g_bounds_registration;
     do {                                                                        \
         if ((i) < 1 || (i) > kMaxVecIndex) { bounds_hit(); (i) = 1; }          \
     } while (0)
+#define VES_CHECK_LT(i, n)                                                      \
+    do {                                                                        \
+        if ((i) < 0 || (i) >= (n)) { bounds_hit(); (i) = 0; }                  \
+    } while (0)
+// elements a .. a + reach of the storage of matrix M
+#define VES_CHECK_SPAN(M, a, reach, count)                                      \
+    do {                                                                        \
+        if ((count) > 0 && !(M).holds(a, reach)) { bounds_hit(); (count) = 0; } \
+    } while (0)
+__device__ __forceinline__ unsigned dynamic_smem_bytes()
+{
+    unsigned v = 0;
+#ifdef __CUDA_ARCH__
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(v));
+#endif
+    return v;
+}
+#define VES_CHECK_SMEM(base, end)                                               \
+    do {                                                                        \
+        if ((const char *)(end) - (const char *)(base) > (long long)dynamic_smem_bytes()) { bounds_hit(); return; } \
+    } while (0)
 #else
 #define VES_CHECK_IJ(i, j, n) do { } while (0)
 #define VES_CHECK_I(i) do { } while (0)
+#define VES_CHECK_LT(i, n) do { } while (0)
+#define VES_CHECK_SPAN(M, a, reach, count) do { } while (0)
+#define VES_CHECK_SMEM(base, end) do { } while (0)
 #endif
 constexpr int kMaxVecIndex = 128;  // vectors hold at most 2 n entries, n <= 64
 

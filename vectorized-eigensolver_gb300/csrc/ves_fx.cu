@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(FxShape<G>::threads) fx_kernel(const FxArgs a)
     const int lda = fx_lda(n);
     const FxMat<1> H{sm, lda, n}, Z{sm + (kVec ? n * lda : 0), lda, n};
     const FxVec<1> U{sm + (kVec ? 2 : 1) * n * lda};
+    VES_CHECK_SMEM(fxsm, fxsm + M * fx_slot(n, G, kVec));
     const long long Nw = fx_count(a);
     for (long long base = (long long)blockIdx.x * M; base < Nw; base += (long long)gridDim.x * M) {
         const long long w = base + (G < 32 ? threadIdx.x / G : 0);

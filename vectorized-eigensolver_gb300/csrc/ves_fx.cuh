@@ -132,6 +132,10 @@ template <int ST> struct FxMat {
         VES_CHECK_IJ(i, j, n);
         return p + ((i - 1) + (j - 1) * lda) * ST;
     }
+    __device__ __forceinline__ bool holds(const longlong2 *a, long long reach) const
+    {
+        return a >= p && reach >= 0 && (a - p) + reach < (long long)lda * n * ST;
+    }
     __device__ __forceinline__ cx64 ld(int i, int j) const { const longlong2 v = *at(i, j); return {v.x, v.y}; }
     __device__ __forceinline__ void st(int i, int j, cx64 v) const { *at(i, j) = make_longlong2(v.r, v.i); }
     __device__ __forceinline__ cx<double> ldd(int i, int j) const
@@ -630,13 +634,15 @@ __device__ __noinline__ void fx_reflect(longlong2 *a, const int step, const int 
         p = p1;
     }
 }
-// vectors gl, gl + G, ... of count, kFxReflect at a time
+// vectors gl, gl + G, ... of count in A, kFxReflect at a time; u in H
 constexpr int kFxReflect = 4;
 template <int G, int ST>
-__device__ __forceinline__ void fx_reflect_all(const int gl, longlong2 *a, const int step, const int blk,
-                                               const int count, const longlong2 *u, const cx64 u1, const int m,
-                                               const bool cj)
+__device__ __forceinline__ void fx_reflect_all(const int gl, const FxMat<ST> &A, longlong2 *a, const int step, const int blk,
+                                               int count, const FxMat<ST> &H, const longlong2 *u, const cx64 u1,
+                                               const int m, const bool cj)
 {
+    VES_CHECK_SPAN(A, a, (long long)(count - 1) * blk + (m - 1) * step, count);
+    VES_CHECK_SPAN(H, u, (long long)(m - 2) * ST, count);
     constexpr int NB = G > 8 ? 1 : kFxReflect;  // larger groups have one or two vectors per lane
     int v = gl;
     if (NB > 1)
@@ -705,9 +711,9 @@ __device__ __forceinline__ void fx_reduce(const GR &gr, const int n, const FxMat
         ok = ok && fx_abs1(beta) >= kFxMinSub;
         if (!gr.any(ok)) return;
         const longlong2 *u = H.at(i + 2, i);
-        fx_reflect_all<G, ST>(gr.gl, H.at(1, i + 1), cs, rs, n, u, u1, n - i, true);  // rows of A(:, i+1:n)
+        fx_reflect_all<G, ST>(gr.gl, H, H.at(1, i + 1), cs, rs, n, H, u, u1, n - i, true);  // rows of A(:, i+1:n)
         gr.sync();
-        fx_reflect_all<G, ST>(gr.gl, H.at(i + 1, i + 1), rs, cs, n - i, u, u1, n - i, false);  // columns of A(i+1:n, i+1:n)
+        fx_reflect_all<G, ST>(gr.gl, H, H.at(i + 1, i + 1), rs, cs, n - i, H, u, u1, n - i, false);  // columns of A(i+1:n, i+1:n)
         gr.sync();
     }
 }
@@ -721,7 +727,7 @@ __device__ __forceinline__ void fx_form_q(const GR &gr, const int n, const FxMat
         for (int r = 1; r <= n; ++r) Z.st(r, c, {r == c ? 1LL << 61 : 0, 0});
     gr.sync();
     for (int i = n - 2; i >= 1; --i) {
-        fx_reflect_all<G, ST>(gr.gl, Z.at(i + 1, i + 1), ST, Z.lda * ST, n - i, H.at(i + 2, i), U.ld(i), n - i, false);
+        fx_reflect_all<G, ST>(gr.gl, Z, Z.at(i + 1, i + 1), ST, Z.lda * ST, n - i, H, H.at(i + 2, i), U.ld(i), n - i, false);
         gr.sync();
     }
 }
@@ -969,16 +975,22 @@ struct FxChunk {
     i64 *si;
     __device__ __forceinline__ void put(int k, const FxRot &q) const
     {
+        VES_CHECK_LT(k, kFxChunk);
         cs[k * 32] = make_longlong2(q.c, q.sr);
         si[k * 32] = q.si;
     }
     __device__ __forceinline__ FxCoef get(int k) const
     {
+        VES_CHECK_LT(k, kFxChunk);
         const longlong2 a = cs[k * 32];
         return FxCoef(a.x, a.y, si[k * 32]);
     }
     // G > 1: entry of the lane's row t of the chunk in the column that the next rotation turns
-    template <int G> __device__ __forceinline__ longlong2 *row(int t) const { return cs + (FxChunkOf<G>::k + t) * 32; }
+    template <int G> __device__ __forceinline__ longlong2 *row(int t) const
+    {
+        VES_CHECK_LT(t, FxChunkOf<G>::k / G);
+        return cs + (FxChunkOf<G>::k + t) * 32;
+    }
 };
 
 // Apply ns rotations (c, s at cs[k * 32], si[k * 32]) to NB chains of entries:
@@ -1031,10 +1043,11 @@ __device__ __noinline__ void fx_stream(longlong2 *p, const int step, const int b
 #pragma unroll
     for (int b = 0; b < NB; ++b) p[b * blk] = make_longlong2(x[b].r, x[b].i);
 }
-template <int G>
-__device__ __forceinline__ void fx_stream_all(const int gl, longlong2 *p, const int step, const int blk, const int count,
-                                              const FxChunk &ch, const int ns, const bool col)
+template <int G, int ST>
+__device__ __forceinline__ void fx_stream_all(const int gl, const FxMat<ST> &A, longlong2 *p, const int step, const int blk,
+                                              int count, const FxChunk &ch, const int ns, const bool col)
 {
+    VES_CHECK_SPAN(A, p, (long long)(count - 1) * blk + (long long)ns * step, count);
     int b = G == 1 ? 0 : gl;  // chains gl, gl + G, ... of count
     for (; b + kFxStream * G <= count + G - 1; b += kFxStream * G) {
         const bool more = b + 2 * kFxStream * G <= count + G - 1;
@@ -1107,7 +1120,10 @@ __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, co
                 }
                 ch.put(K - Kc, R);
                 const FxCoef C(R), CC = C.columns();
-                for (int q = 0; q < K - Kc; ++q) {
+                int turned = K - Kc;
+                VES_CHECK_SPAN(H, pc, (K + 1 - Kc) * rs, turned);
+                VES_CHECK_SPAN(H, pl, (K - Kc) * rs, turned);
+                for (int q = 0; q < turned; ++q) {
                     cx64 y = {v.x, v.y};
                     v = pc[2 * rs];
                     fx_pair(x, y, ch.get(q));
@@ -1160,10 +1176,10 @@ __device__ __forceinline__ void fx_qr_lane(const int group_lane, const int n, co
             }
             // rows above the chunk
             const int r0 = kVec ? 1 : Kmin;
-            if (Kc > r0) fx_stream_all<G>(gl, H.at(r0, Kc), cs, rs, Kc - r0, ch, ns, true);
-            if (kVec) fx_stream_all<G>(gl, Z.at(1, Kc), cs, rs, n, ch, ns, true);
+            if (Kc > r0) fx_stream_all<G>(gl, H, H.at(r0, Kc), cs, rs, Kc - r0, ch, ns, true);
+            if (kVec) fx_stream_all<G>(gl, Z, Z.at(1, Kc), cs, rs, n, ch, ns, true);
             const int je = kVec ? n : Kmax + 1;
-            if (je > Ke + 1) fx_stream_all<G>(gl, H.at(Kc, Ke + 2), rs, cs, je - Ke - 1, ch, ns, false);
+            if (je > Ke + 1) fx_stream_all<G>(gl, H, H.at(Kc, Ke + 2), rs, cs, je - Ke - 1, ch, ns, false);
             if (G > 1) __syncwarp();
         }
     }

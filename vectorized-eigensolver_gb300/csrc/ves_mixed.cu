@@ -1136,7 +1136,8 @@ __device__ __forceinline__ void mat_rows(const int n, const int ld, const float2
     const float2 *p[TR];
 #pragma unroll
     for (int t = 0; t < TR; ++t) {
-        const int r = min(r0 + 4 * t, n - 1);
+        int r = min(r0 + 4 * t, n - 1);
+        VES_CHECK_LT(r, n);
         p[t] = L + (kAdj ? r * ld : r);
         s[t] = mk(0.f, 0.f);
     }
@@ -1180,6 +1181,7 @@ __global__ void __launch_bounds__(256) refine_mat_kernel(const MixedArgs a, cons
     float2 *const sR = reinterpret_cast<float2 *>(sA + refine_a_units(n, TR));
     float2 *const sT = sR + ld * n, *const sZ = sT + ld * n;
     VEntry *const V = reinterpret_cast<VEntry *>(sV);
+    VES_CHECK_SMEM(rsm, sZ + ld * n);
     const float2 *const bT = buf + m * mat_elems(n), *const bX = bT + 2 * nn, *const bA = bT + 3 * nn + n;
     const float nA2 = bT[3 * nn].x;
     const float nb = fmaf(nA2, 1.002f, 1e-37f);  // >= ||A||_F^2, also where squares underflowed
@@ -1292,7 +1294,10 @@ __global__ void __launch_bounds__(256) refine_mat_kernel(const MixedArgs a, cons
                 const int4 L = sL[cc];
                 int ri[TR];  // the lane's rows in the block
 #pragma unroll
-                for (int t = 0; t < TR; ++t) ri[t] = min(lr + 4 * t, rows - 1);
+                for (int t = 0; t < TR; ++t) {
+                    ri[t] = min(lr + 4 * t, rows - 1);
+                    VES_CHECK_LT(ri[t], n - rb * RB);
+                }
                 float or_[TR], oi[TR];
                 if (ff) {
                     const float lhr = __int_as_float(L.x), lhi = __int_as_float(L.y);
