@@ -6,7 +6,7 @@ import pytest
 import oracle
 import ves
 from gpu_util import dev, run_fused
-from parity import match_eigs
+from parity import match_eigs, residuals
 from test_fx_host import bordered
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +76,77 @@ def test_weak_block_beside_strong_row_keeps_relative_accuracy(n, first):
     flat = A.transpose(0, 2, 1).ravel()
     ves.eigensolve_varsize(N, n, dev(np.full(N, n, np.int32)), dev(flat.real.copy()), dev(flat.imag.copy()), *E, *V)
     check_small((E[0].cpu().numpy() + 1j * E[1].cpu().numpy()).reshape(N, n), norms, want)
+
+
+# lengths on both sides of the one at which a list goes from a matrix per warp (two rows and
+# columns per lane for n > 32) to one per lane
+@pytest.mark.parametrize("n,N", [(3, 2600), (10, 5000), (24, 4400), (32, 3800), (40, 2600), (64, 1900)])
+def test_fp64_list_kernels_same_bits(n, N):
+    rng = np.random.default_rng(1000 + n)
+    A = cgauss(rng, (N, n, n))
+    A[:, n // 2:, :n // 2] = 0
+    A[3] = np.triu(A[3])  # the reflectors' trivial branch
+    long_list = run_fused(A, N, want_T=True, vnorm=1)
+    assert (long_list["status"] == 0).all()
+    for s in (0, N - 60):
+        short = run_fused(A[s:s + 60], 60, want_T=True, vnorm=1)
+        for key, want in short.items():
+            assert np.array_equal(long_list[key][s:s + 60], want), key
+    # (the oracle, like the reference, divides by a subdiagonal that is exactly zero)
+    _, err, _ = match_eigs(long_list["E"][:60], np.linalg.eigvals(A[:60]))
+    assert (err / np.linalg.norm(A[:60], axis=(1, 2))).max() <= 1e-12
+
+
+# orders whose Newton step keeps its scratch beside the slot, not in Z, and the next one
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 6])
+@pytest.mark.parametrize("polish", [0, 4])
+def test_shifts_of_small_orders(n, polish, monkeypatch):
+    import torch
+    monkeypatch.setenv("VES_POLISH_FP64_STEP", "2")
+    rng = np.random.default_rng(1100 + n)
+    N, tc = 96, 8
+    A = cgauss(rng, (N, n, n))
+    A[::9, n // 2:, :n // 2] = 0  # solved in FP64
+    ref = np.linalg.eigvals(A)
+    planes = [dev(x) for x in ves.soa_from_complex(A, tc)]
+    S = [dev(x) for x in ves.soa_vec_from_complex(ref + 1e-3 * cgauss(rng, ref.shape), tc)]
+    E = [torch.empty(N * n, dtype=torch.float64, device="cuda") for _ in range(2)]
+    V = [torch.empty_like(planes[0]) for _ in range(2)]
+    st = torch.full((N,), -1, dtype=torch.int32, device="cuda")
+    ves.eigensolve_shifts(n, N // tc, tc, *planes, *E, *V, *S, status=st, options=ves.default_options(shift_polish=polish))
+    torch.cuda.synchronize()
+    got = ves.complex_vec_from_soa(E[0].cpu().numpy(), E[1].cpu().numpy(), n, tc)
+    vec = ves.complex_from_soa(V[0].cpu().numpy(), V[1].cpu().numpy(), n, tc)
+    assert ((st.cpu().numpy() & ~ves.VES_STATUS_SHIFT_FALLBACK) == 0).all()
+    _, err, _ = match_eigs(got, ref)
+    assert (err / np.linalg.norm(A, axis=(1, 2))).max() <= 1e-12
+    assert residuals(A, got, vec).max() <= 1e-13
+
+
+def test_noalloc_beyond_one_slice():
+    """More matrices than the allocation-free call lists at once (2^20): the slices after the
+    first start inside the batch; refused matrices in each."""
+    import ctypes
+    import torch
+    n, N = 3, (1 << 20) + 37
+    g = torch.Generator(device="cuda").manual_seed(3)
+    A = [torch.randn(n, n, N, generator=g, dtype=torch.float64, device="cuda") for _ in range(2)]  # [column][row][matrix]
+    for p in A:
+        p[0, 1:, ::5] = 0  # first column: reducible
+        p[0, 1:, N - 1] = 0
+    planes = [p.view(-1) for p in A]
+    outs = []
+    for noalloc in (False, True):
+        o = [torch.full((k,), float("nan"), dtype=torch.float64, device="cuda") for k in (N * n, N * n, N * n * n, N * n * n)]
+        st = torch.full((N,), -1, dtype=torch.int32, device="cuda")
+        if noalloc:
+            ptr = [ctypes.c_void_p(t.data_ptr()) for t in planes + o + [st]]
+            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+            assert ves.lib().ves_eigensolve_noalloc(n, 1, N, *ptr, stream) == 0, ves.last_error()
+        else:
+            ves.eigensolve(n, 1, N, *planes, *o, status=st)
+        torch.cuda.synchronize()
+        assert int(st.abs().max()) == 0
+        outs.append(o)
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
