@@ -24,7 +24,8 @@ roofline  the solver applies its unitary transformations in 64-bit fixed point
         on the integer pipe: achieved = IMAD.WIDE operations per launch (36 for
         a rotated pair of entries, 12 for a complex multiply-add: 36 n^3 +
         36 s n^3 per matrix, s = device-counted QR sweeps per eigenvalue) /
-        launch time, against 26 per clock and SM at the maximum SM clock.
+        launch time, against the rate measured on this GPU in this run.  The 36
+        and 12 are this implementation's instructions, not a lower bound.
         `fp64` beside it is the same work as 24 n^3 + 20 s n^3 flops against
         the FP64 FMA rate measured on this GPU in this run: the rate that FP64
         arithmetic could reach at most, so it may exceed 1.  The HBM view
@@ -99,11 +100,6 @@ def log(*a):
 def r4(x):
     """A number rounded to 4 significant digits (keeps the JSON line short)."""
     return float("%.4g" % x) if isinstance(x, float) else x
-
-
-# IMAD.WIDE (32 x 32 + 64 bit) operations per clock and SM, measured on a GB300
-# with a chain-free loop of them
-IMAD_PER_CLK_SM = 26.0
 
 
 def imad_ops(n, sweeps_total, matrices):
@@ -679,8 +675,7 @@ def run_gpu_arm(args, d):
         pass
     PEAKS.update(fp64=peak_fp64, fp32=ves.fp32_fma_rate(stream),
                  bf16=peaks_file.get("bf16_tflops", 1900.0) * 1e12, hbm=peaks_file.get("hbm_gbs", 6800.0) * 1e9,
-                 imad=IMAD_PER_CLK_SM * torch.cuda.get_device_properties(d.local).multi_processor_count
-                 * peaks_file.get("sm_max_mhz", 2070.0) * 1e6)
+                 imad=ves.imad_wide_rate(stream))
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize()
@@ -779,7 +774,8 @@ def run_gpu_arm(args, d):
                    "sweeps_per_eigenvalue": s_mean},
         "roofline": {"bound": "imad", "achieved": achieved / 1e12, "peak": PEAKS["imad"] / 1e12,
                      "unit": "T IMAD.WIDE/s", "frac": achieved / PEAKS["imad"], "traffic": traffic,
-                     "peak_source": "26 IMAD.WIDE per clock and SM, measured once on a GB300, at the maximum SM clock",
+                     "peak_source": "IMAD.WIDE rate measured in this run (ves_imad_wide_rate); 36 per rotated pair and "
+                                    "12 per complex multiply-add are this implementation's counts",
                      "flops_per_matrix": flops_per_matrix(n, s_mean),
                      "fp64": {"achieved": flops / 1e12, "peak": peak_fp64 / 1e12, "unit": "TFLOP/s",
                               "frac": flops / peak_fp64,

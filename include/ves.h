@@ -356,6 +356,9 @@ int ves_fp64_fma_rate(double *flops_per_s, void *stream);
 /* The same for FP32 FMAs: the roofline denominator of the FP32 stages of the
  * FP32 + refinement form and of the learned-shift polish. */
 int ves_fp32_fma_rate(double *flops_per_s, void *stream);
+/* The same for 32 x 32 + 64-bit integer multiply-adds, in operations per second:
+ * the roofline denominator of the fixed-point transformations. */
+int ves_imad_wide_rate(double *ops_per_s, void *stream);
 
 /* Allocation-free variant of ves_eigensolve (FP64, reference eigenvector
  * scaling, no Schur-form or sweep output).  No counterpart in the reference.

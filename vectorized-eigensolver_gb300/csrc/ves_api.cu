@@ -1199,6 +1199,13 @@ int ves_fp32_fma_rate(double *flops_per_s, void *stream)
     return native(cuda_ok(ves::fp32_fma_rate(flops_per_s, (cudaStream_t)stream), "fp32 probe"));
 }
 
+int ves_imad_wide_rate(double *ops_per_s, void *stream)
+{
+    begin_call();
+    if (!ops_per_s) { set_error("null pointer"); return VES_ERR_ARG; }
+    return native(cuda_ok(ves::imad_wide_rate(ops_per_s, (cudaStream_t)stream), "integer probe"));
+}
+
 int ves_bounds_violations(unsigned long long *count, int reset)
 {
     if (!count) { set_error("ves_bounds_violations: null pointer"); return VES_ERR_ARG; }

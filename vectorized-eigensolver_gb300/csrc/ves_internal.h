@@ -220,6 +220,7 @@ void set_error_message(const char *msg);
 // Measured FP64 / FP32 FMA throughput of this GPU (2 flops per FMA).
 cudaError_t fp64_fma_rate(double *flops_per_s, cudaStream_t st);
 cudaError_t fp32_fma_rate(double *flops_per_s, cudaStream_t st);
+cudaError_t imad_wide_rate(double *ops_per_s, cudaStream_t st);
 
 // Work counters of ves_options.work_counts (device, accumulated with atomics).
 enum { WORK_RES64 = 0, WORK_CORR32 = 1, WORK_RESFF = 2, WORK_POLISH = 3 };

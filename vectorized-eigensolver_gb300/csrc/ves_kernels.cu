@@ -939,10 +939,27 @@ cudaError_t launch_backsubs(Geom g, const double *rT, const double *iT, double *
     return cudaGetLastError();
 }
 
+// Eight chains per thread, each step's low word an operand of the next.
+__global__ void imad_probe_kernel(long long *out, const int iters, const long long b, const long long)
+{
+    long long x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = (long long)threadIdx.x * 77 + i;
+#pragma unroll 4
+    for (int it = 0; it < iters; ++it)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(x[i]) : "r"((int)x[i]), "r"((int)b));
+    long long s = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += x[i];
+    out[(long long)blockIdx.x * blockDim.x + threadIdx.x] = s;
+}
+
+// Instructions per second and lane of a probe kernel with eight chains per thread.
 // threads per SM: 8 warps keep the FP64 pipe full; the FP32 pipe (about 58x
-// the FP64 rate) needs 32 warps of independent chains
+// the FP64 rate) and the integer multiplier need 32 warps of independent chains
 template <class R>
-cudaError_t fma_rate(double *flops_per_s, cudaStream_t st, int threads, int iters)
+cudaError_t probe_rate(double *per_s, cudaStream_t st, int threads, int iters, void (*probe)(R *, int, R, R), R b, R c)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -953,11 +970,10 @@ cudaError_t fma_rate(double *flops_per_s, cudaStream_t st, int threads, int iter
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    const R b = R(1.0000001), c = R(1e-9);
-    fma_probe_kernel<R><<<sms, threads, 0, st>>>(out, iters, b, c);  // warm-up
+    probe<<<sms, threads, 0, st>>>(out, iters, b, c);  // warm-up
     cudaEventRecord(e0, st);
     const int reps = 5;
-    for (int r = 0; r < reps; ++r) fma_probe_kernel<R><<<sms, threads, 0, st>>>(out, iters, b, c);
+    for (int r = 0; r < reps; ++r) probe<<<sms, threads, 0, st>>>(out, iters, b, c);
     cudaEventRecord(e1, st);
     e = cudaEventSynchronize(e1);
     float ms = 0.f;
@@ -966,12 +982,22 @@ cudaError_t fma_rate(double *flops_per_s, cudaStream_t st, int threads, int iter
     cudaEventDestroy(e1);
     cudaFreeAsync(out, st);
     if (e == cudaSuccess) e = cudaGetLastError();
-    *flops_per_s = 2.0 * 8.0 * iters * (double)sms * threads * reps / (ms * 1e-3);
+    *per_s = 8.0 * iters * (double)sms * threads * reps / (ms * 1e-3);
     return e;
 }
 
+template <class R> cudaError_t fma_rate(double *flops_per_s, cudaStream_t st, int threads, int iters)
+{
+    const cudaError_t e = probe_rate<R>(flops_per_s, st, threads, iters, fma_probe_kernel<R>, R(1.0000001), R(1e-9));
+    *flops_per_s *= 2.0;
+    return e;
+}
 cudaError_t fp64_fma_rate(double *flops_per_s, cudaStream_t st) { return fma_rate<double>(flops_per_s, st, 256, 4096); }
 cudaError_t fp32_fma_rate(double *flops_per_s, cudaStream_t st) { return fma_rate<float>(flops_per_s, st, 1024, 16384); }
+cudaError_t imad_wide_rate(double *ops_per_s, cudaStream_t st)
+{
+    return probe_rate<long long>(ops_per_s, st, 1024, 8192, imad_probe_kernel, 12345, 0);
+}
 
 void load_fused_kernels()
 {
@@ -989,6 +1015,7 @@ void load_fused_kernels()
     load_kernel(backsubs_kernel);
     load_kernel(fma_probe_kernel<double>);
     load_kernel(fma_probe_kernel<float>);
+    load_kernel(imad_probe_kernel);
 }
 
 }  // namespace ves

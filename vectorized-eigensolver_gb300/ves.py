@@ -81,6 +81,7 @@ SIGNATURES = {
     "ves_backsubstitution": (_int, [_int, _int, _int, _VP, _VP, _VP, _VP, _VP]),
     "ves_fp64_fma_rate": (_int, [_D, _VP]),
     "ves_fp32_fma_rate": (_int, [_D, _VP]),
+    "ves_imad_wide_rate": (_int, [_D, _VP]),
     "ves_polyroots_workspace_size": (_size, [_int, _int, _int]),
     "ves_eigensolve_varsize_workspace_size": (_size, [ctypes.c_longlong, _int, ctypes.POINTER(Options)]),
     "ves_eigensolve_varsize": (_int, [ctypes.c_longlong, _int, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP,
@@ -544,6 +545,13 @@ def fp32_fma_rate(stream=None):
     """Measured FP32 FMA throughput of the current GPU, flop/s."""
     v = ctypes.c_double(0.0)
     _check(lib().ves_fp32_fma_rate(ctypes.byref(v), _stream_ptr(stream)), "ves_fp32_fma_rate")
+    return v.value
+
+
+def imad_wide_rate(stream=None):
+    """Measured rate of 32 x 32 + 64-bit integer multiply-adds of the current GPU, operations/s."""
+    v = ctypes.c_double(0.0)
+    _check(lib().ves_imad_wide_rate(ctypes.byref(v), _stream_ptr(stream)), "ves_imad_wide_rate")
     return v.value
 
 
