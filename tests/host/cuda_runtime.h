@@ -212,6 +212,7 @@ inline unsigned long long __umul64hi(unsigned long long a, unsigned long long b)
 inline int __clz(int x) { return x ? __builtin_clz(x) : 32; }
 inline int __clzll(long long x) { return x ? __builtin_clzll(x) : 64; }
 inline unsigned __funnelshift_l(unsigned lo, unsigned hi, unsigned s) { return s & 31 ? (hi << (s & 31)) | (lo >> (32 - (s & 31))) : hi; }
+inline int __ffsll(long long x) { return __builtin_ffsll(x); }
 inline int __ffs(int x) { return __builtin_ffs(x); }
 inline double rsqrt(double x) { return 1.0 / sqrt(x); }
 inline float rsqrtf(float x) { return 1.0f / sqrtf(x); }

@@ -86,3 +86,25 @@ def test_ordinary_matrices_stay_in_fixed_point(n):
     chain[0] = np.diag(rng.uniform(-1, 1, n)) + np.diag(np.ones(n - 1), 1) + np.diag(np.ones(n - 1), -1)
     for B in (A, H, A.real + 0j, phase, bordered(rng, N, n, 1 / 4, False), chain):
         assert fx_host.solve(B)["ok"].all()
+
+
+@pytest.mark.parametrize("n", [3, 5, 16, 33, 64])
+@pytest.mark.parametrize("form", ["l1", "l2", "g8"])
+def test_matrices_not_connected_from_the_first_index(n, form):
+    """Diagonal, triangular and block-triangular matrices are refused; those whose nonzeros
+    lead from index 1 to all others, in one step or in n - 1, are not."""
+    rng = np.random.default_rng(70 + n)
+    A = rng.standard_normal((1, n, n)) + 1j * rng.standard_normal((1, n, n))
+    p = n // 2
+    refused = [A * np.eye(n), np.triu(A), A.copy(), A.copy()]
+    refused[2][:, p:, :p] = 0
+    refused[3][:, n - 1, :n - 1] = 0
+    out = fx_host.solve(np.concatenate(refused), form)
+    assert not out["error"] and not out["ok"].any()
+    cycle = np.zeros((1, n, n), complex)
+    cycle[0, np.arange(n), (np.arange(n) + 1) % n] = 1  # the last index is reached first
+    chain = np.triu(np.tril(A, 1), -1)
+    arrow = A * ((np.arange(n)[:, None] == 0) | (np.arange(n) == 0) | np.eye(n, dtype=bool))
+    out = fx_host.solve(np.concatenate([A, A.conj().transpose(0, 2, 1), chain, cycle + 0.1 * np.eye(n), arrow]), form)
+    assert not out["error"]
+    assert out["ok"].all()

@@ -475,13 +475,53 @@ __device__ __forceinline__ int fx_blocks(const int n, const int r, const int mt)
 }
 constexpr int kFxBlocks = 7, kFxBlocksInA = 8;
 
+// Functions below that are not inlined keep one copy of their code: the lane
+// kernel's warps run out of step, and with everything inlined its code did not
+// fit the instruction caches (n=16: 4.0 M/s on one wave, 2.6 M/s on eight).
+// ST tells the memory space: 1 = shared, 32 = global.
+template <int ST> __device__ __forceinline__ void fx_assume_space(const void *p)
+{
+#ifdef __CUDA_ARCH__
+    if (ST == 1) __builtin_assume(__isShared(p));
+    else __builtin_assume(__isGlobal(p));
+#endif
+}
+
+// Does the graph of A's nonzero entries lead from index 1 to every other?  Where it
+// does not (diagonal, triangular, block triangular matrices) the reduction meets a
+// zero subdiagonal, at which the matrix would be refused after half the work: n=24 x
+// 30,720 block-triangular, eigenvalues only, 23.9 -> 21.2 ms (as in FP64 alone), n=16
+// x 100,000 50.0 -> 47.8 (46.8).
+// One column's entries for a full matrix.
+template <class GR, int ST>
+__device__ __forceinline__ bool fx_connected(const GR &gr, const int n, const FxMat<ST> &H)
+{
+    const i64 all = (i64)(~0ULL >> (64 - n));
+    i64 reached = 1, done = 0;
+    for (;;) {
+        const i64 todo = reached == all ? 0 : reached & ~done;
+        if (!gr.any(todo != 0)) break;
+        const int r = todo ? __ffsll(todo) : 1;
+        i64 to = 0;
+        for (int i = gr.rl + 1; i <= n; i += GR::RG) {
+            const cx64 x = H.ld(i, r);
+            to |= (i64)((x.r | x.i) != 0) << (i - 1);
+        }
+        reached |= gr.orr(to);
+        done |= 1LL << (r - 1);
+    }
+    return reached == all;
+}
+
 // Load A (element e of the column-major matrix at e * s) into H as integers.
 // Returns false for a matrix that is left to the FP64 kernels; unit = 2^(e-61);
-// blocks: fx_blocks of A.
+// blocks: fx_blocks of A.  (Inlined, with fx_connected in it, the lane kernel took
+// 271 to 274 ms for n=16 x 1,048,576 instead of 266.)
 template <int G, class GR, int ST>
-__device__ __forceinline__ bool fx_load(const GR &gr, const int n, const FxMat<ST> &H, const bool valid,
-                                        const double *rA, const double *iA, const long long s, double &unit, int &blocks)
+__device__ __noinline__ bool fx_load(const GR gr, const int n, const FxMat<ST> H, const bool valid, const double *rA,
+                                     const double *iA, const long long s, double &unit, int &blocks)
 {
+    fx_assume_space<ST>(H.p);
     unit = 1.0;
     int emax = 0;
     FxIndex i0(gr.gl, n);
@@ -543,20 +583,9 @@ __device__ __forceinline__ bool fx_load(const GR &gr, const int n, const FxMat<S
         large |= fx_blocks(n, r, mt);
     }
     blocks = (int)gr.orr(large);
+    ok = fx_connected(gr, n, H) && ok;
     // A(2:n, 2:n) is only rotated within itself: that it is small is known already
     return gr.all(ok && (blocks & kFxBlocksInA));
-}
-
-// Functions below that are not inlined keep one copy of their code: the lane
-// kernel's warps run out of step, and with everything inlined its code did not
-// fit the instruction caches (n=16: 4.0 M/s on one wave, 2.6 M/s on eight).
-// ST tells the memory space: 1 = shared, 32 = global.
-template <int ST> __device__ __forceinline__ void fx_assume_space(const void *p)
-{
-#ifdef __CUDA_ARCH__
-    if (ST == 1) __builtin_assume(__isShared(p));
-    else __builtin_assume(__isGlobal(p));
-#endif
 }
 
 // Bring the line of p into L2 (no register is held for it).
