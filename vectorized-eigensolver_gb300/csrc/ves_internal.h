@@ -71,6 +71,7 @@ struct MixedArgs {
     int vnorm;
     int max_steps;  // Newton corrections per eigenpair
     double tol;     // ||r|| <= tol ||A||_F ||v||
+    double tol_fx;  // the same for a fixed-point residual, less its own rounding (set where it is used)
     int *fb_list;   // matrices handed to the FP64 solver
     int *fb_count;
     int *plain_count;  // the FP64 solver's own two counters (nullable), set to zero by the last kernel here

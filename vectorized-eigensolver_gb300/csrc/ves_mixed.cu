@@ -44,6 +44,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 
@@ -1213,13 +1214,7 @@ __global__ void __launch_bounds__(256) refine_mat_kernel(const MixedArgs a, cons
     cx<double> lam = up(mk(sT[k + k * ld].x, sT[k + k * ld].y));
     const float xkk = sD[k + k * ld].x;
     int f = 0;  // v's scale once it is in fixed point
-    // The products that the fixed-point residual leaves out are random: along r they
-    // add up to 2^-59.6 sqrt(2 n) of 2^(eA + f) <= 2^2.5 ||A|| ||v|| (one standard
-    // deviation).  Six of them, 0.45% of the default tolerance at n=16, are kept from
-    // the limit, so that no pair above it is accepted: without them the largest of 16.8
-    // million accepted residuals was 5.004e-14 for a tolerance of 5e-14 (n=16 x
-    // 1,048,576; now 4.868e-14).
-    const double tolr = a.tol - fmin(0x1p-54 * (double)fsqrt<float>((float)n), 0.5 * a.tol), tol2 = tolr * tolr;
+    const double tol2 = a.tol_fx * a.tol_fx;
     // eigenvalue acceptance: the Newton correction from a certified residual
     // estimates the eigenvalue's remaining error; it must be <= 4 tol ||A||_F
     const float etol2 = (float)(16.0 * a.tol * a.tol);
@@ -1750,10 +1745,18 @@ template <int TR> cudaError_t launch_refine_mat(const MixedArgs &a, const MixedB
 {
     const int n = a.g.n, W = n <= 16 ? 1 : n <= 28 ? 2 : n <= 40 ? 4 : 8;
     const size_t smem = refine_smem(n, TR);
+    // The products that the fixed-point residual leaves out are random: along r they
+    // add up to 2^-59.6 sqrt(2 n) of 2^(eA + f) <= 2^2.5 ||A|| ||v|| (one standard
+    // deviation).  Six of them, 0.45% of the default tolerance at n=16, are kept from
+    // the limit, so that no pair above it is accepted: without them the largest of 16.8
+    // million accepted residuals was 5.004e-14 for a tolerance of 5e-14 (n=16 x
+    // 1,048,576; now 4.868e-14).
+    MixedArgs f = a;
+    f.tol_fx = a.tol - std::min(0x1p-54 * std::sqrt((double)n), 0.5 * a.tol);
     const cudaError_t e = cudaFuncSetAttribute(refine_mat_kernel<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)refine_smem(64, 4));
     if (e != cudaSuccess) return e;
-    refine_mat_kernel<TR><<<(unsigned)(a.m_end - a.m_begin), 32 * W, smem, st>>>(a, b.buf, b.flags);
+    refine_mat_kernel<TR><<<(unsigned)(a.m_end - a.m_begin), 32 * W, smem, st>>>(f, b.buf, b.flags);
     return cudaGetLastError();
 }
 
