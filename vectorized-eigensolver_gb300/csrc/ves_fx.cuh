@@ -1,7 +1,7 @@
 // ves_fx.cuh -- the FP64 solver's unitary transformations in 64-bit fixed
 // point on the integer pipe.
 //
-// Why.  GB300 retires 1.8 FP64 FMAs per clock and SM but about 26 32x32+64-bit
+// Why.  GB300 retires 1.9 FP64 FMAs per clock and SM but 25 32x32+64-bit
 // integer multiply-adds (IMAD.WIDE).  The Hessenberg reduction and the QR
 // sweeps only apply unitary transformations, under which no entry of the
 // matrix can grow past ||A||_F, so one scale per matrix is enough and the
@@ -515,13 +515,12 @@ __device__ __forceinline__ bool fx_connected(const GR &gr, const int n, const Fx
 
 // Load A (element e of the column-major matrix at e * s) into H as integers.
 // Returns false for a matrix that is left to the FP64 kernels; unit = 2^(e-61);
-// blocks: fx_blocks of A.  (Inlined, with fx_connected in it, the lane kernel took
-// 271 to 274 ms for n=16 x 1,048,576 instead of 266.)
-template <int G, class GR, int ST>
-__device__ __noinline__ bool fx_load(const GR gr, const int n, const FxMat<ST> H, const bool valid, const double *rA,
-                                     const double *iA, const long long s, double &unit, int &blocks)
+// blocks: fx_blocks of A.
+template <int G, bool kConnected, class GR, int ST>
+__device__ __forceinline__ bool fx_load_inline(const GR &gr, const int n, const FxMat<ST> &H, const bool valid,
+                                               const double *rA, const double *iA, const long long s, double &unit,
+                                               int &blocks)
 {
-    fx_assume_space<ST>(H.p);
     unit = 1.0;
     int emax = 0;
     FxIndex i0(gr.gl, n);
@@ -583,9 +582,21 @@ __device__ __noinline__ bool fx_load(const GR gr, const int n, const FxMat<ST> H
         large |= fx_blocks(n, r, mt);
     }
     blocks = (int)gr.orr(large);
-    ok = fx_connected(gr, n, H) && ok;
+    if (kConnected) ok = fx_connected(gr, n, H) && ok;
     // A(2:n, 2:n) is only rotated within itself: that it is small is known already
     return gr.all(ok && (blocks & kFxBlocksInA));
+}
+// One copy beside the kernel's own code, but for the shift-seeded kernel, which has it
+// inlined and without fx_connected (a reflector refuses those matrices there): its code
+// is the largest, and warps out of step over many waves miss the instruction cache.
+// Whole solves, ms: plain n=16 x 1,048,576 266 (inlined 271 .. 274), shift-seeded n=24 x
+// 1,048,576 622 (as a function 742; over 3.4 waves, 262,144, no different).
+template <int G, class GR, int ST>
+__device__ __noinline__ bool fx_load(const GR gr, const int n, const FxMat<ST> H, const bool valid, const double *rA,
+                                     const double *iA, const long long s, double &unit, int &blocks)
+{
+    fx_assume_space<ST>(H.p);
+    return fx_load_inline<G, true>(gr, n, H, valid, rA, iA, s, unit, blocks);
 }
 
 // Bring the line of p into L2 (no register is held for it).
@@ -1410,7 +1421,9 @@ __device__ __forceinline__ bool fx_solve(const GR &gr, const int n, const FxMat<
 {
     double unit;
     int blocks;
-    bool ok = fx_load<G>(gr, n, H, valid, rA, iA, s, unit, blocks);
+    bool ok;
+    if constexpr (SH::kOn) ok = fx_load_inline<G, false>(gr, n, H, valid, rA, iA, s, unit, blocks);
+    else ok = fx_load<G>(gr, n, H, valid, rA, iA, s, unit, blocks);
     if (gr.any(ok)) fx_reduce<G>(gr, n, H, U, ok);
     if (gr.any(ok)) {
         const bool irreducible = fx_irreducible<G>(gr, n, H, blocks);  // every lane takes part, whatever ok is
