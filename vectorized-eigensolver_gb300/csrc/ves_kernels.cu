@@ -799,7 +799,7 @@ cudaError_t launch_polish32(Geom g, const double *rA, const double *iA, const do
 // first wave per warp and the rest per lane -> this, ms: n=48, 500 block-triangular
 // matrices 227 -> 29.6; every tenth matrix block-triangular, n=16 x 100,000 41.1 ->
 // 36.1, n=32 x 20,000 125 -> 68.6, n=48 x 4,000 274 -> 80.1; all of them, n=16 x
-// 100,000 55.0 -> 50.0 (but n=32 x 20,000 98.8 -> 111).
+// 100,000 47.8 (lanes alone, all in FP64: 46.8), n=32 x 20,000 108 (106).
 cudaError_t launch_fp64_list(FusedArgs a, cudaStream_t st)
 {
     if (a.g.N <= 0) return cudaSuccess;

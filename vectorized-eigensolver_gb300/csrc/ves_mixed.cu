@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(kRefineThreads, 16) refine16_lane_kernel(const
 // as a signed high and a balanced signed low word.  Of a product the low-by-low
 // part (below 2^-58 of the scales, of random sign) is dropped, sums are exact;
 // FP64 rounds every partial sum, of size |lambda| |v_i|, to 2^-53 of it.  A
-// complex multiply-add takes twelve IMAD.WIDE (12 / 26 clocks per lane and SM)
+// complex multiply-add takes twelve IMAD.WIDE (12 / 25 clocks per lane and SM)
 // where FP64 takes 4 / 1.8.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ i64 fx_join(int h, int l) { return ((i64)h << 32) + l; }
@@ -1602,37 +1602,20 @@ namespace {
 
 // Which FP32 Schur kernel: 0 = schur32_kernel (a matrix per lane), G = 4 or
 // 8 = schur32_group_kernel<G>, G = 16 or 32 = schur32_warp_kernel<G> (a
-// matrix per G lanes).  With the fast FP32 division and square root, measured
-// on GB300 (FP32+refine eigensolves/s, stages in sequence, two float-float
-// steps): n=8 lane 47.9, group4 43.0, group8 36.1 M/s; n=12 lane 14.4,
-// group4 15.4, group8 12.9 M/s; n=16 lane 6.10 (6.43 overlapped), group4
-// 6.78, group8 7.04 M/s; later, with the division-free FP64 deflation test
-// and unrolled lane shares: n=11 lane 17.95, group4 19.88, group8 16.44;
-// n=14 8.72, 10.64, 10.16; n=16 5.95, 7.23, 7.72 M/s.  Default: the group
-// kernel with G = 4 for 11 <= n <= 14 and G = 8 for n = 15, 16.  Older
-// measurements, before the fast FP32 arithmetic and the group kernels:  Measured on GB300,
-// FP32+refine eigensolves/s, lane -> warp (G = 32): n=16 5.34 -> 4.26 M/s,
-// n=24 1.59 -> 1.63 M/s, n=32 0.66 -> 0.72 M/s (below 24 too many lanes of a
-// warp idle).  Two matrices per warp (G = 16) does not recover it: with the
-// Schur and refinement stages overlapped, lane -> G = 16 measured n=8 39.9 ->
-// 21.0, n=12 14.1 -> 9.3, n=16 5.84 -> 4.75 M/s (its Schur stage alone at
-// n=16: 90 ms per 1,048,576 matrices against about 78 for the lane kernel,
-// and it leaves less of each SM to the refinement running beside it).
-// Default: G = 32 for 24 <= n <= 32, the lane kernel otherwise.  Later, with
-// the warp kernel's two synchronisations per step and the float-float
-// refinement, stages one after the other: n=17 lane 4.88 (5.30 overlapped),
-// warp 5.38 M/s; n=20 lane 3.03 (3.36), warp 3.78 M/s.  The group kernel
-// generalised to n <= 32 (a matrix per 8 or 16 lanes) measured slower than
-// the warp kernel at n = 17..32 (n=20 3.64 / 3.73, n=24 1.77 / 2.16, n=32
-// 0.58 / 0.95 M/s against 3.78, 2.42, 1.10).  Default now: G = 32 for
-// 17 <= n <= 32.
-// Small batches, and n > 32 (two rows and columns per lane): a lane kernel's wave
-// takes 0.5 ms at n=9, 3 ms at n=16, 175 ms at n=64 however few matrices there
-// are, and above n=32 it is the slower one at every size.  ms, lane -> chosen:
-// 512 matrices n=9 0.523 -> 0.251 (G = 16), n=16 (group, G = 8) 0.610 -> 0.476
-// (G = 32); 8,192 n=9 0.634 -> 0.415 (group, G = 8); n=48 512 73.6 -> 4.88, 8,192
-// 147 -> 43.3; n=64 512 176 -> 12.4, 8,192 365 -> 110; n=40 32,768 192 -> 78.
-// At 32,768 n=9 the lane kernel is ahead again (1.24 against 1.28).
+// matrix per G lanes; n > 32: two rows and columns per lane).
+// Large batches: lane for n <= 10, G = 4 for n = 11 .. 14, G = 8 for n = 15, 16,
+// G = 32 above.  FP32+refine, M eigensolves/s, lane / G = 4 / G = 8: n=8 47.9 43.0
+// 36.1, n=11 17.95 19.88 16.44, n=14 8.72 10.64 10.16, n=16 5.95 7.23 7.72; lane
+// (stages overlapped) / G = 32: n=17 5.30 5.38, n=20 3.36 3.78, n=24 1.59 1.63, n=32
+// 0.66 0.72.  For n <= 16 the warp kernels leave too many lanes idle (n=16: G = 16
+// 4.75, G = 32 4.26), for n > 16 the group kernel holds too few matrices per SM
+// (n=20 3.73, n=32 0.95 against 1.10 of a later warp kernel).
+// Small batches, and n > 32: a lane kernel's wave takes 0.5 ms at n=9, 3 ms at n=16,
+// 175 ms at n=64 however few matrices there are, and above n=32 it is the slower one
+// at every size.  ms, lane -> chosen: 512 matrices n=9 0.523 -> 0.251 (G = 16), n=16
+// (G = 8) 0.610 -> 0.476 (G = 32); 8,192 n=9 0.634 -> 0.415 (G = 8); n=48 512 73.6 ->
+// 4.88, 8,192 147 -> 43.3; n=64 512 176 -> 12.4, 8,192 365 -> 110; n=40 32,768 192 ->
+// 78.  At 32,768 n=9 the lane kernel is ahead again (1.24 against 1.28).
 // The choice goes by the whole batch, so chunks of it take the same kernel.
 // VES_MIXED_SCHUR overrides (tests and tuning): lane; warp (G = 16 for
 // n <= 16, G = 32 above); warp16; warp32; warp64 (G = 32 for any n).
